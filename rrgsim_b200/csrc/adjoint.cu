@@ -782,6 +782,7 @@ struct rrg_adjoint {
     ABuf w;                 // FP32: half-step velocity of the reverse steps
     ABuf mflags;            // uniform-mass check: mismatch flag, mass bits
     int splits = 1;
+    bool force_sym = false;  // scratch holds the pair slots of the symmetric direct sum
     int vjp_splits = 1;
     double uniform_m = -1;  // >= 0 while every particle of the last forward has this mass
     bool mass_grad = true;  // compute dL/dm (the w slot of the position gradient)
@@ -806,6 +807,7 @@ void forces(rrg_adjoint* A, const void* x, void* acc, cudaStream_t s) {
     L.splits = A->splits;
     L.scratch = A->scratch.p;
     L.scratch_bytes = A->scratch.bytes;
+    L.sym_scratch = A->force_sym ? A->scratch.p : nullptr;
     L.stream = s;
     launch_direct(L);
 }
@@ -831,6 +833,7 @@ void direct_step(rrg_adjoint* A, const void* in, void* out, void* vel, void* acc
     L.splits = A->splits;
     L.scratch = A->scratch.p;
     L.scratch_bytes = A->scratch.bytes;
+    L.sym_scratch = A->force_sym ? A->scratch.p : nullptr;
     L.stream = s;
     launch_direct(L);
 }
@@ -974,7 +977,18 @@ RRG_API rrg_status rrg_adjoint_create(int device, int precision, int64_t n, doub
         const int sms = num_sms(device);
         A->splits = direct_choose_splits(precision, n, sms);
         const size_t sb = direct_scratch_bytes(precision, n, A->splits);
-        if (sb) A->scratch.alloc(sb);
+        // (whether the masses are equal is known only in the forward pass)
+        const size_t fs = std::max(direct_sym_scratch_bytes(precision, n, true, sms),
+                                   direct_sym_scratch_bytes(precision, n, false, sms));
+        if (fs) {
+            try {
+                A->scratch.alloc(fs);
+                A->force_sym = true;
+            } catch (const Error&) {
+                // no room for the slots: the ordered kernels
+            }
+        }
+        if (!A->force_sym && sb) A->scratch.alloc(sb);
         if (precision == RRG_PREC_FP64) {
             A->sym_slots.alloc(vjp_sym_slot_bytes<double>(n));
         } else {

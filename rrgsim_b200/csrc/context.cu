@@ -114,7 +114,7 @@ struct rrg_ctx {
     double uniform_mass = -1.0;  // >= 0 when every particle has this mass
     bool sorted = false;
     int splits = 1;
-    Buf scratch;
+    Buf scratch, sym_scratch;
 
     // grid
     bool has_grid = false;
@@ -256,8 +256,26 @@ void direct(rrg_ctx* c, bool want_pot, const DirectEpi& epi) {
     L.splits = c->splits;
     L.scratch = c->scratch.p;
     L.scratch_bytes = c->scratch.bytes;
+    L.sym_scratch = c->sym_scratch.p;
     L.stream = c->stream;
     launch_direct(L);
+}
+
+void drop_graphs(rrg_ctx* c);
+
+// The pair slots of the symmetric direct sum (direct_sym.cu), where that is the faster path; a
+// device without room for them runs the ordered kernels. Called before the first direct sum on
+// new particles, never while a graph is recorded.
+void ensure_sym(rrg_ctx* c) {
+    if (c->n <= 0) return;
+    const void* before = c->sym_scratch.p;
+    try {
+        c->sym_scratch.alloc(
+            direct_sym_scratch_bytes(c->prec, c->n, c->uniform_mass >= 0.0, c->sms));
+    } catch (const Error&) {
+        c->sym_scratch.release();
+    }
+    if (c->sym_scratch.p != before) drop_graphs(c);
 }
 
 void wave_source(rrg_ctx* c, bool zero_other) {
@@ -881,6 +899,7 @@ RRG_API rrg_status rrg_load_particles(rrg_ctx* ctx, int64_t n, const double* pos
         std::memcpy(&mmax, &ck.mass_max_bits, sizeof(double));
         const bool uniform = ck.soft_varies == 0;
         const bool umass = ck.mass_varies == 0;
+        const double uniform_mass_before = ctx->uniform_mass;
         ctx->uniform_mass = umass ? mass[0] : -1.0;
 
         // recorded graphs stay valid when the new particles reuse every buffer and launch value
@@ -888,7 +907,7 @@ RRG_API rrg_status rrg_load_particles(rrg_ctx* ctx, int64_t n, const double* pos
             return std::vector<const void*>{ctx->posm[0].p, ctx->posm[1].p, ctx->poslo[0].p,
                                             ctx->poslo[1].p, ctx->vel.p, ctx->acc.p, ctx->u.p,
                                             ctx->pot.p, ctx->hsoft.p, ctx->scratch.p,
-                                            ctx->step_partial.p};
+                                            ctx->sym_scratch.p, ctx->step_partial.p};
         };
         const auto before = layout();
         const int64_t n_before = ctx->n;
@@ -931,12 +950,14 @@ RRG_API rrg_status rrg_load_particles(rrg_ctx* ctx, int64_t n, const double* pos
         ctx->splits = direct_choose_splits(ctx->prec, n, ctx->sms);
         const size_t sb = direct_scratch_bytes(ctx->prec, n, ctx->splits);
         if (sb) ctx->scratch.alloc(sb);
+        if (ctx->sym_scratch.p || (ctx->solver_ready && !ctx->wave_mode)) ensure_sym(ctx);
         const int rb = conservation_blocks(n);
         ctx->red_partial.alloc(static_cast<size_t>(rb) * 12 * 2 * sizeof(double));  // (hi, lo)
         ctx->red_out.alloc(16 * sizeof(double));
         alloc_step_partial(ctx);
         if (layout() != before || n != n_before || ctx->shift_s != shift_before ||
-            ctx->uniform_hsoft != hsoft_before || ctx->soft_uniform != uniform_before)
+            ctx->uniform_hsoft != hsoft_before || ctx->soft_uniform != uniform_before ||
+            ctx->uniform_mass != uniform_mass_before)
             drop_graphs(ctx);
 
         // pack the staged arrays into the device state
@@ -1128,6 +1149,7 @@ RRG_API rrg_status rrg_nbody_acceleration(rrg_ctx* ctx) {
     RRG_ENTRY(ctx, {
         drop_pending(ctx);
         require_particles(ctx);
+        ensure_sym(ctx);
         DirectEpi e;
         e.mode = EPI_STORE;
         e.acc = ctx->acc.p;
@@ -1138,6 +1160,7 @@ RRG_API rrg_status rrg_nbody_acceleration(rrg_ctx* ctx) {
 RRG_API rrg_status rrg_nbody_grav(rrg_ctx* ctx) {
     RRG_ENTRY(ctx, {
         require_particles(ctx);
+        ensure_sym(ctx);
         // potential only: accelerations go to the scratch download buffer and are dropped
         ensure_download(ctx, v4b(ctx) * ctx->n);
         DirectEpi e;
@@ -1368,9 +1391,8 @@ RRG_API rrg_status rrg_solver_init(rrg_ctx* ctx, const rrg_sim_params* sim) {
             RRG_REQUIRE(ctx->has_wave, RRG_ERR_STATE,
                         "No wave params for rect wave integration solver");
         }
-        for (auto& kv : ctx->graphs)
-            if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
-        ctx->graphs.clear();
+        drop_graphs(ctx);
+        if (!ctx->wave_mode) ensure_sym(ctx);
         ctx->solver_ready = true;
     })
 }

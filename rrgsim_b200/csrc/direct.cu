@@ -14,83 +14,14 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "direct_epi.cuh"
 #include "kernels.cuh"
 
 namespace rrg {
 namespace {
 
-constexpr int kBS = 256;         // threads per block = j-tile length
-constexpr float kPadPos = 1e18f; // padding j: far away and massless -> contributes exactly 0
-
-template <typename R>
-struct EpiDev {
-    int mode;
-    R dt;
-    V4<R>* acc;
-    R* pot;
-    V4<R>* vel;
-    V4<R>* u;
-    V4<R>* pos_out;
-    V4<float>* lo_out;
-};
-
-template <typename R>
-EpiDev<R> make_epi(const DirectEpi& e) {
-    EpiDev<R> d;
-    d.mode = e.mode;
-    d.dt = static_cast<R>(e.dt);
-    d.acc = static_cast<V4<R>*>(e.acc);
-    d.pot = static_cast<R*>(e.pot);
-    d.vel = static_cast<V4<R>*>(e.vel);
-    d.u = static_cast<V4<R>*>(e.u);
-    d.pos_out = static_cast<V4<R>*>(e.pos_out);
-    d.lo_out = static_cast<V4<float>*>(e.lo_out);
-    return d;
-}
-
-// Per-particle epilogue. Arithmetic order follows predict_step_ / correct_step_
-// (nbody.cu:139-151, 175-180): v = 0.5 (u + dt a) with u = v_old + v*, v* = v + dt a,
-// x += (dt 0.5) (v + v*).
-template <typename R, bool MIXED>
-__device__ __forceinline__ void apply_epi(const EpiDev<R>& e, int64_t i, R ax, R ay, R az,
-                                          R phi, bool want_pot, const V4<R>* posm,
-                                          const V4<float>* poslo) {
-    if (want_pot && e.pot) e.pot[i] = phi;
-    if (e.mode == EPI_STORE) {
-        e.acc[i] = v4<R>(ax, ay, az, R(0));
-        return;
-    }
-    const V4<R> u = e.u[i];
-    const R dt = e.dt;
-    const R vx = R(0.5) * (u.x + dt * ax);
-    const R vy = R(0.5) * (u.y + dt * ay);
-    const R vz = R(0.5) * (u.z + dt * az);
-    if (e.mode == EPI_CORRECT) {
-        e.vel[i] = v4<R>(vx, vy, vz, R(0));
-        e.acc[i] = v4<R>(ax, ay, az, R(0));
-        return;
-    }
-    // EPI_CORRECT_PREDICT: next step's predict on the corrected velocity; the synced (v, a)
-    // of this step are stored too where the caller asks (checkpoints)
-    if (e.vel) e.vel[i] = v4<R>(vx, vy, vz, R(0));
-    if (e.acc) e.acc[i] = v4<R>(ax, ay, az, R(0));
-    const R sx = vx + dt * ax, sy = vy + dt * ay, sz = vz + dt * az;  // v*
-    const R ux = vx + sx, uy = vy + sy, uz = vz + sz;
-    e.u[i] = v4<R>(ux, uy, uz, R(0));
-    const R hdt = dt * R(0.5);
-    const V4<R> p = posm[i];
-    if constexpr (MIXED) {
-        const V4<float> lo = poslo[i];
-        float hx = p.x, lx = lo.x, hy = p.y, ly = lo.y, hz = p.z, lz = lo.z;
-        df_add(hx, lx, hdt * ux);
-        df_add(hy, ly, hdt * uy);
-        df_add(hz, lz, hdt * uz);
-        e.pos_out[i] = v4<R>(hx, hy, hz, p.w);
-        e.lo_out[i] = v4<float>(lx, ly, lz, 0.f);
-    } else {
-        e.pos_out[i] = v4<R>(p.x + hdt * ux, p.y + hdt * uy, p.z + hdt * uz, p.w);
-    }
-}
+constexpr int kBS = kDirectThreads;  // threads per block = j-tile length
+constexpr float kPadPos = kDirectPad;
 
 struct F32Params {
     const V4<float>* posm;
@@ -517,7 +448,9 @@ __global__ void direct_f32_finish(const F32Params p, int splits) {
 }
 
 // ----------------------------------------------------------------------------------------------
-// FP64: the reference arithmetic (1 / sqrt, cube), one i per thread.
+// FP64: one i per thread. The reciprocal square root is CUDA's rsqrt (within 1 ulp): 1 / sqrt
+// spent most of the FP64 pipe on its two Newton sequences (N = 8,192: 177 us per evaluation
+// against 116 with rsqrt).
 // ----------------------------------------------------------------------------------------------
 struct F64Params {
     const V4<double>* posm;
@@ -561,7 +494,7 @@ __global__ void __launch_bounds__(kBS) direct_f64_kernel(const F64Params p) {
             const V4<double> pj = s_pos[k];
             const double dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
             const double hs = USOFT ? (h + h) : (h + s_h[k]);
-            const double inv = 1.0 / sqrt(dx * dx + dy * dy + dz * dz + hs);
+            const double inv = rsqrt(dx * dx + dy * dy + dz * dz + hs);
             const double kk = pj.w * (inv * inv * inv);
             ax += dx * kk;
             ay += dy * kk;
@@ -701,6 +634,12 @@ size_t direct_scratch_bytes(int prec, int64_t n, int splits) {
 
 void launch_direct(const DirectLaunch& L) {
     RRG_REQUIRE(L.n > 0, RRG_ERR_INVALID, "direct sum: n must be positive");
+    if (L.sym_scratch) {
+        int dev = 0;
+        RRG_CUDA(cudaGetDevice(&dev));
+        launch_direct_sym(L, num_sms(dev));
+        return;
+    }
     const int splits = L.splits > 0 ? L.splits : 1;
     const int64_t tiles = (L.n + kBS - 1) / kBS;
     const int64_t tiles_per = (tiles + splits - 1) / splits;

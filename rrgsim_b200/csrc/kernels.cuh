@@ -42,12 +42,17 @@ struct DirectLaunch {
     int variant = 0;              // FP32 kernel variant (direct.cu); 0 = choose
     void* scratch = nullptr;      // partial sums when splits > 1
     size_t scratch_bytes = 0;
+    void* sym_scratch = nullptr;  // direct_sym_scratch_bytes of slots: each pair once (direct_sym.cu)
     cudaStream_t stream = nullptr;
 };
 
 int direct_choose_splits(int prec, int64_t n, int sms);
 size_t direct_scratch_bytes(int prec, int64_t n, int splits);
 void launch_direct(const DirectLaunch& L);
+// The same with each unordered pair evaluated once (direct_sym.cu); 0 where the ordered kernels
+// are the faster ones (launch_direct takes this path when sym_scratch is given).
+size_t direct_sym_scratch_bytes(int prec, int64_t n, bool umass, int sms);
+void launch_direct_sym(const DirectLaunch& L, int sms);
 
 // VJP of a(x, m) (FP32): out_i = (d<lam,a>/dx_i, d<lam,a>/dm_i).
 void launch_direct_vjp_f32(const void* posm, const void* hsoft, float uniform_hsoft, int64_t n,
