@@ -246,6 +246,13 @@ bool launch_wave_solve(int nx, int iterations, float* phi0, float* phi1, int cur
                        const unsigned long long* mg, unsigned long long* mg_zero, int shift_s,
                        double dx, double rho_sub, const WaveCoef& w, float* src, float4* acc4,
                        unsigned int* sync, size_t sync_bytes, cudaStream_t s);
+// `iterations` substeps on the full levels (the operator path) in the same persistent kernel's
+// other form, the source read from src: the same bits as launch_wave_step x iterations. maxbits
+// != nullptr: the last substep's max|dphi|, max|phi| folded into maxbits[0..1] as
+// launch_wave_step does. Returns false, launching nothing, where it does not apply.
+bool launch_wave_relax(int nx, int iterations, float* phi0, float* phi1, int cur,
+                       const float* src, const WaveCoef& w, unsigned long long* maxbits,
+                       unsigned int* sync, size_t sync_bytes, cudaStream_t s);
 // Trilinear gather of acc4 to particles (rm_mesh2p.cu:48-114).
 void launch_interp(int prec, int64_t n, const void* posm, const void* poslo, const GridDev& g,
                    const void* acc4, void* acc, cudaStream_t s);

@@ -57,6 +57,11 @@
 // arithmetic takes 74.7 us: its 10 exchanges (two cells deep, eight neighbours) cost about as
 // much as the 20 one-deep ones.
 //
+// The operator path (setup relaxation, rrg_solve_wave_equation) runs the same kernel on the full
+// levels (FULL): the substeps between two steady checks in one launch, the check's maxima from
+// the registers of the last one. 300 substeps with their nine checks at 128^3: 2.19 ms one launch
+// per substep (4.7 us each and their launches) -> 1.32 ms.
+//
 // All blocks must be resident together: the launch is cooperative and the host checks capacity
 // first. Every wait is bounded; one that runs out sets the error word and the block leaves (the
 // step's results are then invalid), and later launches return at once until the host, which
@@ -131,10 +136,14 @@ struct SolveArgs {
     double kf_d, km_d, kao_d;         // K_F, K_MAIN, K_ACTUAL + K_OLD - 1 for the increments' source
     float* src;                     // nullptr, or where the source is also stored
     float4* acc4;                   // nullptr: no gradient
+    unsigned long long* maxbits;    // FULL: nullptr, or where max|dphi|, max|phi| of the last
+                                    // substep are folded in
     unsigned int* sync;             // sync_bytes_for(blocks), zeroed before the first launch
 };
 
-template <int W>
+// FULL: `iterations` substeps on the levels themselves with the source read from a.src (the
+// operator path's form: no increments, no gradient, mg and mg_zero unused; kf = K_F).
+template <int W, bool FULL>
 __global__ void __launch_bounds__(kThreads, 2) wave_solve_kernel(const SolveArgs a) {
     using S = Shape<W>;
     constexpr int nx = S::nx, RB = S::RB, ZC = kZC;
@@ -290,7 +299,14 @@ __global__ void __launch_bounds__(kThreads, 2) wave_solve_kernel(const SolveArgs
     // the increments' source g from phi0 and its halo (wave_inc_source); the plain source stored
     // where asked, the other deposit cleared; then level 0 of the increments is zero everywhere
     // and the one before it phi_prev - phi0
-    {
+    if constexpr (FULL) {
+        const float4* const s4 = reinterpret_cast<const float4*>(a.src);
+#pragma unroll
+        for (int k = 0; k < ZC; ++k) {
+            old[k] = __ldcg(p4 + col + k * plane4);
+            srcs[k * kThreads + tid] = __ldcg(s4 + col + k * plane4);
+        }
+    } else {
         ulonglong2* z2 = reinterpret_cast<ulonglong2*>(a.mg_zero);
         float4 zm = zh[r * W + q];
         const float4 ztop = zh[(RB + r) * W + q];
@@ -333,7 +349,7 @@ __global__ void __launch_bounds__(kThreads, 2) wave_solve_kernel(const SolveArgs
         for (int k = 0; k < ZC; ++k) {
             const float4 out = cell(k, zm, k + 1 < ZC ? cur[k + 1] : ztop);
             zm = cur[k];
-            if (last) {
+            if (!FULL && last) {
                 // the solve's last substep: full levels, phi0 + d (phi0 read again: only this
                 // block writes its cells, after its last exchange)
                 const float4 p0 = __ldcg(c4 + col + k * plane4);
@@ -364,6 +380,32 @@ __global__ void __launch_bounds__(kThreads, 2) wave_solve_kernel(const SolveArgs
         }
     }
 
+    if constexpr (FULL) {
+        if (a.maxbits == nullptr) return;
+        // the last substep's max |dphi| and max |phi|, differences in FP64 as
+        // wave_periodic_x4_kernel takes them
+        double dmax = 0.0;
+        float amax = 0.f;
+#pragma unroll
+        for (int k = 0; k < ZC; ++k) {
+            const float4 c = cur[k], o = old[k];
+            dmax = fmax(dmax, fmax(fmax(fabs(double(c.x) - double(o.x)), fabs(double(c.y) - double(o.y))),
+                                   fmax(fabs(double(c.z) - double(o.z)), fabs(double(c.w) - double(o.w)))));
+            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(c.z), fabsf(c.w))));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            dmax = fmax(dmax, __shfl_down_sync(0xffffffffu, dmax, o));
+            amax = fmaxf(amax, __shfl_down_sync(0xffffffffu, amax, o));
+        }
+        if (lane == 0) {
+            // (non-negative doubles compare as their bit patterns)
+            atomicMax(a.maxbits, static_cast<unsigned long long>(__double_as_longlong(dmax)));
+            atomicMax(a.maxbits + 1, static_cast<unsigned long long>(
+                                         __double_as_longlong(static_cast<double>(amax))));
+        }
+        return;
+    }
     // ---- gradient of the final level (its halo is in place): central inside, one-sided at
     // the faces
     if (a.acc4 != nullptr) {
@@ -826,18 +868,31 @@ bool use_tb() {
     return on;
 }
 
-template <int W>
+template <int W, bool FULL>
 void set_smem_attr() {
-    RRG_CUDA(cudaFuncSetAttribute(wave_solve_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    RRG_CUDA(cudaFuncSetAttribute(wave_solve_kernel<W, FULL>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(Shape<W>::smem)));
 }
 
-template <int W>
+template <int W, bool FULL>
 int blocks_per_sm() {
     int per_sm = 0;
-    RRG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wave_solve_kernel<W>,
+    RRG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wave_solve_kernel<W, FULL>,
                                                            kThreads, Shape<W>::smem));
     return per_sm;
+}
+
+template <int W>
+int blocks_per_sm(bool full) {
+    return full ? blocks_per_sm<W, true>() : blocks_per_sm<W, false>();
+}
+
+template <int W>
+void launch_cooperative(cudaLaunchConfig_t& cfg, bool full, const SolveArgs& a) {
+    cfg.dynamicSmemBytes = Shape<W>::smem;
+    if (full) RRG_CUDA(cudaLaunchKernelEx(&cfg, wave_solve_kernel<W, true>, a));
+    else RRG_CUDA(cudaLaunchKernelEx(&cfg, wave_solve_kernel<W, false>, a));
 }
 
 int64_t block_count(int nx) {
@@ -859,12 +914,12 @@ size_t wave_solve_sync_bytes(int nx) {
     return (nx == 32 || nx == 64) ? sync_bytes_for(block_count(nx)) : kFaceOffset;
 }
 
-bool launch_wave_solve(int nx, int iterations, float* phi0, float* phi1, int cur,
-                       const unsigned long long* mg, unsigned long long* mg_zero, int shift_s,
-                       double dx, double rho_sub, const WaveCoef& w, float* src, float4* acc4,
-                       unsigned int* sync, size_t sync_bytes, cudaStream_t s) {
-    if (!wave_solve_applicable(nx) || iterations < 1) return false;
-    const bool tbk = nx == 128 && use_tb();
+namespace {
+
+// Launches the persistent kernel of the grid (the two-substep one for tbk); false, launching
+// nothing, where not all its blocks could be resident at once.
+bool launch_persistent(int nx, bool full, bool tbk, const SolveArgs& a, size_t sync_bytes,
+                       cudaStream_t s) {
     const int W = nx / 4, RB = (tbk ? tb::T : kThreads) / W;
     const dim3 grid(nx / RB, nx / kZC);
     const int64_t nblocks = static_cast<int64_t>(grid.x) * grid.y;
@@ -879,9 +934,12 @@ bool launch_wave_solve(int nx, int iterations, float* phi0, float* phi1, int cur
         static bool done[64] = {};
         std::lock_guard<std::mutex> lock(mu);
         if (dev < 0 || dev >= 64 || !done[dev]) {
-            set_smem_attr<8>();
-            set_smem_attr<16>();
-            set_smem_attr<32>();
+            set_smem_attr<8, false>();
+            set_smem_attr<16, false>();
+            set_smem_attr<32, false>();
+            set_smem_attr<8, true>();
+            set_smem_attr<16, true>();
+            set_smem_attr<32, true>();
             RRG_CUDA(cudaFuncSetAttribute(wave_solve_tb_kernel,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           static_cast<int>(tb::smem)));
@@ -893,10 +951,41 @@ bool launch_wave_solve(int nx, int iterations, float* phi0, float* phi1, int cur
         RRG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wave_solve_tb_kernel,
                                                                tb::T, tb::smem));
     else
-        per_sm = W == 8 ? blocks_per_sm<8>() : (W == 16 ? blocks_per_sm<16>() : blocks_per_sm<32>());
-    if (static_cast<int64_t>(per_sm) * num_sms(dev) < nblocks)
-        return false;  // not all blocks could be resident at once
-    SolveArgs a;
+        per_sm = W == 8 ? blocks_per_sm<8>(full)
+                        : (W == 16 ? blocks_per_sm<16>(full) : blocks_per_sm<32>(full));
+    if (static_cast<int64_t>(per_sm) * num_sms(dev) < nblocks) return false;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (tbk) {
+        cfg.blockDim = dim3(tb::T);
+        cfg.dynamicSmemBytes = tb::smem;
+        RRG_CUDA(cudaLaunchKernelEx(&cfg, wave_solve_tb_kernel, a));
+    } else if (W == 8) {
+        launch_cooperative<8>(cfg, full, a);
+    } else if (W == 16) {
+        launch_cooperative<16>(cfg, full, a);
+    } else {
+        launch_cooperative<32>(cfg, full, a);
+    }
+    RRG_LAUNCHED();
+    return true;
+}
+
+}  // namespace
+
+bool launch_wave_solve(int nx, int iterations, float* phi0, float* phi1, int cur,
+                       const unsigned long long* mg, unsigned long long* mg_zero, int shift_s,
+                       double dx, double rho_sub, const WaveCoef& w, float* src, float4* acc4,
+                       unsigned int* sync, size_t sync_bytes, cudaStream_t s) {
+    if (!wave_solve_applicable(nx) || iterations < 1) return false;
+    SolveArgs a{};
     a.phi0 = phi0;
     a.phi1 = phi1;
     a.cur = cur;
@@ -917,31 +1006,26 @@ bool launch_wave_solve(int nx, int iterations, float* phi0, float* phi1, int cur
     a.src = src;
     a.acc4 = acc4;
     a.sync = sync;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(kThreads);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (tbk) {
-        cfg.blockDim = dim3(tb::T);
-        cfg.dynamicSmemBytes = tb::smem;
-        RRG_CUDA(cudaLaunchKernelEx(&cfg, wave_solve_tb_kernel, a));
-    } else if (W == 8) {
-        cfg.dynamicSmemBytes = Shape<8>::smem;
-        RRG_CUDA(cudaLaunchKernelEx(&cfg, wave_solve_kernel<8>, a));
-    } else if (W == 16) {
-        cfg.dynamicSmemBytes = Shape<16>::smem;
-        RRG_CUDA(cudaLaunchKernelEx(&cfg, wave_solve_kernel<16>, a));
-    } else {
-        cfg.dynamicSmemBytes = Shape<32>::smem;
-        RRG_CUDA(cudaLaunchKernelEx(&cfg, wave_solve_kernel<32>, a));
-    }
-    RRG_LAUNCHED();
-    return true;
+    return launch_persistent(nx, false, nx == 128 && use_tb(), a, sync_bytes, s);
+}
+
+bool launch_wave_relax(int nx, int iterations, float* phi0, float* phi1, int cur,
+                       const float* src, const WaveCoef& w, unsigned long long* maxbits,
+                       unsigned int* sync, size_t sync_bytes, cudaStream_t s) {
+    if (!wave_solve_applicable(nx) || iterations < 1 || (nx == 128 && use_tb())) return false;
+    SolveArgs a{};
+    a.phi0 = phi0;
+    a.phi1 = phi1;
+    a.cur = cur;
+    a.iterations = iterations;
+    a.km = static_cast<float>(w.K_MAIN);
+    a.ka = static_cast<float>(w.K_ACTUAL);
+    a.ko = static_cast<float>(w.K_OLD);
+    a.kf = static_cast<float>(w.K_F);
+    a.src = const_cast<float*>(src);
+    a.maxbits = maxbits;
+    a.sync = sync;
+    return launch_persistent(nx, true, false, a, sync_bytes, s);
 }
 
 }  // namespace rrg
