@@ -21,6 +21,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -122,6 +123,7 @@ struct rrg_ctx {
     GridDev gdev{};
     Buf arena;                       // holds mg[0], mg[1], phi[0], phi[1] (views)
     cudaStream_t l2_stream = nullptr;  // the stream that carries the arena's L2 window
+    size_t l2_want = 0;                // its share of the persisting set-aside; 0: no window
     Buf mg[2], src, phi[2], acc4;
     int mg_cur = 0;
     int phi_cur = 0;
@@ -360,11 +362,14 @@ bool solve_step_fused(rrg_ctx* c, const WaveCoef& w, int iterations, bool store_
 
 // The deposit grids and the wave levels (the arena, 48 MB at 128^3) stay resident in L2 across
 // a step's kernels: a persisting access-policy window over the arena on the context stream, with
-// the process's persisting L2 set-aside sized to it (at most what the device allows; 79 MB of
-// the 126 MB on B200). Every step reads and rewrites all four grids, and the particle data and
-// the field would otherwise push them out between the particle pass and the solve: 121.8
-// against 125.4 us per PM step on 128^3 (the field in the window too: 123.8). Best effort: a
-// device or configuration without persisting L2 runs without it. RRG_L2_PERSIST=0 turns it off.
+// the process's persisting L2 set-aside sized to it. Every step reads and rewrites all four
+// grids, and the particle data and the field would otherwise push them out between the particle
+// pass and the solve: 121.8 against 125.4 us per PM step on 128^3 (the field in the window too:
+// 123.8). Only the FP32 / MIXED grids of the persistent solve have one: on the others every
+// substep goes through L2 as well, in buffers outside the arena, and the set-aside takes their
+// room. Per PM step with a window / without, us: FP32 144^3 332 / 302, 160^3 526 / 366, 192^3
+// 936 / 650, 256^3 2313 / 1358, FP64 128^3 292 / 265; 96^3 114 / 114. Best effort: a device or
+// configuration without persisting L2 runs without it. RRG_L2_PERSIST=0 turns it off.
 bool l2_persist_enabled() {
     static const bool on = [] {
         const char* e = std::getenv("RRG_L2_PERSIST");
@@ -384,8 +389,39 @@ void set_l2_window(cudaStream_t s, const void* base, size_t bytes, float hit) {
         (void)cudaGetLastError();
 }
 
+// The set-aside of a device (the current one) is the largest that its live windows want; with
+// the last window it is given back, and the lines that persist in it with it.
+void l2_set_aside(int device, size_t add, size_t remove) {
+    static std::mutex mu;
+    static std::map<int, std::multiset<size_t>> wants;
+    std::lock_guard<std::mutex> lock(mu);
+    auto& w = wants[device];
+    if (add) w.insert(add);
+    if (remove) {
+        const auto it = w.find(remove);
+        if (it != w.end()) w.erase(it);
+    }
+    if (cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, w.empty() ? 0 : *w.rbegin()) !=
+            cudaSuccess ||
+        (w.empty() && cudaCtxResetPersistingL2Cache() != cudaSuccess))
+        (void)cudaGetLastError();
+}
+
+// the window off again, on a stream that the context leaves (a caller's stream keeps no trace)
+// or before a grid without one
+void clear_l2_window(rrg_ctx* c) {
+    if (c->l2_want == 0) return;
+    set_l2_window(c->l2_stream, nullptr, 0, 0.f);
+    l2_set_aside(c->device, 0, c->l2_want);
+    c->l2_stream = nullptr;
+    c->l2_want = 0;
+}
+
 void apply_l2_window(rrg_ctx* c) {
-    if (!l2_persist_enabled() || !c->arena.p) return;
+    clear_l2_window(c);
+    if (!l2_persist_enabled() || !c->arena.p || c->prec == RRG_PREC_FP64 ||
+        !(c->grid.nx == 32 || c->grid.nx == 64 || c->grid.nx == 128))
+        return;
     int maxp = 0, maxw = 0;
     if (cudaDeviceGetAttribute(&maxp, cudaDevAttrMaxPersistingL2CacheSize, c->device) !=
             cudaSuccess ||
@@ -396,21 +432,12 @@ void apply_l2_window(rrg_ctx* c) {
     }
     if (maxp <= 0 || maxw <= 0) return;
     const size_t want = std::min(c->arena.bytes, static_cast<size_t>(maxp));
-    if (cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, want) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return;
-    }
+    l2_set_aside(c->device, want, 0);
+    c->l2_want = want;
     const size_t win = std::min(c->arena.bytes, static_cast<size_t>(maxw));
     set_l2_window(c->stream, c->arena.p, win,
                   std::min(1.0f, static_cast<float>(want) / static_cast<float>(win)));
     c->l2_stream = c->stream;
-}
-
-// the window off again on a stream that the context leaves (a caller's stream keeps no trace)
-void clear_l2_window(rrg_ctx* c) {
-    if (c->l2_stream == nullptr) return;
-    set_l2_window(c->l2_stream, nullptr, 0, 0.f);
-    c->l2_stream = nullptr;
 }
 
 // After a synchronisation: the persistent solve's error word is set when a wait between its
@@ -846,7 +873,7 @@ RRG_API rrg_status rrg_destroy(rrg_ctx* ctx) {
     if (!ctx) return RRG_OK;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
-    if (ctx->l2_stream != ctx->own_stream) clear_l2_window(ctx);
+    clear_l2_window(ctx);
     delete ctx;
     return RRG_OK;
 }
