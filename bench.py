@@ -510,7 +510,7 @@ def run_native(args):
                          "step": {"alg_bytes": step_bytes,
                                   "achieved": step_bytes / (el / args.steps) / 1e9,
                                   "frac": step_bytes / (el / args.steps) / 1e9 / hbm},
-                         "operator_substep": {"kernel": "wave_periodic_x4_kernel",
+                         "operator_substep": {"kernel": "wave_periodic_vec_kernel",
                                               "ms_per_launch": sub_ms,
                                               "achieved": 16 * cells / (sub_ms * 1e-3) / 1e9}},
             "cpu_baseline": cpu,

@@ -9,6 +9,7 @@
 
 #include "kernels.cuh"
 #include "sums.cuh"
+#include "wave_cells.cuh"
 
 namespace rrg {
 namespace {
@@ -295,6 +296,7 @@ __global__ void wave_inc_finish_kernel(int64_t nc, const float* phi0, const floa
 // thread), so two grid buffers rotate instead of the reference's three.
 // ----------------------------------------------------------------------------------------------
 constexpr int kTX = 32, kTY = 8;
+constexpr int kVecThreads = 128;
 
 struct WaveDev {
     int nx;
@@ -385,157 +387,106 @@ __device__ __forceinline__ void block_max_to(double dmax, double amax, int tid,
     }
 }
 
-// Periodic box without an absorbing layer (the reference's wired path, wave.cu:177-181):
-// constant coefficients, wrapped neighbours, and a compile-time z-chunk so the column's
-// ZC + 2 potential values are all requested before the first update (memory-level
-// parallelism for a latency-bound stencil).
-template <typename R, int ZC, bool CHECK>
-__global__ void __launch_bounds__(kTX* kTY, 8) wave_periodic_kernel(
-    const R* __restrict__ phi, R* __restrict__ phi_old, const R* __restrict__ src,
-    const WaveDev w, unsigned long long* __restrict__ maxbits) {
-    const int nx = w.nx;
-    const int plane = nx * nx;
-    const int tid = threadIdx.y * kTX + threadIdx.x;
-    const int x = blockIdx.x * kTX + threadIdx.x;
-    const int y = blockIdx.y * kTY + threadIdx.y;
-    double dmax = 0.0, amax = 0.0;
-    if (x < nx && y < nx) {
-        const int oxm = x > 0 ? -1 : nx - 1;
-        const int oxp = x < nx - 1 ? 1 : -(nx - 1);
-        const int oym = y > 0 ? -nx : (nx - 1) * nx;
-        const int oyp = y < nx - 1 ? nx : -(nx - 1) * nx;
-        const int col = x + y * nx;
-        const int z0 = blockIdx.z * ZC;
-        const R km = static_cast<R>(w.K_MAIN), ka = static_cast<R>(w.K_ACTUAL),
-                ko = static_cast<R>(w.K_OLD), kf = static_cast<R>(w.K_F);
-        R pv[ZC + 2];  // phi at z0 - 1 ... z0 + ZC (wrapped)
-#pragma unroll
-        for (int k = 0; k < ZC + 2; ++k) {
-            int z = z0 - 1 + k;
-            z = z < 0 ? z + nx : (z >= nx ? z - nx : z);
-            pv[k] = __ldg(phi + col + z * plane);
-        }
-#pragma unroll
-        for (int k = 0; k < ZC; ++k) {
-            const int z = z0 + k;
-            if (z < nx) {
-                const int c = col + z * plane;
-                const R lap = __ldg(phi + c + oxm) + __ldg(phi + c + oxp) +
-                              __ldg(phi + c + oym) + __ldg(phi + c + oyp) + pv[k] + pv[k + 2];
-                const R out = lap * km + pv[k + 1] * ka + phi_old[c] * ko + src[c] * kf;
-                phi_old[c] = out;
-                if constexpr (CHECK) {
-                    dmax = fmax(dmax, fabs(static_cast<double>(out) - static_cast<double>(pv[k + 1])));
-                    amax = fmax(amax, fabs(static_cast<double>(out)));
-                }
-            }
-        }
-    }
-    if constexpr (CHECK) block_max_to(dmax, amax, tid, maxbits);
-}
-
-// FP32 periodic box, four x-cells per thread as one float4 (nx % 4 == 0, and nx / 4 either
-// divides 32 or is a multiple of 32): a warp covers whole rows (nx <= 128) or 32 consecutive
-// float4 of one row, so the x - 1 / x + 4 neighbours are warp shuffles with the periodic wrap
-// inside the row's lanes (a scalar load at the two warp edges only when rows are wider than a
-// warp). Rows y +- 1 are coalesced float4 loads, the z neighbours a register pipeline of ZC + 2
-// planes. About 1.5 memory instructions per cell instead of 7. Same arithmetic as
-// wave_periodic_kernel: lap = x- + x+ + y- + y+ + z- + z+, out = lap K_MAIN + phi K_ACTUAL +
-// phi_old K_OLD + src K_F.
+// Periodic box without an absorbing layer (the reference's wired path, wave.cu:177-181): constant
+// coefficients, V consecutive x-cells per thread (16 bytes: four FP32 or two FP64, fewer where
+// the row length does not divide). A warp takes 32 V consecutive cells of a plane, so the x
+// neighbours are shuffles, with a scalar load where a row or the warp ends; rows y +- 1 are
+// coalesced vector loads, the z neighbours a register pipeline over ZC planes whose ZC + 2 values
+// are all requested before the first update (a latency-bound stencil). The arithmetic is
+// wave_cell's, every rounding written out, in every V and precision.
 // ADJ: the adjoint substep of the PM adjoint instead (phi the current cotangent C, phi_old the
 // previous one P, no source): P <- K_MAIN L6(C) + K_ACTUAL C + K_OLD P and F += K_F C.
-template <int ZC, bool CHECK, int BS, bool ADJ = false>
-__global__ void __launch_bounds__(BS, 1024 / BS) wave_periodic_x4_kernel(
-    const float* __restrict__ phi, float* __restrict__ phi_old, const float* __restrict__ src,
-    const WaveDev w, unsigned long long* __restrict__ maxbits, float* __restrict__ fadj = nullptr) {
+// Successive substeps are launched with programmatic dependence: a block's indices are ready when
+// the substep before it ends (no load is ahead of the wait).
+//
+// Bound: launch and L2 latency up to ~100^3 (2.1 us a substep at 64^3), L2 bandwidth to ~160^3,
+// HBM beyond (256^3: 268 MB in 46 us, 0.89 of the copy peak). Per substep in a graph on B200, us,
+// one-cell columns (FP64, and rows that do not tile a warp) or float4 rows without programmatic
+// launches -> here: FP32 33^3 2.61 -> 2.05, 64^3 2.39 -> 2.13, 96^3 4.68 -> 3.05, 100^3 7.21 ->
+// 3.16, 128^3 4.59 -> 4.35, 160^3 13.2 -> 8.5, 200^3 34.5 -> 20.4; FP64 64^3 2.99 -> 2.80, 100^3
+// 9.90 -> 4.69, 128^3 9.89 -> 8.19.
+template <typename R, int V, int ZC, bool CHECK, bool ADJ>
+__global__ void __launch_bounds__(kVecThreads, 8) wave_periodic_vec_kernel(
+    const R* phi, R* phi_old, const R* src, const WaveDev w,
+    unsigned long long* __restrict__ maxbits, R* fadj) {
+    using C = Cells<R, V>;
     const int nx = w.nx;
-    const int W = nx >> 2;       // float4 per row
-    const int plane4 = W * nx;   // float4 per plane
-    const int tid = threadIdx.x;
-    const int lane = tid & 31;
-    const int g = blockIdx.x * BS + tid;  // float4 index within a plane
-    const bool valid = g < plane4;
-    const int y = g / W, q = g - (g / W) * W;
-    int lsrc, rsrc;
-    bool lload = false, rload = false;
-    if (W >= 32) {
-        lsrc = (lane + 31) & 31;
-        rsrc = (lane + 1) & 31;
-        lload = W > 32 && lane == 0;
-        rload = W > 32 && lane == 31;
-    } else {
-        const int seg = lane - lane % W;
-        lsrc = seg + (lane - seg + W - 1) % W;
-        rsrc = seg + (lane - seg + 1) % W;
-    }
-    const float4* phi4 = reinterpret_cast<const float4*>(phi);
-    const float4* src4 = reinterpret_cast<const float4*>(src);
-    float4* old4 = reinterpret_cast<float4*>(phi_old);
-    const float km = static_cast<float>(w.K_MAIN), ka = static_cast<float>(w.K_ACTUAL),
-                ko = static_cast<float>(w.K_OLD), kf = static_cast<float>(w.K_F);
+    const int W = nx / V;        // V-cell units per row
+    const int plane = nx * nx;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int g = blockIdx.x * kVecThreads + tid;  // unit within a plane
+    const bool valid = g < W * nx;
+    const int y = valid ? g / W : 0, q = valid ? g - y * W : 0;
+    const int at = y * nx + q * V;
+    // rows that tile a warp keep the x neighbours in it; else those across the row's ends
+    // (periodic) or the warp's ends are loaded
+    const bool tiles = W <= 32 && 32 % W == 0;
+    const int lsrc = tiles && q == 0 ? lane + W - 1 : lane - 1;
+    const int rsrc = tiles && q == W - 1 ? lane - (W - 1) : lane + 1;
+    const bool lload = valid && !tiles && (lane == 0 || q == 0);
+    const bool rload = valid && !tiles && (lane == 31 || q == W - 1);
+    const int xl = (q == 0 ? nx : q * V) - 1 + y * nx, xr = (q == W - 1 ? 0 : q * V + V) + y * nx;
+    const int aym = y > 0 ? at - nx : at + plane - nx, ayp = y < nx - 1 ? at + nx : at - plane + nx;
+    const R km = static_cast<R>(w.K_MAIN), ka = static_cast<R>(w.K_ACTUAL),
+            ko = static_cast<R>(w.K_OLD), kf = static_cast<R>(w.K_F);
     const int z0 = blockIdx.y * ZC;
-    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 pv[ZC + 2];  // phi at z0 - 1 ... z0 + ZC (wrapped)
+    pdl_next();
+    pdl_wait();
+    C pv[ZC + 2];  // phi at z0 - 1 ... z0 + ZC (wrapped)
 #pragma unroll
     for (int k = 0; k < ZC + 2; ++k) {
         int z = z0 - 1 + k;
-        z = z < 0 ? z + nx : (z >= nx ? z - nx : z);
-        pv[k] = valid ? __ldg(phi4 + g + z * plane4) : zero4;
+        z = z < 0 ? z + nx : z;
+        while (z >= nx) z -= nx;
+        pv[k] = load_cells<R, V>(phi + (at + z * plane));
     }
-    const int gym = y > 0 ? g - W : g + (nx - 1) * W;
-    const int gyp = y < nx - 1 ? g + W : g - (nx - 1) * W;
-    const int xl = q == 0 ? nx - 1 : 4 * q - 1;      // row-local x of the left edge value
-    const int xr = q == W - 1 ? 0 : 4 * q + 4;       // and of the right one
     double dmax = 0.0, amax = 0.0;
 #pragma unroll
     for (int k = 0; k < ZC; ++k) {
         const int z = z0 + k;
-        const float4 c = pv[k + 1];
-        float lft = __shfl_sync(0xffffffffu, c.w, lsrc);
-        float rgt = __shfl_sync(0xffffffffu, c.x, rsrc);
+        if (z >= nx) break;
+        const C c = pv[k + 1];
+        R lft = __shfl_sync(0xffffffffu, c.v[V - 1], lsrc & 31);
+        R rgt = __shfl_sync(0xffffffffu, c.v[0], rsrc & 31);
         if (valid) {
-            const int rowbase = z * nx * nx + y * nx;
-            if (lload) lft = __ldg(phi + rowbase + xl);
-            if (rload) rgt = __ldg(phi + rowbase + xr);
-            const int o = g + z * plane4;
-            const float4 ym = __ldg(phi4 + gym + z * plane4);
-            const float4 yp = __ldg(phi4 + gyp + z * plane4);
-            const float4 zm = pv[k], zp = pv[k + 2];
-            const float4 po = old4[o];
-            if constexpr (ADJ) {
-                old4[o] = wave_cell4(c, lft, rgt, ym, yp, zm, zp, po, zero4, km, ka, ko, 0.f);
-                float4* f4 = reinterpret_cast<float4*>(fadj) + o;
-                float4 f = *f4;
-                f.x = __fmaf_rn(kf, c.x, f.x);
-                f.y = __fmaf_rn(kf, c.y, f.y);
-                f.z = __fmaf_rn(kf, c.z, f.z);
-                f.w = __fmaf_rn(kf, c.w, f.w);
-                *f4 = f;
-                continue;
+            const int zb = z * plane;
+            if (lload) lft = load_cells<R, 1>(phi + (xl + zb)).v[0];
+            if (rload) rgt = load_cells<R, 1>(phi + (xr + zb)).v[0];
+            const C ym = load_cells<R, V>(phi + (aym + zb));
+            const C yp = load_cells<R, V>(phi + (ayp + zb));
+            const C po = load_cells<R, V>(phi_old + (at + zb));
+            C other;  // the source, or F
+            if constexpr (ADJ) other = load_cells<R, V>(fadj + (at + zb));
+            else other = load_cells<R, V>(src + (at + zb));
+            C out;
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                const R l = i == 0 ? lft : c.v[i > 0 ? i - 1 : 0];
+                const R r = i == V - 1 ? rgt : c.v[i < V - 1 ? i + 1 : 0];
+                const R t = wave_cell_adj(l, r, ym.v[i], yp.v[i], pv[k].v[i], pv[k + 2].v[i],
+                                          c.v[i], po.v[i], km, ka, ko);
+                if constexpr (ADJ) {
+                    out.v[i] = t;
+                    other.v[i] = rfma(kf, c.v[i], other.v[i]);
+                } else {
+                    out.v[i] = rfma(other.v[i], kf, t);
+                }
+                if constexpr (CHECK) {
+                    // differences in FP64
+                    dmax = fmax(dmax, fabs(double(out.v[i]) - double(c.v[i])));
+                    amax = fmax(amax, fabs(double(out.v[i])));
+                }
             }
-            const float4 s = __ldg(src4 + o);
-            const float4 out = wave_cell4(c, lft, rgt, ym, yp, zm, zp, po, s, km, ka, ko, kf);
-            old4[o] = out;
-            if constexpr (CHECK) {
-                // differences in FP64, as the scalar kernels take them
-                const double d = fmax(fmax(fabs(double(out.x) - double(c.x)),
-                                           fabs(double(out.y) - double(c.y))),
-                                      fmax(fabs(double(out.z) - double(c.z)),
-                                           fabs(double(out.w) - double(c.w))));
-                const float a = fmaxf(fmaxf(fabsf(out.x), fabsf(out.y)),
-                                      fmaxf(fabsf(out.z), fabsf(out.w)));
-                dmax = fmax(dmax, d);
-                amax = fmax(amax, static_cast<double>(a));
-            }
+            *reinterpret_cast<C*>(phi_old + (at + zb)) = out;
+            if constexpr (ADJ) *reinterpret_cast<C*>(fadj + (at + zb)) = other;
         }
     }
     if constexpr (CHECK) block_max_to(dmax, amax, tid, maxbits);
 }
 
-// UNIFORM is the periodic box without an absorbing layer (the reference's wired path): the
-// boundary code compiles away and the kernel fits 8 resident blocks per SM.
-template <typename R, bool UNIFORM, bool CHECK>
-__global__ void __launch_bounds__(kTX* kTY, UNIFORM ? 8 : 2) wave_step_kernel(
+// Every other boundary, and the absorbing layer.
+template <typename R, bool CHECK>
+__global__ void __launch_bounds__(kTX* kTY, 2) wave_step_kernel(
     const R* __restrict__ phi, R* __restrict__ phi_old, const R* __restrict__ src,
     const WaveDev w, unsigned long long* __restrict__ maxbits) {
     // One thread per (x, y) column marches through zc planes: phi(z - 1), phi(z), phi(z + 1)
@@ -547,7 +498,7 @@ __global__ void __launch_bounds__(kTX* kTY, UNIFORM ? 8 : 2) wave_step_kernel(
     const int x = blockIdx.x * kTX + threadIdx.x;
     const int y = blockIdx.y * kTY + threadIdx.y;
     const bool valid = (x < nx) && (y < nx);
-    const bool periodic = UNIFORM ? true : (w.bc == RRG_BC_PERIODIC);
+    const bool periodic = w.bc == RRG_BC_PERIODIC;
     double dmax = 0.0, amax = 0.0;
     if (valid) {
         // in-plane neighbour offsets: periodic wrap, or clamped (unused on the boundary nodes)
@@ -578,25 +529,17 @@ __global__ void __launch_bounds__(kTX* kTY, UNIFORM ? 8 : 2) wave_step_kernel(
             } else {
                 const R lap = __ldg(phi + c + oxm) + __ldg(phi + c + oxp) +
                               __ldg(phi + c + oym) + __ldg(phi + c + oyp) + pm + pn;
-                R kmain, kact, kold, kf;
-                if constexpr (UNIFORM) {
-                    kmain = static_cast<R>(w.K_MAIN);
-                    kact = static_cast<R>(w.K_ACTUAL);
-                    kold = static_cast<R>(w.K_OLD);
-                    kf = static_cast<R>(w.K_F);
-                } else {
-                    double diss = w.diss_base;
-                    diss += layer_diss(w, w.domain_min + x * w.DX);
-                    diss += layer_diss(w, w.domain_min + y * w.DX);
-                    diss += layer_diss(w, w.domain_min + z * w.DX);
-                    const double Q = diss * w.C * w.DT * 0.5;
-                    const double W = 1 + Q;
-                    const double K = w.C * w.C * w.DT * w.DT / (w.DX * w.DX);
-                    kmain = static_cast<R>(K / W);
-                    kf = static_cast<R>(-w.C * w.C * w.DT * w.DT / W);
-                    kact = static_cast<R>(2 * (1 - 3 * K) / W);
-                    kold = static_cast<R>((Q - 1) / W);
-                }
+                double diss = w.diss_base;
+                diss += layer_diss(w, w.domain_min + x * w.DX);
+                diss += layer_diss(w, w.domain_min + y * w.DX);
+                diss += layer_diss(w, w.domain_min + z * w.DX);
+                const double Q = diss * w.C * w.DT * 0.5;
+                const double W = 1 + Q;
+                const double K = w.C * w.C * w.DT * w.DT / (w.DX * w.DX);
+                const R kmain = static_cast<R>(K / W);
+                const R kf = static_cast<R>(-w.C * w.C * w.DT * w.DT / W);
+                const R kact = static_cast<R>(2 * (1 - 3 * K) / W);
+                const R kold = static_cast<R>((Q - 1) / W);
                 out = lap * kmain + pc * kact + phi_old[c] * kold + src[c] * kf;
             }
             phi_old[c] = out;
@@ -662,11 +605,11 @@ __global__ void __launch_bounds__(kTX* kTY) gradient_kernel(int nx, R coef,
     acc4[c] = v4<R>(dx * coef, dy * coef, dz * coef, pc);
 }
 
-// FP32 gradient with four x-cells per thread (float4 rows, as wave_periodic_x4_kernel): x +- 1
-// by warp shuffles (a scalar load at warp edges when a row is wider than a warp), rows y +- 1 as
-// coalesced float4 loads, the z neighbours from a register pipeline over ZC planes, and the four
+// FP32 gradient with four x-cells per thread (float4 rows, as wave_periodic_vec_kernel): x +- 1
+// by warp shuffles (a scalar load where a warp ends inside a row), rows y +- 1 as coalesced
+// float4 loads, the z neighbours from a register pipeline over ZC planes, and the four
 // (ax, ay, az, phi) cells written as four float4 stores. Same expressions, faces one-sided, as
-// gradient_kernel. Needs nx % 4 == 0, nx % ZC == 0 and nx / 4 dividing 32 or a multiple of 32.
+// gradient_kernel. Needs nx % 4 == 0 and nx % ZC == 0.
 template <int ZC, int BS>
 __global__ void __launch_bounds__(BS) gradient_x4_kernel(int nx, float coef,
                                                          const float* __restrict__ phi,
@@ -677,18 +620,8 @@ __global__ void __launch_bounds__(BS) gradient_x4_kernel(int nx, float coef,
     const int g = blockIdx.x * BS + tid;
     const bool valid = g < plane4;
     const int y = g / W, q = g - (g / W) * W;
-    int lsrc, rsrc;
-    bool lload = false, rload = false;
-    if (W >= 32) {
-        lsrc = (lane + 31) & 31;
-        rsrc = (lane + 1) & 31;
-        lload = W > 32 && lane == 0 && q > 0;
-        rload = W > 32 && lane == 31 && q < W - 1;
-    } else {
-        const int seg = lane - lane % W;
-        lsrc = seg + (lane - seg + W - 1) % W;
-        rsrc = seg + (lane - seg + 1) % W;
-    }
+    // (a neighbour across the row's end is not used: the faces are one-sided)
+    const bool lload = lane == 0 && q > 0, rload = lane == 31 && q < W - 1;
     const float4* phi4 = reinterpret_cast<const float4*>(phi);
     const int z0 = blockIdx.y * ZC;
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -705,8 +638,8 @@ __global__ void __launch_bounds__(BS) gradient_x4_kernel(int nx, float coef,
     for (int k = 0; k < ZC; ++k) {
         const int z = z0 + k;
         const float4 c = pv[k + 1];
-        float lft = __shfl_sync(0xffffffffu, c.w, lsrc);
-        float rgt = __shfl_sync(0xffffffffu, c.x, rsrc);
+        float lft = __shfl_up_sync(0xffffffffu, c.w, 1);
+        float rgt = __shfl_down_sync(0xffffffffu, c.x, 1);
         if (!valid) continue;
         const int rowbase = z * nx * nx + y * nx;
         if (lload) lft = __ldg(phi + rowbase + x - 1);
@@ -1083,12 +1016,79 @@ void launch_wave_inc_finish(int nx, const float* phi0, const float* d_fin, const
     RRG_LAUNCHED();
 }
 
-// One adjoint substep of the PM adjoint with the float4 stencil (FP32, periodic): false,
-// launching nothing, on grids whose rows do not tile into warps.
-bool launch_wave_adjoint_step(int nx, const float* C, float* P, float* F, double km, double ka,
-                              double beta, double kf, cudaStream_t s) {
-    const int W4 = nx / 4;
-    if (nx < 16 || nx % 8 != 0 || !(32 % W4 == 0 || W4 % 32 == 0)) return false;
+namespace {
+
+// V-cell units of a thread's 16 bytes (or fewer, for the row length)
+int cells_per_thread(int nx, bool f64) {
+    if (!f64 && nx % 4 == 0) return 4;
+    return nx % 2 == 0 ? 2 : 1;
+}
+
+template <typename R, int V, int ZC, bool ADJ>
+void launch_vec(const WaveDev& w, const R* phi, R* old, const R* src, R* f,
+                unsigned long long* maxbits, cudaStream_t s) {
+    const dim3 grid(div_up(static_cast<int64_t>(w.nx / V) * w.nx, kVecThreads), div_up(w.nx, ZC));
+    if constexpr (!ADJ) {
+        if (maxbits) {
+            launch_pdl(wave_periodic_vec_kernel<R, V, ZC, true, false>, grid, kVecThreads, 0, s, phi,
+                       old, src, w, maxbits, f);
+            RRG_LAUNCHED();
+            return;
+        }
+    }
+    launch_pdl(wave_periodic_vec_kernel<R, V, ZC, false, ADJ>, grid, kVecThreads, 0, s, phi, old, src,
+               w, maxbits, f);
+    RRG_LAUNCHED();
+}
+
+// z-chunk: the longest of 8, 4, 2 planes that still gives four 128-thread blocks per SM (at
+// 128^3 FP32 that is 4, measured fastest inside the PM step; RRG_WAVE_ZC fixes it, for sweeps)
+template <typename R, int V, bool ADJ>
+void launch_vec_z(const WaveDev& w, const R* phi, R* old, const R* src, R* f,
+                  unsigned long long* maxbits, cudaStream_t s) {
+    static const int fixed = [] {
+        const char* e = std::getenv("RRG_WAVE_ZC");
+        return e ? std::atoi(e) : 0;
+    }();
+    int dev = 0;
+    RRG_CUDA(cudaGetDevice(&dev));
+    const int sms = num_sms(dev);
+    const int64_t rows = div_up(static_cast<int64_t>(w.nx / V) * w.nx, kVecThreads);
+    int z = 2;
+    for (int cand : {8, 4})
+        if (rows * div_up(w.nx, cand) >= 4 * sms) {
+            z = cand;
+            break;
+        }
+    if (fixed == 2 || fixed == 4 || fixed == 8) z = fixed;
+    if (z == 8) launch_vec<R, V, 8, ADJ>(w, phi, old, src, f, maxbits, s);
+    else if (z == 4) launch_vec<R, V, 4, ADJ>(w, phi, old, src, f, maxbits, s);
+    else launch_vec<R, V, 2, ADJ>(w, phi, old, src, f, maxbits, s);
+}
+
+template <bool ADJ>
+void launch_vec_any(int prec, const WaveDev& w, const void* phi, void* old, const void* src,
+                    void* f, unsigned long long* maxbits, cudaStream_t s) {
+    const bool f64 = prec == RRG_PREC_FP64;
+    const int V = cells_per_thread(w.nx, f64);
+#define RRG_VEC(R, VV)                                                                        \
+    launch_vec_z<R, VV, ADJ>(w, static_cast<const R*>(phi), static_cast<R*>(old),             \
+                             static_cast<const R*>(src), static_cast<R*>(f), maxbits, s)
+    if (f64) {
+        if (V == 2) RRG_VEC(double, 2);
+        else RRG_VEC(double, 1);
+    } else {
+        if (V == 4) RRG_VEC(float, 4);
+        else if (V == 2) RRG_VEC(float, 2);
+        else RRG_VEC(float, 1);
+    }
+#undef RRG_VEC
+}
+
+}  // namespace
+
+void launch_wave_adjoint_step(int prec, int nx, const void* C, void* P, void* F, double km,
+                              double ka, double beta, double kf, cudaStream_t s) {
     WaveDev w{};
     w.nx = nx;
     w.uniform = 1;
@@ -1097,46 +1097,7 @@ bool launch_wave_adjoint_step(int nx, const float* C, float* P, float* F, double
     w.K_ACTUAL = ka;
     w.K_OLD = beta;
     w.K_F = kf;
-    // z-chunk as the forward stencil chooses it: the longest of 8, 4, 2 planes that still gives
-    // two 256-thread blocks' worth of threads per SM
-    int dev = 0;
-    RRG_CUDA(cudaGetDevice(&dev));
-    const int sms = num_sms(dev);
-    const int bs = 128;
-    const int rows_blocks = div_up(static_cast<int64_t>(W4) * nx, bs);
-    int zx = 2;
-    for (int cand : {8, 4})
-        if (static_cast<int64_t>(rows_blocks) * (nx / cand) * bs >= 2 * 256 * sms) {
-            zx = cand;
-            break;
-        }
-    const dim3 g4(rows_blocks, nx / zx);
-    if (zx == 8)
-        wave_periodic_x4_kernel<8, false, 128, true><<<g4, bs, 0, s>>>(C, P, nullptr, w, nullptr, F);
-    else if (zx == 4)
-        wave_periodic_x4_kernel<4, false, 128, true><<<g4, bs, 0, s>>>(C, P, nullptr, w, nullptr, F);
-    else
-        wave_periodic_x4_kernel<2, false, 128, true><<<g4, bs, 0, s>>>(C, P, nullptr, w, nullptr, F);
-    RRG_LAUNCHED();
-    return true;
-}
-
-// RRG_WAVE_BS = 128 / 256 fixes the block size of the float4 stencil (for sweeps).
-int wave_bs_override() {
-    static const int v = [] {
-        const char* e = std::getenv("RRG_WAVE_BS");
-        return e ? std::atoi(e) : 0;
-    }();
-    return v;
-}
-
-// RRG_WAVE_ZC = 2 / 4 / 8 fixes the z-chunk of the float4 stencil (for sweeps).
-int wave_zc_override() {
-    static const int v = [] {
-        const char* e = std::getenv("RRG_WAVE_ZC");
-        return e ? std::atoi(e) : 0;
-    }();
-    return v;
+    launch_vec_any<true>(prec, w, C, P, nullptr, F, nullptr, s);
 }
 
 void launch_wave_step(int prec, int nx, const void* phi, void* phi_old_inout, const void* src,
@@ -1161,13 +1122,17 @@ void launch_wave_step(int prec, int nx, const void* phi, void* phi_old_inout, co
     w.comy = c.com[1];
     w.comz = c.com[2];
     w.r_min = c.r_min;
+    const bool check = maxbits != nullptr;
+    if (w.uniform) {
+        launch_vec_any<false>(prec, w, phi, phi_old_inout, src, nullptr, maxbits, s);
+        return;
+    }
     const int gx = div_up(nx, kTX), gy = div_up(nx, kTY);
     // z-chunk: trade wave efficiency (blocks against 8 resident 256-thread blocks per SM)
     // against the one extra plane each column loads per chunk
     int dev = 0;
     RRG_CUDA(cudaGetDevice(&dev));
-    static int sms = 0;
-    if (!sms) sms = num_sms(dev);
+    const int sms = num_sms(dev);
     const int64_t slots = static_cast<int64_t>(sms) * 8;
     int zc = 32;
     double best = -1.0;
@@ -1185,86 +1150,13 @@ void launch_wave_step(int prec, int nx, const void* phi, void* phi_old_inout, co
     w.zc = zc;
     dim3 grid(gx, gy, div_up(nx, zc));
     dim3 block(kTX, kTY);
-    const bool check = maxbits != nullptr;
-    const int W4 = nx / 4;
-    if (w.uniform && prec != RRG_PREC_FP64 && nx >= 16 && nx % 4 == 0 &&
-        (32 % W4 == 0 || W4 % 32 == 0)) {
-        // float4 rows: z-chunk of 2, 4 or 8 planes (dividing nx), at least two blocks per SM
-        // (at 128^3 that is 4, measured fastest inside the PM step on B200)
-        // 128-thread blocks: at 128^3 with 4-plane chunks 1024 blocks fill 8 per SM to 99%
-        // (256-thread blocks: 512 on 4 per SM, 86%); measured faster inside the PM step
-        const int bs = wave_bs_override() == 256 ? 256 : 128;
-        const int rows_blocks = div_up(static_cast<int64_t>(W4) * nx, bs);
-        int zx = wave_zc_override();
-        if (zx != 2 && zx != 4 && zx != 8) {
-            zx = 2;
-            for (int cand : {8, 4})
-                if (nx % cand == 0 &&
-                    static_cast<int64_t>(rows_blocks) * (nx / cand) * bs >= 2 * 256 * sms) {
-                    zx = cand;
-                    break;
-                }
-        }
-        if (nx % zx != 0) zx = 2;
-        dim3 g4(rows_blocks, nx / zx);
-        const float* p = static_cast<const float*>(phi);
-        float* po = static_cast<float*>(phi_old_inout);
-        const float* sr = static_cast<const float*>(src);
-#define RRG_WAVE_X4B(Z, B)                                                                   \
-    do {                                                                                      \
-        if (check) wave_periodic_x4_kernel<Z, true, B><<<g4, B, 0, s>>>(p, po, sr, w, maxbits); \
-        else wave_periodic_x4_kernel<Z, false, B><<<g4, B, 0, s>>>(p, po, sr, w, maxbits);      \
-    } while (0)
-#define RRG_WAVE_X4(Z)                  \
-    do {                                \
-        if (bs == 128) RRG_WAVE_X4B(Z, 128); \
-        else RRG_WAVE_X4B(Z, 256);      \
-    } while (0)
-        if (zx == 8) RRG_WAVE_X4(8);
-        else if (zx == 4) RRG_WAVE_X4(4);
-        else RRG_WAVE_X4(2);
-#undef RRG_WAVE_X4
-#undef RRG_WAVE_X4B
-        RRG_LAUNCHED();
-        return;
-    }
-    if (w.uniform) {
-        // compile-time chunk of 2, 4 or 8 planes, the nearest the chooser's pick
-        const int zcf = zc >= 8 ? 8 : (zc >= 4 ? 4 : 2);
-        dim3 g2(gx, gy, div_up(nx, zcf));
-#define RRG_WAVE_P(R, Z)                                                                      \
-    do {                                                                                      \
-        const R* p = static_cast<const R*>(phi);                                              \
-        R* po = static_cast<R*>(phi_old_inout);                                               \
-        const R* sr = static_cast<const R*>(src);                                             \
-        if (check) wave_periodic_kernel<R, Z, true><<<g2, block, 0, s>>>(p, po, sr, w, maxbits); \
-        else wave_periodic_kernel<R, Z, false><<<g2, block, 0, s>>>(p, po, sr, w, maxbits);      \
-    } while (0)
-        if (prec == RRG_PREC_FP64) {
-            if (zcf == 8) RRG_WAVE_P(double, 8);
-            else if (zcf == 4) RRG_WAVE_P(double, 4);
-            else RRG_WAVE_P(double, 2);
-        } else {
-            if (zcf == 8) RRG_WAVE_P(float, 8);
-            else if (zcf == 4) RRG_WAVE_P(float, 4);
-            else RRG_WAVE_P(float, 2);
-        }
-#undef RRG_WAVE_P
-        RRG_LAUNCHED();
-        return;
-    }
 #define RRG_WAVE_LAUNCH(R)                                                                    \
     do {                                                                                      \
         const R* p = static_cast<const R*>(phi);                                              \
         R* po = static_cast<R*>(phi_old_inout);                                               \
         const R* sr = static_cast<const R*>(src);                                             \
-        if (w.uniform) {                                                                      \
-            if (check) wave_step_kernel<R, true, true><<<grid, block, 0, s>>>(p, po, sr, w, maxbits); \
-            else wave_step_kernel<R, true, false><<<grid, block, 0, s>>>(p, po, sr, w, maxbits);     \
-        } else {                                                                              \
-            if (check) wave_step_kernel<R, false, true><<<grid, block, 0, s>>>(p, po, sr, w, maxbits); \
-            else wave_step_kernel<R, false, false><<<grid, block, 0, s>>>(p, po, sr, w, maxbits);     \
-        }                                                                                     \
+        if (check) wave_step_kernel<R, true><<<grid, block, 0, s>>>(p, po, sr, w, maxbits);   \
+        else wave_step_kernel<R, false><<<grid, block, 0, s>>>(p, po, sr, w, maxbits);        \
     } while (0)
     if (prec == RRG_PREC_FP64) RRG_WAVE_LAUNCH(double);
     else RRG_WAVE_LAUNCH(float);
@@ -1275,7 +1167,7 @@ void launch_wave_step(int prec, int nx, const void* phi, void* phi_old_inout, co
 void launch_gradient(int prec, int nx, double dx, const void* phi, void* acc4, cudaStream_t s) {
     const double coef = -1.0 / dx;
     const int W4 = nx / 4;
-    if (prec != RRG_PREC_FP64 && nx >= 8 && nx % 4 == 0 && (32 % W4 == 0 || W4 % 32 == 0)) {
+    if (prec != RRG_PREC_FP64 && nx >= 8 && nx % 4 == 0) {
         dim3 g4(div_up(static_cast<int64_t>(W4) * nx, 128), nx / 4);
         gradient_x4_kernel<4, 128><<<g4, 128, 0, s>>>(nx, static_cast<float>(coef),
                                                       static_cast<const float*>(phi),

@@ -118,28 +118,6 @@ __global__ void __launch_bounds__(256) gradient_adjoint_kernel(int nx, R coef, c
     phi_bar[c] += coef * s;
 }
 
-// adjoint substep on the periodic box: P <- K_M L6(C) + K_A C + beta P;  F += K_F C
-template <typename R>
-__global__ void __launch_bounds__(256) wave_adjoint_kernel(int nx, const R* __restrict__ C, R* __restrict__ P,
-                                                           R* __restrict__ F, R km, R ka, R beta,
-                                                           R kf) {
-    const int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t nc = static_cast<int64_t>(nx) * nx * nx;
-    if (c >= nc) return;
-    const int64_t plane = static_cast<int64_t>(nx) * nx;
-    const int x = static_cast<int>(c % nx), y = static_cast<int>((c / nx) % nx),
-              z = static_cast<int>(c / plane);
-    const int64_t xm = x > 0 ? c - 1 : c + nx - 1, xp = x < nx - 1 ? c + 1 : c - (nx - 1);
-    const int64_t ym = y > 0 ? c - nx : c + (nx - 1) * nx,
-                  yp = y < nx - 1 ? c + nx : c - static_cast<int64_t>(nx - 1) * nx;
-    const int64_t zm = z > 0 ? c - plane : c + (nx - 1) * plane,
-                  zp = z < nx - 1 ? c + plane : c - (nx - 1) * plane;
-    const R cc = C[c];
-    const R lap = C[xm] + C[xp] + C[ym] + C[yp] + C[zm] + C[zp];
-    P[c] = km * lap + ka * cc + beta * P[c];
-    F[c] += kf * cc;
-}
-
 // deposit adjoint at x: m_bar += sum_c W_c Mbar_c; Xd = m sum_c dW_c/dx Mbar_c
 // (CIC weights of rm_p2mesh.cu:191-216; derivative zero where u is clamped)
 __device__ __forceinline__ void cic_axis_d(double x, double dmin, double inv_dx, int nx, int& i0,
@@ -345,20 +323,8 @@ void backward_step(rrg_pm_adjoint* P, const void* xn1, const void* phin1, cudaSt
     RRG_CUDA(cudaMemsetAsync(P->F.p, 0, P->F.bytes, s));
     R beta = R(1);
     for (int k = 0; k < P->substeps; ++k) {
-        // FP32: the float4 stencil (x +- 1 by shuffles, z from a register pipeline)
-        const bool x4 = sizeof(R) == 4 &&
-                        launch_wave_adjoint_step(P->grid.nx, static_cast<const float*>(P->Cb.p),
-                                                 static_cast<float*>(P->Pb.p),
-                                                 static_cast<float*>(P->F.p), P->wc.K_MAIN,
-                                                 P->wc.K_ACTUAL, static_cast<double>(beta),
-                                                 P->wc.K_F, s);
-        if (!x4) {
-            wave_adjoint_kernel<R><<<bg, 256, 0, s>>>(
-                P->grid.nx, static_cast<const R*>(P->Cb.p), static_cast<R*>(P->Pb.p),
-                static_cast<R*>(P->F.p), static_cast<R>(P->wc.K_MAIN),
-                static_cast<R>(P->wc.K_ACTUAL), beta, static_cast<R>(P->wc.K_F));
-            RRG_LAUNCHED();
-        }
+        launch_wave_adjoint_step(P->prec, P->grid.nx, P->Cb.p, P->Pb.p, P->F.p, P->wc.K_MAIN,
+                                 P->wc.K_ACTUAL, static_cast<double>(beta), P->wc.K_F, s);
         std::swap(P->Cb.p, P->Pb.p);  // the new current cotangent; old C becomes P / K_O
         beta = static_cast<R>(P->wc.K_OLD);
     }

@@ -66,7 +66,7 @@
 // first. Every wait is bounded; one that runs out sets the error word and the block leaves (the
 // step's results are then invalid), and later launches return at once until the host, which
 // turns the word into an error, clears the sync memory. The arithmetic is that of
-// wave_source_kernel<float>, wave_periodic_x4_kernel and gradient_x4_kernel, expression for
+// wave_source_kernel<float>, wave_periodic_vec_kernel and gradient_x4_kernel, expression for
 // expression, so the results are the same bits.
 #include <algorithm>
 #include <cstdlib>
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kThreads, 2) wave_solve_kernel(const SolveArgs
     if constexpr (FULL) {
         if (a.maxbits == nullptr) return;
         // the last substep's max |dphi| and max |phi|, differences in FP64 as
-        // wave_periodic_x4_kernel takes them
+        // wave_periodic_vec_kernel takes them
         double dmax = 0.0;
         float amax = 0.f;
 #pragma unroll
