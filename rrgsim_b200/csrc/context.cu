@@ -336,22 +336,31 @@ bool solve_step_fused(rrg_ctx* c, const WaveCoef& w, int iterations, bool store_
         float* d[2] = {a4, a4 + nc};
         float* g = a4 + 2 * nc;
         float* phi0 = c->phi[c->phi_cur].as<float>();
-        launch_wave_inc_prep(nx, c->mg[c->mg_cur].as<unsigned long long>(),
+        // the grids of the persistent kernels keep one launch per stage (RRG_WAVE_PERSIST=0);
+        // elsewhere the preparation takes the first substep along and the last one the finish
+        // (from 23 launches a step to 21, and two passes less over the increments)
+        const bool staged = nx == 32 || nx == 64 || nx == 128;
+        const bool first = !staged && iterations >= 2;
+        launch_wave_inc_prep(nx, first, c->mg[c->mg_cur].as<unsigned long long>(),
                              c->mg[1 - c->mg_cur].as<unsigned long long>(), c->shift_s,
                              c->grid.dx, c->rho_mean, phi0, c->phi[1 - c->phi_cur].as<float>(),
                              w, g, d[0], d[1], store_src ? c->src.as<float>() : nullptr,
                              c->stream);
         WaveCoef wi = w;
         wi.K_F = 1.0;
-        int cur = 0;
-        for (int k = 0; k < iterations; ++k) {
+        int cur = first ? 1 : 0;
+        for (int k = first ? 1 : 0; k < (staged ? iterations : iterations - 1); ++k) {
             launch_wave_step(c->prec, nx, d[cur], d[1 - cur], g, wi, nullptr, c->stream);
             cur = 1 - cur;
         }
         // final level into phi[phi_cur ^ (iterations & 1)], the one before into the other
         const int fin = c->phi_cur ^ (iterations & 1);
-        launch_wave_inc_finish(nx, phi0, d[cur], d[1 - cur], c->phi[fin].as<float>(),
-                               c->phi[1 - fin].as<float>(), c->stream);
+        if (staged)
+            launch_wave_inc_finish(nx, phi0, d[cur], d[1 - cur], c->phi[fin].as<float>(),
+                                   c->phi[1 - fin].as<float>(), c->stream);
+        else
+            launch_wave_inc_last(nx, d[cur], d[1 - cur], g, phi0, c->phi[fin].as<float>(),
+                                 c->phi[1 - fin].as<float>(), w, c->stream);
         gradient_after(c, fin);
     }
     if (iterations % 2 == 1) c->phi_cur = 1 - c->phi_cur;

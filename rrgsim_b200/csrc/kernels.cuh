@@ -215,15 +215,20 @@ __device__ __forceinline__ float4 f4_add(const float4 a, const float4 b) {
 }
 
 // The incremental solve's preparation, one streaming launch over the grid: g and
-// d_old = phi_prev - phi0 per cell, d = 0 (unless null), the plain FP32 source into src (unless
-// null), the next deposit target mg_zero cleared (unless null). One launch per substep (where
-// the persistent kernels do not apply, and RRG_WAVE_PERSIST=0) then runs launch_wave_step on
-// (d, d_old, g) with K_F = 1, and finish writes phi0 + d_final and
-// phi0 + d_before into fin and prv (either may be phi0 itself). FP32 grids, periodic, uniform.
-void launch_wave_inc_prep(int nx, const unsigned long long* mg, unsigned long long* mg_zero,
-                          int shift_s, double dx, double rho_sub, const float* phi0,
-                          const float* phi_prev, const WaveCoef& w, float* g, float* d,
-                          float* d_old, float* src, cudaStream_t s);
+// d_old = phi_prev - phi0 per cell, d = 0, the plain FP32 source into src (unless null), the next
+// deposit target mg_zero cleared (unless null). One launch per substep (where the persistent
+// kernels do not apply, and RRG_WAVE_PERSIST=0) then runs launch_wave_step on (d, d_old, g) with
+// K_F = 1, and finish writes phi0 + d_final and phi0 + d_before into fin and prv (either may be
+// phi0 itself). FP32 grids, periodic, uniform.
+// first: the first substep as well (d_old then holds level 1 of the increments, d level 0).
+void launch_wave_inc_prep(int nx, bool first, const unsigned long long* mg,
+                          unsigned long long* mg_zero, int shift_s, double dx, double rho_sub,
+                          const float* phi0, const float* phi_prev, const WaveCoef& w, float* g,
+                          float* d, float* d_old, float* src, cudaStream_t s);
+// The last substep and the finish in one: fin = phi0 + d_new, prv = phi0 + d.
+void launch_wave_inc_last(int nx, const float* d, const float* d_old, const float* g,
+                          const float* phi0, float* fin, float* prv, const WaveCoef& w,
+                          cudaStream_t s);
 void launch_wave_inc_finish(int nx, const float* phi0, const float* d_fin, const float* d_prv,
                             float* fin, float* prv, cudaStream_t s);
 

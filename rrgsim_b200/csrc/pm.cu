@@ -248,35 +248,64 @@ __global__ void wave_source_kernel(int64_t ncells, unsigned long long* __restric
     }
 }
 
-// The incremental solve's preparation and finish (wave_inc_source): one thread per cell,
-// periodic neighbours.
-__global__ void wave_inc_prep_kernel(int nx, const unsigned long long* __restrict__ mg,
-                                     unsigned long long* __restrict__ mg_zero,
-                                     double inv_scale, double inv_dx3, double rho_sub,
-                                     const float* __restrict__ phi0,
-                                     const float* __restrict__ phi_prev, double kf, double km,
-                                     double kao, float* __restrict__ g, float* __restrict__ d,
-                                     float* __restrict__ d_old, float* __restrict__ src) {
-    const int64_t nc = static_cast<int64_t>(nx) * nx * nx;
-    const int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (c >= nc) return;
-    const int x = static_cast<int>(c % nx), y = static_cast<int>((c / nx) % nx),
-              z = static_cast<int>(c / (static_cast<int64_t>(nx) * nx));
-    const int64_t row = c - x, plane = static_cast<int64_t>(nx) * nx;
-    const int64_t cz = c - static_cast<int64_t>(z) * plane;
-    const float p = phi0[c];
-    const float l = phi0[row + (x == 0 ? nx - 1 : x - 1)];
-    const float r = phi0[row + (x == nx - 1 ? 0 : x + 1)];
-    const float ym = phi0[c + (y == 0 ? (nx - 1) * nx : -nx)];
-    const float yp = phi0[c + (y == nx - 1 ? -(nx - 1) * nx : nx)];
-    const float zm = phi0[cz + (z == 0 ? nx - 1 : z - 1) * plane];
-    const float zp = phi0[cz + (z == nx - 1 ? 0 : z + 1) * plane];
-    const double sd = wave_source_value(mg[c], inv_scale, inv_dx3, rho_sub);
-    g[c] = wave_inc_source(sd, l, r, ym, yp, zm, zp, p, kf, km, kao);
-    if (d) d[c] = 0.f;
-    d_old[c] = __fsub_rn(phi_prev[c], p);
-    if (src) src[c] = static_cast<float>(sd);
-    if (mg_zero) mg_zero[c] = 0ull;
+// The incremental solve's preparation (wave_inc_source), V consecutive x-cells per thread.
+// FIRST: also the first substep, which needs no neighbours (the increments start at zero):
+// d_1 = K_OLD d_old + g, stored over d_old's place, with level 0 of the increments (zero) in d.
+// Bound: HBM at 256^3 (32 to 36 B per cell); below, the FP64 arithmetic of g.
+template <int V, bool FIRST>
+__global__ void __launch_bounds__(256) wave_inc_prep_kernel(
+    int nx, const unsigned long long* __restrict__ mg, unsigned long long* __restrict__ mg_zero,
+    double inv_scale, double inv_dx3, double rho_sub, const float* __restrict__ phi0,
+    const float* __restrict__ phi_prev, double kf, double km, double kao, float ko,
+    float* __restrict__ g, float* __restrict__ d, float* __restrict__ d_old,
+    float* __restrict__ src) {
+    using C = Cells<float, V>;
+    const int W = nx / V;
+    const int64_t u = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t units = static_cast<int64_t>(W) * nx * nx;
+    if (u >= units) return;
+    const int q = static_cast<int>(u % W);
+    const int64_t row = u / W;
+    const int y = static_cast<int>(row % nx), z = static_cast<int>(row / nx);
+    const int64_t plane = static_cast<int64_t>(nx) * nx;
+    const int64_t c = row * nx + q * V;
+    auto cells = [&](int64_t at) { return *reinterpret_cast<const C*>(phi0 + at); };
+    const C p = cells(c), pp = *reinterpret_cast<const C*>(phi_prev + c);
+    const float l = phi0[row * nx + (q == 0 ? nx : q * V) - 1];
+    const float r = phi0[row * nx + (q == W - 1 ? 0 : q * V + V)];
+    const C ym = cells(c + (y == 0 ? (nx - 1) * nx : -nx));
+    const C yp = cells(c + (y == nx - 1 ? -(nx - 1) * nx : nx));
+    const C zm = cells(c + (z == 0 ? (nx - 1) * plane : -plane));
+    const C zp = cells(c + (z == nx - 1 ? -(nx - 1) * plane : plane));
+    unsigned long long q8[V];
+#pragma unroll
+    for (int i = 0; i < V; i += (V > 1 ? 2 : 1)) {
+        if constexpr (V > 1) {
+            const ulonglong2 m = *reinterpret_cast<const ulonglong2*>(mg + c + i);
+            q8[i] = m.x;
+            q8[i + 1] = m.y;
+            if (mg_zero) *reinterpret_cast<ulonglong2*>(mg_zero + c + i) = make_ulonglong2(0ull, 0ull);
+        } else {
+            q8[i] = mg[c];
+            if (mg_zero) mg_zero[c] = 0ull;
+        }
+    }
+    C og, od, oo, os;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const double sd = wave_source_value(q8[i], inv_scale, inv_dx3, rho_sub);
+        og.v[i] = wave_inc_source(sd, i == 0 ? l : p.v[i > 0 ? i - 1 : 0],
+                                  i == V - 1 ? r : p.v[i < V - 1 ? i + 1 : 0], ym.v[i], yp.v[i],
+                                  zm.v[i], zp.v[i], p.v[i], kf, km, kao);
+        const float before = __fsub_rn(pp.v[i], p.v[i]);
+        od.v[i] = 0.f;
+        oo.v[i] = FIRST ? __fmaf_rn(og.v[i], 1.f, __fmaf_rn(before, ko, 0.f)) : before;
+        os.v[i] = static_cast<float>(sd);
+    }
+    *reinterpret_cast<C*>(g + c) = og;
+    *reinterpret_cast<C*>(d + c) = od;
+    *reinterpret_cast<C*>(d_old + c) = oo;
+    if (src) *reinterpret_cast<C*>(src + c) = os;
 }
 
 __global__ void wave_inc_finish_kernel(int64_t nc, const float* phi0, const float* d_fin,
@@ -399,17 +428,25 @@ __device__ __forceinline__ void block_max_to(double dmax, double amax, int tid,
 // Successive substeps are launched with programmatic dependence: a block's indices are ready when
 // the substep before it ends (no load is ahead of the wait).
 //
-// Bound: launch and L2 latency up to ~100^3 (2.1 us a substep at 64^3), L2 bandwidth to ~160^3,
-// HBM beyond (256^3: 268 MB in 46 us, 0.89 of the copy peak). Per substep in a graph on B200, us,
-// one-cell columns (FP64, and rows that do not tile a warp) or float4 rows without programmatic
-// launches -> here: FP32 33^3 2.61 -> 2.05, 64^3 2.39 -> 2.13, 96^3 4.68 -> 3.05, 100^3 7.21 ->
-// 3.16, 128^3 4.59 -> 4.35, 160^3 13.2 -> 8.5, 200^3 34.5 -> 20.4; FP64 64^3 2.99 -> 2.80, 100^3
-// 9.90 -> 4.69, 128^3 9.89 -> 8.19.
-template <typename R, int V, int ZC, bool CHECK, bool ADJ>
-__global__ void __launch_bounds__(kVecThreads, 8) wave_periodic_vec_kernel(
+// Bound: launch and L2 latency up to ~100^3, L2 bandwidth to ~160^3, HBM beyond (256^3: 268 MB in
+// 38.9 us, 1.05 of the copy peak, part of it L2 hits). Per substep in a graph on B200, us: one-cell
+// columns (FP64, and rows that do not tile a warp) or float4 rows, chunks of up to 8 planes, normal
+// launches -> vectors everywhere and programmatic launches -> loads a plane ahead, 2 planes: FP32
+// 33^3 2.61 -> 2.05 -> 1.5, 64^3 2.39 -> 2.13 -> 1.72, 96^3 4.68 -> 3.05 -> 2.64, 128^3 4.59 -> 4.35
+// -> 4.5, 160^3 13.2 -> 8.5 -> 7.3, 256^3 48.1 -> 45.6 -> 38.9; FP64 64^3 2.99 -> 2.80 -> 2.13,
+// 128^3 9.89 -> 8.19 -> 7.37.
+// LAST: the last substep of an incremental solve (wave_inc_source; phi and phi_old the increments
+// d and d_old, src their source g): instead of d_new, the levels in full, phi0 + d_new to fin and
+// phi0 + d to prv (either may be phi0: a cell's phi0 is read by its own thread alone).
+enum VecMode { VEC_STEP, VEC_ADJ, VEC_LAST };
+template <typename R, int V, int ZC, bool CHECK, VecMode MODE>
+__global__ void __launch_bounds__(kVecThreads, 6) wave_periodic_vec_kernel(
     const R* phi, R* phi_old, const R* src, const WaveDev w,
-    unsigned long long* __restrict__ maxbits, R* fadj) {
+    unsigned long long* __restrict__ maxbits, R* fadj, const R* phi0, R* fin, R* prv) {
     using C = Cells<R, V>;
+    constexpr bool ADJ = MODE == VEC_ADJ;
+    // the first plane's rows are requested with the column, the next plane's before a plane is
+    // computed: one round trip to L2 instead of one per plane
     const int nx = w.nx;
     const int W = nx / V;        // V-cell units per row
     const int plane = nx * nx;
@@ -441,35 +478,50 @@ __global__ void __launch_bounds__(kVecThreads, 8) wave_periodic_vec_kernel(
         pv[k] = load_cells<R, V>(phi + (at + z * plane));
     }
     double dmax = 0.0, amax = 0.0;
+    struct Plane {
+        C ym, yp, po, other;  // other: the source, or F
+        R l, r;
+    };
+    auto fetch = [&](int z) -> Plane {
+        Plane p{};
+        if (valid && z < nx) {
+            const int zb = z * plane;
+            if (lload) p.l = load_cells<R, 1>(phi + (xl + zb)).v[0];
+            if (rload) p.r = load_cells<R, 1>(phi + (xr + zb)).v[0];
+            p.ym = load_cells<R, V>(phi + (aym + zb));
+            p.yp = load_cells<R, V>(phi + (ayp + zb));
+            p.po = load_cells<R, V>(phi_old + (at + zb));
+            if constexpr (ADJ) p.other = load_cells<R, V>(fadj + (at + zb));
+            else p.other = load_cells<R, V>(src + (at + zb));
+        }
+        return p;
+    };
+    Plane next = fetch(z0);
 #pragma unroll
     for (int k = 0; k < ZC; ++k) {
         const int z = z0 + k;
         if (z >= nx) break;
+        Plane p = next;
+        if (k + 1 < ZC) next = fetch(z + 1);
         const C c = pv[k + 1];
         R lft = __shfl_sync(0xffffffffu, c.v[V - 1], lsrc & 31);
         R rgt = __shfl_sync(0xffffffffu, c.v[0], rsrc & 31);
+        if (lload) lft = p.l;
+        if (rload) rgt = p.r;
         if (valid) {
             const int zb = z * plane;
-            if (lload) lft = load_cells<R, 1>(phi + (xl + zb)).v[0];
-            if (rload) rgt = load_cells<R, 1>(phi + (xr + zb)).v[0];
-            const C ym = load_cells<R, V>(phi + (aym + zb));
-            const C yp = load_cells<R, V>(phi + (ayp + zb));
-            const C po = load_cells<R, V>(phi_old + (at + zb));
-            C other;  // the source, or F
-            if constexpr (ADJ) other = load_cells<R, V>(fadj + (at + zb));
-            else other = load_cells<R, V>(src + (at + zb));
             C out;
 #pragma unroll
             for (int i = 0; i < V; ++i) {
                 const R l = i == 0 ? lft : c.v[i > 0 ? i - 1 : 0];
                 const R r = i == V - 1 ? rgt : c.v[i < V - 1 ? i + 1 : 0];
-                const R t = wave_cell_adj(l, r, ym.v[i], yp.v[i], pv[k].v[i], pv[k + 2].v[i],
-                                          c.v[i], po.v[i], km, ka, ko);
+                const R t = wave_cell_adj(l, r, p.ym.v[i], p.yp.v[i], pv[k].v[i], pv[k + 2].v[i],
+                                          c.v[i], p.po.v[i], km, ka, ko);
                 if constexpr (ADJ) {
                     out.v[i] = t;
-                    other.v[i] = rfma(kf, c.v[i], other.v[i]);
+                    p.other.v[i] = rfma(kf, c.v[i], p.other.v[i]);
                 } else {
-                    out.v[i] = rfma(other.v[i], kf, t);
+                    out.v[i] = rfma(p.other.v[i], kf, t);
                 }
                 if constexpr (CHECK) {
                     // differences in FP64
@@ -477,8 +529,20 @@ __global__ void __launch_bounds__(kVecThreads, 8) wave_periodic_vec_kernel(
                     amax = fmax(amax, fabs(double(out.v[i])));
                 }
             }
-            *reinterpret_cast<C*>(phi_old + (at + zb)) = out;
-            if constexpr (ADJ) *reinterpret_cast<C*>(fadj + (at + zb)) = other;
+            if constexpr (MODE == VEC_LAST) {
+                const C p0 = load_cells<R, V>(phi0 + (at + zb));
+                C full, before;
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    full.v[i] = radd(p0.v[i], out.v[i]);
+                    before.v[i] = radd(p0.v[i], c.v[i]);
+                }
+                *reinterpret_cast<C*>(fin + (at + zb)) = full;
+                *reinterpret_cast<C*>(prv + (at + zb)) = before;
+            } else {
+                *reinterpret_cast<C*>(phi_old + (at + zb)) = out;
+            }
+            if constexpr (ADJ) *reinterpret_cast<C*>(fadj + (at + zb)) = p.other;
         }
     }
     if constexpr (CHECK) block_max_to(dmax, amax, tid, maxbits);
@@ -998,15 +1062,28 @@ void launch_wave_source(int prec, int nx, const unsigned long long* mgrid, int s
     RRG_LAUNCHED();
 }
 
-void launch_wave_inc_prep(int nx, const unsigned long long* mg, unsigned long long* mg_zero,
-                          int shift_s, double dx, double rho_sub, const float* phi0,
-                          const float* phi_prev, const WaveCoef& w, float* g, float* d,
-                          float* d_old, float* src, cudaStream_t s) {
-    const int64_t nc = static_cast<int64_t>(nx) * nx * nx;
-    wave_inc_prep_kernel<<<div_up(nc, 256), 256, 0, s>>>(
-        nx, mg, mg_zero, ldexp(1.0, -shift_s), 1.0 / (dx * dx * dx), rho_sub, phi0, phi_prev,
-        w.K_F, w.K_MAIN, w.K_ACTUAL + w.K_OLD - 1.0, g, d, d_old, src);
-    RRG_LAUNCHED();
+void launch_wave_inc_prep(int nx, bool first, const unsigned long long* mg,
+                          unsigned long long* mg_zero, int shift_s, double dx, double rho_sub,
+                          const float* phi0, const float* phi_prev, const WaveCoef& w, float* g,
+                          float* d, float* d_old, float* src, cudaStream_t s) {
+    const int V = nx % 4 == 0 ? 4 : nx % 2 == 0 ? 2 : 1;
+    const int64_t units = static_cast<int64_t>(nx / V) * nx * nx;
+    auto go = [&](auto* kernel) {
+        kernel<<<div_up(units, 256), 256, 0, s>>>(
+            nx, mg, mg_zero, ldexp(1.0, -shift_s), 1.0 / (dx * dx * dx), rho_sub, phi0, phi_prev,
+            w.K_F, w.K_MAIN, w.K_ACTUAL + w.K_OLD - 1.0, static_cast<float>(w.K_OLD), g, d, d_old,
+            src);
+        RRG_LAUNCHED();
+    };
+    if (first) {
+        if (V == 4) go(wave_inc_prep_kernel<4, true>);
+        else if (V == 2) go(wave_inc_prep_kernel<2, true>);
+        else go(wave_inc_prep_kernel<1, true>);
+    } else {
+        if (V == 4) go(wave_inc_prep_kernel<4, false>);
+        else if (V == 2) go(wave_inc_prep_kernel<2, false>);
+        else go(wave_inc_prep_kernel<1, false>);
+    }
 }
 
 void launch_wave_inc_finish(int nx, const float* phi0, const float* d_fin, const float* d_prv,
@@ -1024,80 +1101,98 @@ int cells_per_thread(int nx, bool f64) {
     return nx % 2 == 0 ? 2 : 1;
 }
 
-template <typename R, int V, int ZC, bool ADJ>
-void launch_vec(const WaveDev& w, const R* phi, R* old, const R* src, R* f,
-                unsigned long long* maxbits, cudaStream_t s) {
+struct VecArgs {
+    const void* phi;
+    void* old;
+    const void* src;
+    void* f = nullptr;                      // VEC_ADJ
+    unsigned long long* maxbits = nullptr;  // VEC_STEP
+    const void* phi0 = nullptr;             // VEC_LAST
+    void* fin = nullptr;
+    void* prv = nullptr;
+};
+
+template <typename R, int V, int ZC, VecMode MODE>
+void launch_vec(const WaveDev& w, const VecArgs& a, cudaStream_t s) {
     const dim3 grid(div_up(static_cast<int64_t>(w.nx / V) * w.nx, kVecThreads), div_up(w.nx, ZC));
-    if constexpr (!ADJ) {
-        if (maxbits) {
-            launch_pdl(wave_periodic_vec_kernel<R, V, ZC, true, false>, grid, kVecThreads, 0, s, phi,
-                       old, src, w, maxbits, f);
-            RRG_LAUNCHED();
+    auto go = [&](auto* kernel) {
+        launch_pdl(kernel, grid, kVecThreads, 0, s, static_cast<const R*>(a.phi),
+                   static_cast<R*>(a.old), static_cast<const R*>(a.src), w, a.maxbits,
+                   static_cast<R*>(a.f), static_cast<const R*>(a.phi0), static_cast<R*>(a.fin),
+                   static_cast<R*>(a.prv));
+        RRG_LAUNCHED();
+    };
+    if constexpr (MODE == VEC_STEP) {
+        if (a.maxbits) {
+            go(wave_periodic_vec_kernel<R, V, ZC, true, MODE>);
             return;
         }
     }
-    launch_pdl(wave_periodic_vec_kernel<R, V, ZC, false, ADJ>, grid, kVecThreads, 0, s, phi, old, src,
-               w, maxbits, f);
-    RRG_LAUNCHED();
+    go(wave_periodic_vec_kernel<R, V, ZC, false, MODE>);
 }
 
-// z-chunk: the longest of 8, 4, 2 planes that still gives four 128-thread blocks per SM (at
-// 128^3 FP32 that is 4, measured fastest inside the PM step; RRG_WAVE_ZC fixes it, for sweeps)
-template <typename R, int V, bool ADJ>
-void launch_vec_z(const WaveDev& w, const R* phi, R* old, const R* src, R* f,
-                  unsigned long long* maxbits, cudaStream_t s) {
-    static const int fixed = [] {
-        const char* e = std::getenv("RRG_WAVE_ZC");
-        return e ? std::atoi(e) : 0;
-    }();
+// z-chunk: 2 planes (the most loads in flight, the shortest chain), or 4 where those blocks fill one
+// wave of six per SM and those of 2 planes take a second. Measured with 2 / 4 / 8 planes, us per
+// substep: FP32 64^3 1.72 / 2.28 / 4.59, 96^3 2.64 / 3.09 / 5.38, 112^3 (0.79 of a wave)
+// 3.71 / 3.62 / 6.83, 256^3 38.9 / 40.4 / 46.3; FP64 96^3 (0.97) 4.16 / 3.72 / 8.27, 128^3
+// 7.37 / 7.80 / 9.72.
+template <typename R, int V, VecMode MODE>
+void launch_vec_z(const WaveDev& w, const VecArgs& a, cudaStream_t s) {
     int dev = 0;
     RRG_CUDA(cudaGetDevice(&dev));
-    const int sms = num_sms(dev);
+    const int64_t wave = 6ll * num_sms(dev);
     const int64_t rows = div_up(static_cast<int64_t>(w.nx / V) * w.nx, kVecThreads);
-    int z = 2;
-    for (int cand : {8, 4})
-        if (rows * div_up(w.nx, cand) >= 4 * sms) {
-            z = cand;
-            break;
-        }
-    if (fixed == 2 || fixed == 4 || fixed == 8) z = fixed;
-    if (z == 8) launch_vec<R, V, 8, ADJ>(w, phi, old, src, f, maxbits, s);
-    else if (z == 4) launch_vec<R, V, 4, ADJ>(w, phi, old, src, f, maxbits, s);
-    else launch_vec<R, V, 2, ADJ>(w, phi, old, src, f, maxbits, s);
+    const int64_t b2 = rows * div_up(w.nx, 2), b4 = rows * div_up(w.nx, 4);
+    if (b2 > wave && b4 <= wave && 4 * b4 >= 3 * wave) launch_vec<R, V, 4, MODE>(w, a, s);
+    else launch_vec<R, V, 2, MODE>(w, a, s);
 }
 
-template <bool ADJ>
-void launch_vec_any(int prec, const WaveDev& w, const void* phi, void* old, const void* src,
-                    void* f, unsigned long long* maxbits, cudaStream_t s) {
+template <VecMode MODE>
+void launch_vec_any(int prec, const WaveDev& w, const VecArgs& a, cudaStream_t s) {
     const bool f64 = prec == RRG_PREC_FP64;
     const int V = cells_per_thread(w.nx, f64);
-#define RRG_VEC(R, VV)                                                                        \
-    launch_vec_z<R, VV, ADJ>(w, static_cast<const R*>(phi), static_cast<R*>(old),             \
-                             static_cast<const R*>(src), static_cast<R*>(f), maxbits, s)
     if (f64) {
-        if (V == 2) RRG_VEC(double, 2);
-        else RRG_VEC(double, 1);
+        if constexpr (MODE != VEC_LAST) {  // (the incremental solves are FP32)
+            if (V == 2) launch_vec_z<double, 2, MODE>(w, a, s);
+            else launch_vec_z<double, 1, MODE>(w, a, s);
+        }
     } else {
-        if (V == 4) RRG_VEC(float, 4);
-        else if (V == 2) RRG_VEC(float, 2);
-        else RRG_VEC(float, 1);
+        if (V == 4) launch_vec_z<float, 4, MODE>(w, a, s);
+        else if (V == 2) launch_vec_z<float, 2, MODE>(w, a, s);
+        else launch_vec_z<float, 1, MODE>(w, a, s);
     }
-#undef RRG_VEC
 }
 
-}  // namespace
-
-void launch_wave_adjoint_step(int prec, int nx, const void* C, void* P, void* F, double km,
-                              double ka, double beta, double kf, cudaStream_t s) {
+WaveDev periodic_dev(int nx, double km, double ka, double ko, double kf) {
     WaveDev w{};
     w.nx = nx;
     w.uniform = 1;
     w.bc = RRG_BC_PERIODIC;
     w.K_MAIN = km;
     w.K_ACTUAL = ka;
-    w.K_OLD = beta;
+    w.K_OLD = ko;
     w.K_F = kf;
-    launch_vec_any<true>(prec, w, C, P, nullptr, F, nullptr, s);
+    return w;
+}
+
+}  // namespace
+
+void launch_wave_inc_last(int nx, const float* d, const float* d_old, const float* g,
+                          const float* phi0, float* fin, float* prv, const WaveCoef& w,
+                          cudaStream_t s) {
+    VecArgs a{d, const_cast<float*>(d_old), g};
+    a.phi0 = phi0;
+    a.fin = fin;
+    a.prv = prv;
+    launch_vec_any<VEC_LAST>(RRG_PREC_FP32,
+                             periodic_dev(nx, w.K_MAIN, w.K_ACTUAL, w.K_OLD, 1.0), a, s);
+}
+
+void launch_wave_adjoint_step(int prec, int nx, const void* C, void* P, void* F, double km,
+                              double ka, double beta, double kf, cudaStream_t s) {
+    VecArgs a{C, P, nullptr};
+    a.f = F;
+    launch_vec_any<VEC_ADJ>(prec, periodic_dev(nx, km, ka, beta, kf), a, s);
 }
 
 void launch_wave_step(int prec, int nx, const void* phi, void* phi_old_inout, const void* src,
@@ -1124,7 +1219,9 @@ void launch_wave_step(int prec, int nx, const void* phi, void* phi_old_inout, co
     w.r_min = c.r_min;
     const bool check = maxbits != nullptr;
     if (w.uniform) {
-        launch_vec_any<false>(prec, w, phi, phi_old_inout, src, nullptr, maxbits, s);
+        VecArgs a{phi, phi_old_inout, src};
+        a.maxbits = maxbits;
+        launch_vec_any<VEC_STEP>(prec, w, a, s);
         return;
     }
     const int gx = div_up(nx, kTX), gy = div_up(nx, kTY);
