@@ -43,18 +43,29 @@ __device__ __forceinline__ void interp_axis_w(double x, double dmin, double dx, 
     i1 = max(0, min(a + 1, nx - 1));
 }
 
-// interp adjoint: gbar += T(x)^T A (atomics, when gbar != nullptr; gbar holds 4 values per
-// cell, the fourth unused); X = sum dW/dx (g . A)
+// interp adjoint with the correct adjoint before it: with A' = A + h V (the correction
+// v' = (u + dt a) / 2; V null: A alone), gbar += T(x)^T A' (atomics, when gbar != nullptr; gbar
+// holds 4 values per cell, the fourth unused); X = sum dW/dx (g . A')
 template <typename R>
 __global__ void __launch_bounds__(256) interp_adjoint_kernel(int64_t n, const V4<R>* __restrict__ posm,
                                                              GridDev g, const V4<R>* __restrict__ acc4,
                                                              const V4<R>* __restrict__ A,
+                                                             const V4<R>* __restrict__ V, R h,
                                                              R* __restrict__ gbar,
                                                              V4<R>* __restrict__ X) {
     const int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const V4<R> q = posm[p];
-    const V4<R> a = A[p];
+    const bool active = p < n;
+    V4<R> q = v4<R>(0, 0, 0, 0), a = v4<R>(0, 0, 0, 0);
+    if (active) {
+        q = posm[p];
+        a = A[p];
+        if (V) {
+            const V4<R> v = V[p];
+            a.x += h * v.x;
+            a.y += h * v.y;
+            a.z += h * v.z;
+        }
+    }
     int ii[2], jj[2], kk[2];
     double wx, wy, wz;
     interp_axis_w(q.x, g.domain_min, g.dx, g.nx, ii[0], ii[1], wx);
@@ -78,20 +89,57 @@ __global__ void __launch_bounds__(256) interp_adjoint_kernel(int64_t n, const V4
                 gx += dws[i] * wys[j] * wzs[k] * s;
                 gy += wxs[i] * dws[j] * wzs[k] * s;
                 gz += wxs[i] * wys[j] * dws[k] * s;
-                if (gbar) {
-                    const R W = wxs[i] * wys[j] * wzs[k];
-                    if constexpr (sizeof(R) == 4) {
-                        // one 16-byte vector atomic per corner instead of three scalar ones
-                        atomicAdd(reinterpret_cast<float4*>(gbar) + c,
-                                  make_float4(W * a.x, W * a.y, W * a.z, 0.f));
-                    } else {
-                        atomicAdd(gbar + 4 * c, W * a.x);
-                        atomicAdd(gbar + 4 * c + 1, W * a.y);
-                        atomicAdd(gbar + 4 * c + 2, W * a.z);
+            }
+    if (active) X[p] = v4<R>(gx, gy, gz, R(0));
+    if (!gbar) return;
+    // Lanes of the same eight corners that sit next to each other (particles sorted by cell) are
+    // summed by a segmented scan and their last lane adds the sums: the atomics of a dense cell
+    // otherwise queue on its corners (262,144 sorted disk particles on 64^3: 67 us with one set
+    // of atomics per particle, 41 unsorted). A warp of many runs adds lane by lane.
+    auto side = [&](const int e[2]) {
+        return e[0] != e[1] ? e[0] + 1 : (e[0] == 0 ? 0 : g.nx);
+    };
+    const int n1 = g.nx + 1;  // (n1^3 < 2^31)
+    const int key = active ? side(ii) + n1 * (side(jj) + n1 * side(kk)) : -1;
+    const int lane = threadIdx.x & 31;
+    const int below = __shfl_up_sync(0xffffffffu, key, 1);
+    const int above = __shfl_down_sync(0xffffffffu, key, 1);
+    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || below != key);
+    const bool scan = __popc(heads) < 24;  // warp-uniform
+    const bool tail = !scan || lane == 31 || above != key;
+    const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));  // the run's first lane
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const R w = wxs[i] * wys[j] * wzs[k];
+                R vx = w * a.x, vy = w * a.y, vz = w * a.z;
+                if (scan) {
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const R tx = __shfl_up_sync(0xffffffffu, vx, d);
+                        const R ty = __shfl_up_sync(0xffffffffu, vy, d);
+                        const R tz = __shfl_up_sync(0xffffffffu, vz, d);
+                        if (lane - d >= first) {
+                            vx += tx;
+                            vy += ty;
+                            vz += tz;
+                        }
                     }
                 }
+                if (!tail || !active) continue;
+                const int64_t c = kk[k] * nx * nx + jj[j] * nx + ii[i];
+                if constexpr (sizeof(R) == 4) {
+                    // one 16-byte vector atomic per corner instead of three scalar ones
+                    atomicAdd(reinterpret_cast<float4*>(gbar) + c, make_float4(vx, vy, vz, 0.f));
+                } else {
+                    atomicAdd(gbar + 4 * c, vx);
+                    atomicAdd(gbar + 4 * c + 1, vy);
+                    atomicAdd(gbar + 4 * c + 2, vz);
+                }
             }
-    X[p] = v4<R>(gx, gy, gz, R(0));
 }
 
 // gradient adjoint: phi += -1/dx D^T gbar (D: central inside, one-sided on the faces)
@@ -140,10 +188,13 @@ __device__ __forceinline__ void cic_axis_d(double x, double dmin, double inv_dx,
     w1 = f;
 }
 
+// and the predict adjoint after it, with U = V / 2: Xt = X + Xi + Xd (w: m_bar accumulates);
+// U += dt/2 Xt; V = 2 U; A = dt U; X = Xt
 template <typename R>
-__global__ void __launch_bounds__(256) deposit_adjoint_kernel(int64_t n, const V4<R>* __restrict__ posm,
-                                                              GridDev g, const R* __restrict__ F,
-                                                              R mscale, V4<R>* __restrict__ Xd) {
+__global__ void __launch_bounds__(256) deposit_predict_adjoint_kernel(
+    int64_t n, const V4<R>* __restrict__ posm, GridDev g, const R* __restrict__ F, R mscale,
+    V4<R>* __restrict__ X, const V4<R>* __restrict__ Xi, V4<R>* __restrict__ V,
+    V4<R>* __restrict__ A, R dt) {
     const int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (p >= n) return;
     const V4<R> q = posm[p];
@@ -169,39 +220,12 @@ __global__ void __launch_bounds__(256) deposit_adjoint_kernel(int64_t n, const V
                 gz += wx[i] * wy[j] * sgn[k] * duz * Mb;
             }
     const double m = q.w;
-    Xd[p] = v4<R>(static_cast<R>(m * gx), static_cast<R>(m * gy), static_cast<R>(m * gz),
-                  static_cast<R>(mb));
-}
-
-// correct adjoint: U = V / 2, A += dt/2 V
-template <typename R>
-__global__ void correct_adjoint_kernel(int64_t n, const V4<R>* __restrict__ V, V4<R>* __restrict__ A,
-                                       V4<R>* __restrict__ U, R dt) {
-    const int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const V4<R> v = V[p];
-    V4<R> a = A[p];
+    const V4<R> x = X[p], xi = Xi[p], v = V[p];
+    const R tx = x.x + xi.x + static_cast<R>(m * gx), ty = x.y + xi.y + static_cast<R>(m * gy),
+            tz = x.z + xi.z + static_cast<R>(m * gz);
     const R h = dt * R(0.5);
-    a.x += h * v.x;
-    a.y += h * v.y;
-    a.z += h * v.z;
-    A[p] = a;
-    U[p] = v4<R>(R(0.5) * v.x, R(0.5) * v.y, R(0.5) * v.z, R(0));
-}
-
-// predict adjoint: Xt = X + Xi + Xd (w: m_bar accumulates Xd.w); U += dt/2 Xt; V = 2 U;
-// A = dt U; X = Xt
-template <typename R>
-__global__ void predict_adjoint_kernel(int64_t n, V4<R>* __restrict__ X, const V4<R>* __restrict__ Xi,
-                                       const V4<R>* __restrict__ Xd, const V4<R>* __restrict__ U,
-                                       V4<R>* __restrict__ V, V4<R>* __restrict__ A, R dt) {
-    const int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const V4<R> x = X[p], xi = Xi[p], xd = Xd[p], u = U[p];
-    const R tx = x.x + xi.x + xd.x, ty = x.y + xi.y + xd.y, tz = x.z + xi.z + xd.z;
-    const R h = dt * R(0.5);
-    const R ux = u.x + h * tx, uy = u.y + h * ty, uz = u.z + h * tz;
-    X[p] = v4<R>(tx, ty, tz, x.w + xd.w);
+    const R ux = R(0.5) * v.x + h * tx, uy = R(0.5) * v.y + h * ty, uz = R(0.5) * v.z + h * tz;
+    X[p] = v4<R>(tx, ty, tz, x.w + static_cast<R>(mb));
     V[p] = v4<R>(R(2) * ux, R(2) * uy, R(2) * uz, R(0));
     A[p] = v4<R>(dt * ux, dt * uy, dt * uz, R(0));
 }
@@ -218,10 +242,13 @@ __global__ void add_xyz_kernel(int64_t n, V4<R>* __restrict__ X, const V4<R>* __
     X[p] = x;
 }
 
+// out[i] = in[dest[i]]: particles back into the caller's order
 template <typename R>
-__global__ void scale_kernel(int64_t n, R* __restrict__ a, R s) {
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) a[i] *= s;
+__global__ void __launch_bounds__(256) gather_kernel(int64_t n, const uint32_t* __restrict__ dest,
+                                                     const V4<R>* __restrict__ in,
+                                                     V4<R>* __restrict__ out) {
+    const int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (p < n) out[p] = in[dest[p]];
 }
 
 struct PBuf {
@@ -268,7 +295,13 @@ struct rrg_pm_adjoint {
     PBuf x, v, a, u, mg, src, phi[2], acc4;
     PBuf ck_x, ck_v, ck_a, ck_phi;     // per checkpoint: x, v, a, phi_prev, phi_cur
     PBuf seg_x, seg_phi;               // per step of a segment: x_{n+1}, phi_cur_{n+1}
-    PBuf X, V, A, U, Xi, Xd, gbar, Cb, Pb, F;
+    PBuf X, V, A, Xi, gbar, Cb, Pb, F;
+    // The particles' order inside the object: sorted by the CIC cell of x0 (dest: a particle's
+    // slot), so that deposits, gathers and the field cotangent's scatter of a warp meet in few
+    // cells. Made by each forward pass, undone where states and gradients leave the object.
+    bool sort = false;
+    PBuf keys, dest, counts, offsets, cursor, temp;
+    size_t temp_bytes = 0;
     bool forward_done = false;
     std::string err;
 };
@@ -278,22 +311,54 @@ namespace {
 size_t pvb(const rrg_pm_adjoint* P) { return 4 * P->rsz * static_cast<size_t>(P->n); }
 size_t gvb(const rrg_pm_adjoint* P) { return P->rsz * static_cast<size_t>(P->nc); }
 
-// one PM step in place on (x, v, a, phi[0] = prev, phi[1] = cur)
+// one PM step in place on (x, v, a, phi[0] = prev, phi[1] = cur); mg is zero before and after
 void pm_step(rrg_pm_adjoint* P, cudaStream_t s) {
-    launch_predict(P->prec, P->n, P->x.p, nullptr, P->v.p, P->a.p, P->u.p, P->dt, s);
-    RRG_CUDA(cudaMemsetAsync(P->mg.p, 0, P->mg.bytes, s));
-    launch_cic_deposit(P->prec, P->n, P->x.p, nullptr, P->gdev, P->shift_s,
-                       static_cast<unsigned long long*>(P->mg.p), s);
+    PmParticleArgs a{};
+    a.prec = P->prec;
+    a.n = P->n;
+    a.posm = P->x.p;
+    a.vel = P->v.p;
+    a.acc = P->a.p;
+    a.u = P->u.p;
+    a.acc4 = P->acc4.p;
+    a.g = P->gdev;
+    a.shift_s = P->shift_s;
+    a.mgrid = static_cast<unsigned long long*>(P->mg.p);
+    a.dt = P->dt;
+    launch_pm_particles(a, PM_PREDICT_DEPOSIT, s);
     launch_wave_source(P->prec, P->grid.nx, static_cast<unsigned long long*>(P->mg.p), P->shift_s,
-                       P->grid.dx, P->rho_mean, 1.0, P->src.p, false, s);
+                       P->grid.dx, P->rho_mean, 1.0, P->src.p, true, s);
     for (int k = 0; k < P->substeps; ++k) {
         // phi[1] current, phi[0] previous: the new level overwrites phi[0], then roles swap
         launch_wave_step(P->prec, P->grid.nx, P->phi[1].p, P->phi[0].p, P->src.p, P->wc, nullptr, s);
         std::swap(P->phi[0].p, P->phi[1].p);
     }
     launch_gradient(P->prec, P->grid.nx, P->grid.dx, P->phi[1].p, P->acc4.p, s);
-    launch_interp(P->prec, P->n, P->x.p, nullptr, P->gdev, P->acc4.p, P->a.p, s);
-    launch_correct(P->prec, P->n, P->v.p, P->a.p, P->u.p, P->dt, s);
+    launch_pm_particles(a, PM_INTERP_CORRECT | PM_WRITE_SYNC, s);
+}
+
+// caller's particle array (n x 4) into the object's order, and back
+void take_in(rrg_pm_adjoint* P, const void* in, void* to, cudaStream_t s) {
+    if (P->sort)
+        launch_permute(P->n, 4 * P->rsz, static_cast<const uint32_t*>(P->dest.p), in, to, s);
+    else
+        RRG_CUDA(cudaMemcpyAsync(to, in, pvb(P), cudaMemcpyDeviceToDevice, s));
+}
+
+void give_back(rrg_pm_adjoint* P, const void* from, void* out, cudaStream_t s) {
+    if (!P->sort) {
+        RRG_CUDA(cudaMemcpyAsync(out, from, pvb(P), cudaMemcpyDeviceToDevice, s));
+        return;
+    }
+    const int b = div_up(P->n, 256);
+    const auto* d = static_cast<const uint32_t*>(P->dest.p);
+    if (P->prec == RRG_PREC_FP64)
+        gather_kernel<double><<<b, 256, 0, s>>>(P->n, d, static_cast<const V4<double>*>(from),
+                                               static_cast<V4<double>*>(out));
+    else
+        gather_kernel<float><<<b, 256, 0, s>>>(P->n, d, static_cast<const V4<float>*>(from),
+                                              static_cast<V4<float>*>(out));
+    RRG_LAUNCHED();
 }
 
 template <typename R>
@@ -303,40 +368,29 @@ void backward_step(rrg_pm_adjoint* P, const void* xn1, const void* phin1, cudaSt
     auto* X = static_cast<V4<R>*>(P->X.p);
     auto* V = static_cast<V4<R>*>(P->V.p);
     auto* A = static_cast<V4<R>*>(P->A.p);
-    auto* U = static_cast<V4<R>*>(P->U.p);
     auto* Xi = static_cast<V4<R>*>(P->Xi.p);
-    auto* Xd = static_cast<V4<R>*>(P->Xd.p);
     const R dt = static_cast<R>(P->dt);
-    correct_adjoint_kernel<R><<<bp, 256, 0, s>>>(n, V, A, U, dt);
-    RRG_LAUNCHED();
     launch_gradient(P->prec, P->grid.nx, P->grid.dx, phin1, P->acc4.p, s);
     RRG_CUDA(cudaMemsetAsync(P->gbar.p, 0, P->gbar.bytes, s));
     interp_adjoint_kernel<R><<<bp, 256, 0, s>>>(n, static_cast<const V4<R>*>(xn1), P->gdev,
-                                                static_cast<const V4<R>*>(P->acc4.p), A,
-                                                static_cast<R*>(P->gbar.p), Xi);
+                                                static_cast<const V4<R>*>(P->acc4.p), A, V,
+                                                dt * R(0.5), static_cast<R*>(P->gbar.p), Xi);
     RRG_LAUNCHED();
-    // Cb holds the cotangent of the current level (scale 1), Pb the previous one (scale 1)
+    // Cb holds the cotangent of the current level, Pb that of the one before over K_O (each
+    // reversed substep leaves C in its place, whose share of the level before is K_O C)
     gradient_adjoint_kernel<R><<<bg, 256, 0, s>>>(P->grid.nx, static_cast<R>(-1.0 / P->grid.dx),
                                                   static_cast<const R*>(P->gbar.p),
                                                   static_cast<R*>(P->Cb.p));
     RRG_LAUNCHED();
     RRG_CUDA(cudaMemsetAsync(P->F.p, 0, P->F.bytes, s));
-    R beta = R(1);
     for (int k = 0; k < P->substeps; ++k) {
         launch_wave_adjoint_step(P->prec, P->grid.nx, P->Cb.p, P->Pb.p, P->F.p, P->wc.K_MAIN,
-                                 P->wc.K_ACTUAL, static_cast<double>(beta), P->wc.K_F, s);
-        std::swap(P->Cb.p, P->Pb.p);  // the new current cotangent; old C becomes P / K_O
-        beta = static_cast<R>(P->wc.K_OLD);
+                                 P->wc.K_ACTUAL, P->wc.K_OLD, P->wc.K_F, s);
+        std::swap(P->Cb.p, P->Pb.p);
     }
-    // leave Pb unscaled (Pb *= K_O) so the next step sees both cotangents with scale 1
-    scale_kernel<R><<<bg, 256, 0, s>>>(nc, static_cast<R*>(P->Pb.p), static_cast<R>(P->wc.K_OLD));
-    RRG_LAUNCHED();
-    deposit_adjoint_kernel<R><<<bp, 256, 0, s>>>(n, static_cast<const V4<R>*>(xn1), P->gdev,
-                                                 static_cast<const R*>(P->F.p),
-                                                 static_cast<R>(4.0 * kPi / (P->grid.dx * P->grid.dx * P->grid.dx)),
-                                                 Xd);
-    RRG_LAUNCHED();
-    predict_adjoint_kernel<R><<<bp, 256, 0, s>>>(n, X, Xi, Xd, U, V, A, dt);
+    deposit_predict_adjoint_kernel<R><<<bp, 256, 0, s>>>(
+        n, static_cast<const V4<R>*>(xn1), P->gdev, static_cast<const R*>(P->F.p),
+        static_cast<R>(4.0 * kPi / (P->grid.dx * P->grid.dx * P->grid.dx)), X, Xi, V, A, dt);
     RRG_LAUNCHED();
 }
 
@@ -405,12 +459,23 @@ RRG_API rrg_status rrg_pm_adjoint_create(int device, int precision, int64_t n, d
         P->wc.DX = DX;
         P->wc.domain_min = grid->domain_min;
         const size_t pb = pvb(P), gb = gvb(P);
-        for (PBuf* b : {&P->x, &P->v, &P->a, &P->u, &P->X, &P->V, &P->A, &P->U, &P->Xi, &P->Xd})
+        for (PBuf* b : {&P->x, &P->v, &P->a, &P->u, &P->X, &P->V, &P->A, &P->Xi})
             b->alloc(pb);
         P->mg.alloc(8 * P->nc);
         for (PBuf* b : {&P->src, &P->phi[0], &P->phi[1], &P->Cb, &P->Pb, &P->F}) b->alloc(gb);
         P->acc4.alloc(4 * gb);
         P->gbar.alloc(4 * gb);
+        // sorting costs ~50 us a forward pass and saves ~0.2 ns per particle and deposit (262,144
+        // disk particles on 64^3: predict and deposit 66 -> 9 us, the field cotangent's scatter
+        // 41 -> 13 us), two deposits and a scatter a step
+        P->sort = n * nsteps >= (int64_t(1) << 18) && n < (int64_t(1) << 31);
+        if (P->sort) {
+            P->keys.alloc(4 * n);
+            P->dest.alloc(4 * n);
+            for (PBuf* b : {&P->counts, &P->offsets, &P->cursor}) b->alloc(4 * (P->nc + 1));
+            P->temp_bytes = sort_scan_temp_bytes(P->nc);
+            P->temp.alloc(std::max<size_t>(P->temp_bytes, 256));
+        }
         const int nck = (nsteps + P->every - 1) / P->every;
         P->ck_x.alloc(pb * nck);
         P->ck_v.alloc(pb * nck);
@@ -445,8 +510,22 @@ RRG_API rrg_status rrg_pm_adjoint_forward(rrg_pm_adjoint* P, const void* x0, con
     PMA_ENTRY(P, {
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         const size_t pb = pvb(P), gb = gvb(P);
-        RRG_CUDA(cudaMemcpyAsync(P->x.p, x0, pb, cudaMemcpyDeviceToDevice, s));
-        RRG_CUDA(cudaMemcpyAsync(P->v.p, v0, pb, cudaMemcpyDeviceToDevice, s));
+        if (P->sort) {
+            RRG_CUDA(cudaMemsetAsync(P->counts.p, 0, P->counts.bytes, s));
+            RRG_CUDA(cudaMemsetAsync(P->cursor.p, 0, P->cursor.bytes, s));
+            launch_cell_keys(P->prec, P->n, x0, nullptr, P->gdev, static_cast<uint32_t*>(P->keys.p),
+                             static_cast<uint32_t*>(P->counts.p), s);
+            launch_scan_counts(static_cast<const uint32_t*>(P->counts.p),
+                               static_cast<uint32_t*>(P->offsets.p), P->nc, P->temp.p,
+                               P->temp_bytes, s);
+            launch_sort_dest(P->n, static_cast<const uint32_t*>(P->keys.p),
+                             static_cast<const uint32_t*>(P->offsets.p),
+                             static_cast<uint32_t*>(P->cursor.p),
+                             static_cast<uint32_t*>(P->dest.p), s);
+        }
+        RRG_CUDA(cudaMemsetAsync(P->mg.p, 0, P->mg.bytes, s));
+        take_in(P, x0, P->x.p, s);
+        take_in(P, v0, P->v.p, s);
         RRG_CUDA(cudaMemcpyAsync(P->phi[0].p, phi_prev0, gb, cudaMemcpyDeviceToDevice, s));
         RRG_CUDA(cudaMemcpyAsync(P->phi[1].p, phi_cur0, gb, cudaMemcpyDeviceToDevice, s));
         launch_gradient(P->prec, P->grid.nx, P->grid.dx, P->phi[1].p, P->acc4.p, s);
@@ -462,8 +541,8 @@ RRG_API rrg_status rrg_pm_adjoint_forward(rrg_pm_adjoint* P, const void* x0, con
             }
             pm_step(P, s);
         }
-        if (x_out) RRG_CUDA(cudaMemcpyAsync(x_out, P->x.p, pb, cudaMemcpyDeviceToDevice, s));
-        if (v_out) RRG_CUDA(cudaMemcpyAsync(v_out, P->v.p, pb, cudaMemcpyDeviceToDevice, s));
+        if (x_out) give_back(P, P->x.p, x_out, s);
+        if (v_out) give_back(P, P->v.p, v_out, s);
         if (phi_out) RRG_CUDA(cudaMemcpyAsync(phi_out, P->phi[1].p, gb, cudaMemcpyDeviceToDevice, s));
         P->forward_done = true;
     })
@@ -479,9 +558,9 @@ RRG_API rrg_status rrg_pm_adjoint_backward(rrg_pm_adjoint* P, const void* gx_fin
         RRG_REQUIRE(P->forward_done, RRG_ERR_STATE, "rrg_pm_adjoint_backward before forward");
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         const size_t pb = pvb(P), gb = gvb(P);
-        if (gx_final) RRG_CUDA(cudaMemcpyAsync(P->X.p, gx_final, pb, cudaMemcpyDeviceToDevice, s));
+        if (gx_final) take_in(P, gx_final, P->X.p, s);
         else RRG_CUDA(cudaMemsetAsync(P->X.p, 0, pb, s));
-        if (gv_final) RRG_CUDA(cudaMemcpyAsync(P->V.p, gv_final, pb, cudaMemcpyDeviceToDevice, s));
+        if (gv_final) take_in(P, gv_final, P->V.p, s);
         else RRG_CUDA(cudaMemsetAsync(P->V.p, 0, pb, s));
         RRG_CUDA(cudaMemset2DAsync(P->X.c() + 3 * P->rsz, 4 * P->rsz, 0, P->rsz, P->n, s));
         RRG_CUDA(cudaMemsetAsync(P->A.p, 0, pb, s));
@@ -515,7 +594,7 @@ RRG_API rrg_status rrg_pm_adjoint_backward(rrg_pm_adjoint* P, const void* gx_fin
             interp_adjoint_kernel<double><<<bp, 256, 0, s>>>(
                 P->n, static_cast<const V4<double>*>(P->x.p), P->gdev,
                 static_cast<const V4<double>*>(P->acc4.p), static_cast<const V4<double>*>(P->A.p),
-                nullptr, static_cast<V4<double>*>(P->Xi.p));
+                nullptr, 0.0, nullptr, static_cast<V4<double>*>(P->Xi.p));
             RRG_LAUNCHED();
             add_xyz_kernel<double><<<bp, 256, 0, s>>>(P->n, static_cast<V4<double>*>(P->X.p),
                                                      static_cast<const V4<double>*>(P->Xi.p));
@@ -523,14 +602,14 @@ RRG_API rrg_status rrg_pm_adjoint_backward(rrg_pm_adjoint* P, const void* gx_fin
             interp_adjoint_kernel<float><<<bp, 256, 0, s>>>(
                 P->n, static_cast<const V4<float>*>(P->x.p), P->gdev,
                 static_cast<const V4<float>*>(P->acc4.p), static_cast<const V4<float>*>(P->A.p),
-                nullptr, static_cast<V4<float>*>(P->Xi.p));
+                nullptr, 0.f, nullptr, static_cast<V4<float>*>(P->Xi.p));
             RRG_LAUNCHED();
             add_xyz_kernel<float><<<bp, 256, 0, s>>>(P->n, static_cast<V4<float>*>(P->X.p),
                                                     static_cast<const V4<float>*>(P->Xi.p));
         }
         RRG_LAUNCHED();
-        RRG_CUDA(cudaMemcpyAsync(gx_out, P->X.p, pb, cudaMemcpyDeviceToDevice, s));
-        RRG_CUDA(cudaMemcpyAsync(gv_out, P->V.p, pb, cudaMemcpyDeviceToDevice, s));
+        give_back(P, P->X.p, gx_out, s);
+        give_back(P, P->V.p, gv_out, s);
     })
 }
 
