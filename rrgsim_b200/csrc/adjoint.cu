@@ -36,6 +36,7 @@
 
 #include "host_io.h"
 #include "kernels.cuh"
+#include "pair_plan.cuh"
 
 namespace rrg {
 namespace {
@@ -271,6 +272,262 @@ __global__ void __launch_bounds__(kBS, 2) vjp_f32x2_kernel(const VjpParams<float
             p.out[k] = v4<float>(gx[e], gy[e], gz[e], gm[e]);
         }
     }
+}
+
+// ----------------------------------------------------------------------------------------------
+// FP32 VJP (and force) with each unordered pair evaluated once, on direct_sym.cu's schedule: the
+// pair's geometry, f, g and the vector T = f u - 3 g (d . u) d serve both particles (T changes
+// sign), so a pair with the mass gradient and the force costs 41 FMA-pipe operations (equal
+// masses) instead of twice 29. The j sums (T, m-bar and the force) travel along the warp. G2 packed
+// pairs of i-particles per thread. NV sums per particle: T (3), m-bar, FORCE: the force (3).
+// Slots as in direct_sym.cu, one array of (T, m-bar) and, FORCE, one of the force behind it.
+// Bound: the FP32 pipe (64% of its peak). N = 16,384, equal masses, with the finish, us, ordered
+// pairs (vjp_f32x2_kernel) -> here: with the force and the mass gradient 284 -> 246, without the
+// force 252 -> 205.
+// ----------------------------------------------------------------------------------------------
+struct VjpPairParams {
+    SymPlan plan;
+    const V4<float>* posm;
+    const float* hsoft;
+    float uniform_h, um;  // um: the common mass (UMASS)
+    const V4<float>* lam;
+    V4<float>* js;    // [tiles - 1][n]
+    V4<float>* is;    // [islots][n]
+    V4<float>* js2;   // [blocks][kBS]
+    int64_t force;    // offset of the force's three arrays from these
+};
+
+template <int G2, bool FORCE>
+constexpr size_t vjp_pair_smem() {
+    return sizeof(float) * (FORCE ? 7 : 4) * 2 * G2 * kBS + sizeof(float4) * (FORCE ? 4 : 3) * kBS;
+}
+
+template <int G2, bool USOFT, bool UMASS, bool MGRAD, bool FORCE>
+__global__ void __launch_bounds__(kBS, 2) vjp_pair_kernel(const VjpPairParams p) {
+    constexpr int NV = FORCE ? 7 : 4;
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    float4* const s_p = reinterpret_cast<float4*>(sm_raw);  // x, y, z, m
+    float4* const s_l = s_p + kBS;                          // lam, h
+    V4<float>* const s_j = reinterpret_cast<V4<float>*>(s_l + kBS);
+    V4<float>* const s_jf = s_j + (FORCE ? kBS : 0);
+    float* const s_i = reinterpret_cast<float*>(s_jf + kBS);  // [2 G2][NV][kBS]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const SymPlan& pl = p.plan;
+    const int64_t q0 = pl.run_start(blockIdx.x), q1 = pl.run_start(blockIdx.x + 1);  // rounds
+    const int64_t u0 = q0 / kPairWarps, u1 = (q1 + kPairWarps - 1) / kPairWarps;      // units
+    int a = 0;
+    while (a + 1 < pl.tiles && pl.first_unit(a + 1) <= u0) ++a;
+
+    float2 nx[G2], ny[G2], nz[G2], hs[G2], mi[G2], lx[G2], ly[G2], lz[G2];  // (lam negated)
+    auto load_i = [&]() {
+#pragma unroll
+        for (int g = 0; g < G2; ++g) {
+            V4<float> pi[2], li[2];
+            float h[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int64_t i = static_cast<int64_t>(a) * (kBS * 2 * G2) + (2 * g + e) * kBS + tid;
+                pi[e] = v4<float>(kVjpPad, kVjpPad, kVjpPad, 0.f);
+                li[e] = v4<float>(0.f, 0.f, 0.f, 0.f);
+                h[e] = 1.f;
+                if (i < pl.n) {
+                    pi[e] = p.posm[i];
+                    li[e] = p.lam[i];
+                    if constexpr (!USOFT) h[e] = p.hsoft[i];
+                }
+            }
+            nx[g] = make_float2(-pi[0].x, -pi[1].x);
+            ny[g] = make_float2(-pi[0].y, -pi[1].y);
+            nz[g] = make_float2(-pi[0].z, -pi[1].z);
+            mi[g] = make_float2(pi[0].w, pi[1].w);
+            lx[g] = make_float2(-li[0].x, -li[1].x);
+            ly[g] = make_float2(-li[0].y, -li[1].y);
+            lz[g] = make_float2(-li[0].z, -li[1].z);
+            hs[g] = USOFT ? dup2(p.uniform_h + p.uniform_h) : make_float2(h[0], h[1]);
+        }
+#pragma unroll
+        for (int k = 0; k < 2 * G2 * NV; ++k) s_i[k * kBS + tid] = 0.f;
+    };
+    const float um = UMASS ? p.um : 1.f;
+    auto flush_i = [&]() {
+        const int slot = static_cast<int>(blockIdx.x) - pl.first_block(a);
+#pragma unroll
+        for (int q = 0; q < 2 * G2; ++q) {
+            const int64_t i = static_cast<int64_t>(a) * (kBS * 2 * G2) + q * kBS + tid;
+            if (i >= pl.n) continue;
+            const float* const v = s_i + q * NV * kBS + tid;
+            V4<float>* const to = p.is + static_cast<int64_t>(slot) * pl.n + i;
+            *to = v4<float>(um * v[0], um * v[kBS], um * v[2 * kBS], -v[3 * kBS]);
+            if constexpr (FORCE)
+                to[p.force] = v4<float>(um * v[4 * kBS], um * v[5 * kBS], um * v[6 * kBS], 0.f);
+        }
+    };
+    V4<float> nxt, nxl;
+    auto fetch = [&](int64_t t) {
+        const int64_t j = t * kBS + tid;
+        nxt = v4<float>(kVjpPad, kVjpPad, kVjpPad, 0.f);
+        nxl = v4<float>(0.f, 0.f, 0.f, 1.f);
+        if (j < pl.n) {
+            nxt = p.posm[j];
+            nxl = p.lam[j];
+            if constexpr (!USOFT) nxl.w = p.hsoft[j];
+        }
+    };
+    float2 tT[3][G2], tM[G2], tF[3][G2];
+
+    load_i();
+    int64_t base = pl.first_unit(a);
+    fetch(static_cast<int64_t>(a) * pl.g + (u0 - base));
+    for (int64_t u = u0; u < u1; ++u) {
+        if (u >= base + (pl.nt - static_cast<int64_t>(a) * pl.g)) {
+            flush_i();
+            ++a;
+            base = pl.first_unit(a);
+            load_i();
+        }
+        const int64_t t = static_cast<int64_t>(a) * pl.g + (u - base);
+        const int r0 = u == u0 ? static_cast<int>(q0 - u0 * kPairWarps) : 0;
+        const int r1 = u + 1 == u1 ? static_cast<int>(q1 - u * kPairWarps) : kPairWarps;
+        const bool own = t < static_cast<int64_t>(a + 1) * pl.g;  // a's own tiles: i alone
+        __syncthreads();  // the tile before is done with (its j sums are stored)
+        s_p[tid] = make_float4(nxt.x, nxt.y, nxt.z, nxt.w);
+        s_l[tid] = make_float4(nxl.x, nxl.y, nxl.z, nxl.w);
+        s_j[tid] = v4<float>(0.f, 0.f, 0.f, 0.f);
+        if constexpr (FORCE) s_jf[tid] = v4<float>(0.f, 0.f, 0.f, 0.f);
+        __syncthreads();
+        if (u + 1 < u1) {
+            const bool same = u + 1 < base + (pl.nt - static_cast<int64_t>(a) * pl.g);
+            fetch(same ? t + 1 : static_cast<int64_t>(a + 1) * pl.g);
+        }
+#pragma unroll
+        for (int g = 0; g < G2; ++g) {
+            tM[g] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) tT[k][g] = tF[k][g] = make_float2(0.f, 0.f);
+        }
+        // one j against the thread's i: the i sums, and (BOTH) the j sums jT, jM, jF
+        float2 jT[3], jM, jF[3];
+        auto pairs = [&](auto both, const float4& pj, const float4& lj) {
+            constexpr bool BOTH = decltype(both)::value;
+#pragma unroll
+            for (int g = 0; g < G2; ++g) {
+                const float2 dx = __fadd2_rn(dup2(pj.x), nx[g]);
+                const float2 dy = __fadd2_rn(dup2(pj.y), ny[g]);
+                const float2 dz = __fadd2_rn(dup2(pj.z), nz[g]);
+                const float2 s = USOFT ? hs[g] : __fadd2_rn(hs[g], dup2(lj.w));
+                const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, s)));
+                const float2 inv = make_float2(rsqrt_sfu(r2.x), rsqrt_sfu(r2.y));
+                const float2 inv2 = __fmul2_rn(inv, inv);
+                const float2 f = __fmul2_rn(inv, inv2);
+                const float2 g3 = __fmul2_rn(__fmul2_rn(f, inv2), dup2(-3.f));
+                const float2 mj = dup2(pj.w);
+                float2 ux, uy, uz, dot, dli, dlj;
+                if constexpr (UMASS) {
+                    ux = __fadd2_rn(dup2(lj.x), lx[g]);
+                    uy = __fadd2_rn(dup2(lj.y), ly[g]);
+                    uz = __fadd2_rn(dup2(lj.z), lz[g]);
+                } else {
+                    ux = __ffma2_rn(mi[g], dup2(lj.x), __fmul2_rn(mj, lx[g]));
+                    uy = __ffma2_rn(mi[g], dup2(lj.y), __fmul2_rn(mj, ly[g]));
+                    uz = __ffma2_rn(mi[g], dup2(lj.z), __fmul2_rn(mj, lz[g]));
+                }
+                dot = __ffma2_rn(dz, uz, __ffma2_rn(dy, uy, __fmul2_rn(dx, ux)));
+                if constexpr (MGRAD) {
+                    dlj = __ffma2_rn(dz, dup2(lj.z),
+                                     __ffma2_rn(dy, dup2(lj.y), __fmul2_rn(dx, dup2(lj.x))));
+                    tM[g] = __ffma2_rn(f, dlj, tM[g]);
+                    if constexpr (BOTH) {  // (lam_i is held negated)
+                        dli = __ffma2_rn(dz, lz[g], __ffma2_rn(dy, ly[g], __fmul2_rn(dx, lx[g])));
+                        jM = __ffma2_rn(f, dli, jM);
+                    }
+                }
+                const float2 tt = __fmul2_rn(g3, dot);
+                const float2 Tx = __ffma2_rn(tt, dx, __fmul2_rn(f, ux));
+                const float2 Ty = __ffma2_rn(tt, dy, __fmul2_rn(f, uy));
+                const float2 Tz = __ffma2_rn(tt, dz, __fmul2_rn(f, uz));
+                tT[0][g] = __fadd2_rn(tT[0][g], Tx);
+                tT[1][g] = __fadd2_rn(tT[1][g], Ty);
+                tT[2][g] = __fadd2_rn(tT[2][g], Tz);
+                if constexpr (BOTH) {
+                    jT[0] = __fadd2_rn(jT[0], Tx);
+                    jT[1] = __fadd2_rn(jT[1], Ty);
+                    jT[2] = __fadd2_rn(jT[2], Tz);
+                }
+                if constexpr (FORCE) {
+                    const float2 fi = UMASS ? f : __fmul2_rn(mj, f);
+                    tF[0][g] = __ffma2_rn(fi, dx, tF[0][g]);
+                    tF[1][g] = __ffma2_rn(fi, dy, tF[1][g]);
+                    tF[2][g] = __ffma2_rn(fi, dz, tF[2][g]);
+                    if constexpr (BOTH) {
+                        const float2 fj = UMASS ? f : __fmul2_rn(mi[g], f);
+                        jF[0] = __ffma2_rn(fj, dx, jF[0]);
+                        jF[1] = __ffma2_rn(fj, dy, jF[1]);
+                        jF[2] = __ffma2_rn(fj, dz, jF[2]);
+                    }
+                }
+            }
+        };
+        if (own) {
+#pragma unroll 2
+            for (int k = 32 * r0; k < 32 * r1; ++k) pairs(std::false_type{}, s_p[k], s_l[k]);
+        } else {
+            for (int r = r0; r < r1; ++r) {
+                const int c = ((warp + r) & (kPairWarps - 1)) * 32;
+                const int from = (lane + 1) & 31;
+                float cT[3] = {0.f, 0.f, 0.f}, cM = 0.f, cF[3] = {0.f, 0.f, 0.f};
+#pragma unroll 2
+                for (int s = 0; s < 32; ++s) {
+                    const int k = c + ((lane + s) & 31);
+                    jM = make_float2(cM, 0.f);
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) {
+                        jT[e] = make_float2(cT[e], 0.f);
+                        jF[e] = make_float2(cF[e], 0.f);
+                    }
+                    pairs(std::true_type{}, s_p[k], s_l[k]);
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) {
+                        cT[e] = __shfl_sync(0xffffffffu, half_sum(jT[e]), from);
+                        if constexpr (FORCE) cF[e] = __shfl_sync(0xffffffffu, half_sum(jF[e]), from);
+                    }
+                    if constexpr (MGRAD) cM = __shfl_sync(0xffffffffu, half_sum(jM), from);
+                }
+                V4<float> v = s_j[c + lane];
+                s_j[c + lane] = v4<float>(v.x + cT[0], v.y + cT[1], v.z + cT[2], v.w + cM);
+                if constexpr (FORCE) {
+                    v = s_jf[c + lane];
+                    s_jf[c + lane] = v4<float>(v.x + cF[0], v.y + cF[1], v.z + cF[2], 0.f);
+                }
+                __syncthreads();  // the next warp to add to this chunk comes after
+            }
+            const int64_t j = t * kBS + tid;
+            if (j < pl.n) {
+                V4<float>* const to = r0 == 0 ? p.js + static_cast<int64_t>(a) * pl.n + j
+                                              : p.js2 + static_cast<int64_t>(blockIdx.x) * kBS + tid;
+                // T and the force change sign for j; jM holds f (-lam_i . d) = -(m-bar_j's term)
+                V4<float> v = s_j[tid];
+                *to = v4<float>(-um * v.x, -um * v.y, -um * v.z, -v.w);
+                if constexpr (FORCE) {
+                    v = s_jf[tid];
+                    to[p.force] = v4<float>(-um * v.x, -um * v.y, -um * v.z, 0.f);
+                }
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < G2; ++g) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float* const v = s_i + (2 * g + e) * NV * kBS + tid;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    v[k * kBS] += e ? tT[k][g].y : tT[k][g].x;
+                    if constexpr (FORCE) v[(4 + k) * kBS] += e ? tF[k][g].y : tF[k][g].x;
+                }
+                if constexpr (MGRAD) v[3 * kBS] += e ? tM[g].y : tM[g].x;
+            }
+        }
+    }
+    flush_i();
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -577,6 +834,20 @@ struct RevStep {
     float dt;
 };
 
+// w -= dt a(x_m), x_{m-1} = x_m - dt w for particle k
+__device__ __forceinline__ void reverse_step_at(int64_t k, double ax, double ay, double az,
+                                                const RevStep& r) {
+    V4<float> w = r.w[k];
+    w.x -= r.dt * static_cast<float>(ax);
+    w.y -= r.dt * static_cast<float>(ay);
+    w.z -= r.dt * static_cast<float>(az);
+    r.w[k] = w;
+    if (r.x_next) {
+        const V4<float> x = r.x[k];
+        r.x_next[k] = v4<float>(x.x - r.dt * w.x, x.y - r.dt * w.y, x.z - r.dt * w.z, x.w);
+    }
+}
+
 // Top of a segment: w = v - dt/2 a, x_out = x - dt w (mass carried).
 __global__ void reverse_init_kernel(int64_t n, const V4<float>* __restrict__ x,
                                     const V4<float>* __restrict__ v,
@@ -614,15 +885,7 @@ __global__ void vjp_reverse_finish(const VjpParams<float> p, int splits, const A
     const V4<float> X = v4<float>(static_cast<float>(sx + o.x), static_cast<float>(sy + o.y),
                                   static_cast<float>(sz + o.z), static_cast<float>(sm + o.w));
     p.out[k] = X;
-    V4<float> w = r.w[k];
-    w.x -= r.dt * static_cast<float>(ax);
-    w.y -= r.dt * static_cast<float>(ay);
-    w.z -= r.dt * static_cast<float>(az);
-    r.w[k] = w;
-    if (r.x_next) {
-        const V4<float> x = r.x[k];
-        r.x_next[k] = v4<float>(x.x - r.dt * w.x, x.y - r.dt * w.y, x.z - r.dt * w.z, x.w);
-    }
+    reverse_step_at(k, ax, ay, az, r);
     if (upd.V) adjoint_update_at(k, X.x, X.y, X.z, upd);
 }
 
@@ -669,6 +932,140 @@ void vjp_reverse_launch(const void* hsoft, double uniform_h, double uniform_m, i
 #undef RRG_VJPF
     RRG_LAUNCHED();
     vjp_reverse_finish<<<div_up(n, 256), 256, 0, stream>>>(p, real, upd, r);
+    RRG_LAUNCHED();
+}
+
+// A particle's slots in order, FP64 (direct_sym_finish): (T, m-bar) sums, and with FORCE the force.
+template <bool FORCE>
+__device__ __forceinline__ void vjp_pair_sum(const VjpPairParams& p, int64_t k, double s[4],
+                                             double f[3]) {
+    const SymPlan& pl = p.plan;
+    const int a = static_cast<int>(k / (kBS * pl.g));
+    const int cnt = pl.last_block(a) - pl.first_block(a) + 1;
+    const int64_t t = k / kBS;
+    auto add = [&](const V4<float>* q) {
+        const V4<float> v = *q;
+        s[0] += v.x;
+        s[1] += v.y;
+        s[2] += v.z;
+        s[3] += v.w;
+        if constexpr (FORCE) {
+            const V4<float> w = q[p.force];
+            f[0] += w.x;
+            f[1] += w.y;
+            f[2] += w.z;
+        }
+    };
+#pragma unroll 4
+    for (int i = 0; i < a; ++i) {
+        add(p.js + static_cast<int64_t>(i) * pl.n + k);
+        // the second part of a unit that two runs share
+        const int64_t q = 8 * (pl.first_unit(i) + t - static_cast<int64_t>(i) * pl.g);
+        const int b = pl.block_of(q + 7);
+        if (pl.run_start(b) > q) add(p.js2 + static_cast<int64_t>(b) * kBS + (k & (kBS - 1)));
+    }
+#pragma unroll 4
+    for (int i = 0; i < cnt; ++i) add(p.is + static_cast<int64_t>(i) * pl.n + k);
+}
+
+// vjp_finish and vjp_reverse_finish (FORCE) on those sums.
+template <bool FORCE>
+__global__ void __launch_bounds__(128) vjp_pair_finish(const VjpPairParams p, V4<float>* out,
+                                                       int accumulate, const AdjUpd<float> upd,
+                                                       const RevStep r) {
+    const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k >= p.plan.n) return;
+    double s[4] = {0, 0, 0, 0}, f[3] = {0, 0, 0};
+    vjp_pair_sum<FORCE>(p, k, s, f);
+    if (accumulate) {
+        const V4<float> o = out[k];
+        s[0] += o.x;
+        s[1] += o.y;
+        s[2] += o.z;
+        s[3] += o.w;
+    }
+    const V4<float> X = v4<float>(static_cast<float>(s[0]), static_cast<float>(s[1]),
+                                  static_cast<float>(s[2]), static_cast<float>(s[3]));
+    out[k] = X;
+    if constexpr (FORCE) reverse_step_at(k, f[0], f[1], f[2], r);
+    if (upd.V) adjoint_update_at(k, X.x, X.y, X.z, upd);
+}
+
+int vjp_pair_blocks(int sms, bool umass) {
+    // the kernel of the reversed steps, with equal masses or not
+    const size_t smem = vjp_pair_smem<2, true>();
+    return sms * (umass ? pair_blocks_per_sm(vjp_pair_kernel<2, true, true, true, true>, smem)
+                        : pair_blocks_per_sm(vjp_pair_kernel<2, true, false, true, true>, smem));
+}
+
+SymPlan vjp_pair_plan(int64_t n, int sms, bool umass) {
+    static int cache[2] = {};
+    int& blocks = cache[umass];
+    if (!blocks) blocks = vjp_pair_blocks(sms, umass);
+    return make_pair_plan(n, 4, blocks);
+}
+
+// V4 records of one slot array (js, is and js2 together)
+int64_t vjp_pair_records(const SymPlan& pl) {
+    return static_cast<int64_t>(pl.tiles - 1 + pl.islots) * pl.n +
+           static_cast<int64_t>(pl.blocks) * kBS;
+}
+
+// bytes of the slots ((T, m-bar) and force), 0 where the ordered kernel is the faster one
+size_t vjp_pair_bytes(int64_t n, int sms) {
+    if (!pair_plan_range(n)) return 0;
+    return 2 * sizeof(V4<float>) *
+           static_cast<size_t>(std::max(vjp_pair_records(vjp_pair_plan(n, sms, true)),
+                                        vjp_pair_records(vjp_pair_plan(n, sms, false))));
+}
+
+template <bool USOFT, bool UMASS>
+void vjp_pair_dispatch(const VjpPairParams& p, bool mgrad, bool force, cudaStream_t s) {
+    auto go = [&](auto* k, size_t smem) {
+        if (smem > 48 * 1024)
+            RRG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(smem)));
+        k<<<p.plan.blocks, kBS, smem, s>>>(p);
+    };
+    if (force) {
+        if (mgrad) go(vjp_pair_kernel<2, USOFT, UMASS, true, true>, vjp_pair_smem<2, true>());
+        else go(vjp_pair_kernel<2, USOFT, UMASS, false, true>, vjp_pair_smem<2, true>());
+    } else {
+        if (mgrad) go(vjp_pair_kernel<2, USOFT, UMASS, true, false>, vjp_pair_smem<2, false>());
+        else go(vjp_pair_kernel<2, USOFT, UMASS, false, false>, vjp_pair_smem<2, false>());
+    }
+    RRG_LAUNCHED();
+}
+
+// X (out) += VJP at posm with cotangent lam; r != nullptr: also the force there and the reverse
+// step; then the adjoint update upd.
+void vjp_pair_launch(const void* posm, const void* hsoft, double uniform_h, double uniform_m,
+                     int64_t n, const void* lam, void* out, bool accumulate, void* slots,
+                     int sms, cudaStream_t s, const AdjUpd<float>& upd, const RevStep* r,
+                     bool mgrad) {
+    const bool umass = uniform_m >= 0;
+    VjpPairParams p{};
+    p.plan = vjp_pair_plan(n, sms, umass);
+    p.posm = static_cast<const V4<float>*>(posm);
+    p.hsoft = static_cast<const float*>(hsoft);
+    p.uniform_h = static_cast<float>(uniform_h);
+    p.um = umass ? static_cast<float>(uniform_m) : 1.f;
+    p.lam = static_cast<const V4<float>*>(lam);
+    p.js = static_cast<V4<float>*>(slots);
+    p.is = p.js + static_cast<int64_t>(p.plan.tiles - 1) * n;
+    p.js2 = p.is + static_cast<int64_t>(p.plan.islots) * n;
+    p.force = vjp_pair_records(p.plan);
+    const bool force = r != nullptr;
+    if (hsoft) {
+        if (umass) vjp_pair_dispatch<false, true>(p, mgrad, force, s);
+        else vjp_pair_dispatch<false, false>(p, mgrad, force, s);
+    } else {
+        if (umass) vjp_pair_dispatch<true, true>(p, mgrad, force, s);
+        else vjp_pair_dispatch<true, false>(p, mgrad, force, s);
+    }
+    auto* o = static_cast<V4<float>*>(out);
+    if (force) vjp_pair_finish<true><<<div_up(n, 128), 128, 0, s>>>(p, o, accumulate ? 1 : 0, upd, *r);
+    else vjp_pair_finish<false><<<div_up(n, 128), 128, 0, s>>>(p, o, accumulate ? 1 : 0, upd, RevStep{});
     RRG_LAUNCHED();
 }
 
@@ -777,7 +1174,9 @@ struct rrg_adjoint {
     ABuf ckpt_x, ckpt_v, ckpt_a;  // (nsteps / every + 1) x n x V4: state and a(x) there
     ABuf seg_x;            // (every + 1) x n x V4
     ABuf x, x2, v, a, u, X, V, c, g, xN, scratch, sym_slots;
-    ABuf vjp_part;          // FP32: j-split partials of the paired VJP
+    ABuf vjp_part;          // FP32: pair slots (vjp_pairs) or j-split partials of the VJP
+    bool vjp_pairs = false;
+    int sms = 148;
     ABuf vjp_part_a;        // FP32: force partials of the reverse steps
     ABuf w;                 // FP32: half-step velocity of the reverse steps
     ABuf mflags;            // uniform-mass check: mismatch flag, mass bits
@@ -863,6 +1262,10 @@ void vjp(rrg_adjoint* A, const void* x, int m, cudaStream_t s) {
     if (A->prec == RRG_PREC_FP64)
         vjp_sym_launch<double>(x, A->hsoft.p, A->uniform_h, A->n, A->c.p, A->X.p, true,
                                A->sym_slots.p, s, step_update<double>(A, m));
+    else if (A->vjp_pairs)
+        vjp_pair_launch(x, A->hsoft.p, A->uniform_h, A->uniform_m, A->n, A->c.p, A->X.p, true,
+                        A->vjp_part.p, A->sms, s, step_update<float>(A, m), nullptr,
+                        A->mass_grad);
     else
         vjp_f32x2_launch(x, A->hsoft.p, A->uniform_h, A->uniform_m, A->n, A->c.p, A->X.p, true,
                          A->vjp_part.p, A->vjp_splits, s, step_update<float>(A, m),
@@ -992,12 +1395,23 @@ RRG_API rrg_status rrg_adjoint_create(int device, int precision, int64_t n, doub
         if (precision == RRG_PREC_FP64) {
             A->sym_slots.alloc(vjp_sym_slot_bytes<double>(n));
         } else {
-            A->vjp_splits = vjp_f32x2_splits(n, sms);
-            // the reverse steps write partials even with one split
-            const size_t pb = sizeof(V4<float>) * static_cast<size_t>(n) *
-                              static_cast<size_t>(std::max(1, A->vjp_splits));
-            A->vjp_part.alloc(pb);
-            A->vjp_part_a.alloc(pb);
+            A->sms = sms;
+            if (const size_t pairs = vjp_pair_bytes(n, sms)) {
+                try {
+                    A->vjp_part.alloc(pairs);
+                    A->vjp_pairs = true;
+                } catch (const Error&) {
+                    // no room for the slots: the ordered kernel
+                }
+            }
+            if (!A->vjp_pairs) {
+                A->vjp_splits = vjp_f32x2_splits(n, sms);
+                // the reverse steps write partials even with one split
+                const size_t pb = sizeof(V4<float>) * static_cast<size_t>(n) *
+                                  static_cast<size_t>(std::max(1, A->vjp_splits));
+                A->vjp_part.alloc(pb);
+                A->vjp_part_a.alloc(pb);
+            }
             A->w.alloc(vb(A));
         }
         A->mflags.alloc(16);
@@ -1119,9 +1533,14 @@ RRG_API rrg_status rrg_adjoint_backward(rrg_adjoint* A, const void* gx_final,
                     r.x_next = m - 1 > n0 ? reinterpret_cast<V4<float>*>(xbuf[(m - 1) & 1]) : nullptr;
                     r.w = static_cast<V4<float>*>(A->w.p);
                     r.dt = static_cast<float>(A->dt);
-                    vjp_reverse_launch(A->hsoft.p, A->uniform_h, A->uniform_m, A->n, A->c.p, A->X.p,
-                                       A->vjp_part.p, A->vjp_part_a.p, A->vjp_splits, s,
-                                       step_update<float>(A, m - 1), r, A->mass_grad);
+                    if (A->vjp_pairs)
+                        vjp_pair_launch(r.x, A->hsoft.p, A->uniform_h, A->uniform_m, A->n, A->c.p,
+                                        A->X.p, true, A->vjp_part.p, A->sms, s,
+                                        step_update<float>(A, m - 1), &r, A->mass_grad);
+                    else
+                        vjp_reverse_launch(A->hsoft.p, A->uniform_h, A->uniform_m, A->n, A->c.p,
+                                           A->X.p, A->vjp_part.p, A->vjp_part_a.p, A->vjp_splits,
+                                           s, step_update<float>(A, m - 1), r, A->mass_grad);
                 }
             }
             vjp(A, xc, n0 - 1, s);

@@ -31,53 +31,13 @@
 
 #include "direct_epi.cuh"
 #include "kernels.cuh"
+#include "pair_plan.cuh"
 
 namespace rrg {
 namespace {
 
 constexpr int kBS = kDirectThreads;
-constexpr int kWarps = kBS / 32;
-static_assert(kWarps * 32 == kBS && kWarps == 8, "a j-tile is one chunk of 32 per warp");
-
-// The schedule: units of i-tile a are j-tiles a G .. nt - 1, numbered from first_unit(a); round
-// 8 u + r is round r of unit u.
-struct SymPlan {
-    int n, nt, g, tiles;  // particles, j-tiles, i-particles per thread, i-tiles
-    int64_t rounds;
-    int blocks;           // runs: block b takes rounds [b rounds / blocks, (b + 1) rounds / blocks),
-                          // at least the 8 of one unit
-    int islots;           // i slots: the most blocks that share one i-tile
-
-    __host__ __device__ int64_t first_unit(int64_t a) const {
-        return a * nt - static_cast<int64_t>(g) * (a * (a - 1) / 2);
-    }
-    __host__ __device__ int64_t run_start(int64_t b) const { return b * rounds / blocks; }
-    // the block whose run holds a round
-    __host__ __device__ int block_of(int64_t round) const {
-        return static_cast<int>(((round + 1) * blocks - 1) / rounds);
-    }
-    // the first and last block that work for i-tile a
-    __host__ __device__ int first_block(int64_t a) const { return block_of(8 * first_unit(a)); }
-    __host__ __device__ int last_block(int64_t a) const {
-        return block_of(8 * (first_unit(a) + nt - a * g) - 1);
-    }
-};
-
-SymPlan make_plan(int64_t n, int g, int slots) {
-    SymPlan p;
-    p.n = static_cast<int>(n);
-    p.g = g;
-    p.nt = static_cast<int>((n + kBS - 1) / kBS);
-    p.tiles = (p.nt + g - 1) / g;
-    const int64_t units =
-        p.first_unit(p.tiles - 1) + (p.nt - static_cast<int64_t>(p.tiles - 1) * g);
-    p.rounds = 8 * units;
-    p.blocks = static_cast<int>(std::min<int64_t>(slots, units));
-    p.islots = 1;
-    for (int a = 0; a < p.tiles; ++a)
-        p.islots = std::max(p.islots, p.last_block(a) - p.first_block(a) + 1);
-    return p;
-}
+constexpr int kWarps = kPairWarps;
 
 template <typename R, typename S>
 struct SymParams {
@@ -91,9 +51,6 @@ struct SymParams {
     V4<S>* is;   // [islots][n]
     V4<S>* js2;  // [blocks][kBS]
 };
-
-__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float half_sum(float2 v) { return __fadd_rn(v.x, v.y); }
 
 // ----------------------------------------------------------------------------------------------
 // FP32 and MIXED: G2 packed pairs of i-particles per thread on the paired FP32 instructions
@@ -557,16 +514,6 @@ __global__ void __launch_bounds__(128) direct_sym_finish(const SymParams<R, S> p
                         static_cast<R>(-sp), want_pot, p.posm, p.poslo);
 }
 
-template <typename Kern>
-int resident(Kern k, size_t smem) {
-    if (smem > 48 * 1024)
-        RRG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)));
-    int nb = 0;
-    RRG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, kBS, smem));
-    return std::max(nb, 1);
-}
-
 template <int G2, bool USOFT, bool POT, bool UMASS, bool MIXED>
 void launch32(const SymParams<float, typename Sym32<G2, USOFT, POT, UMASS, MIXED>::S>& p,
               cudaStream_t s) {
@@ -619,15 +566,15 @@ int resident_blocks(int prec, int g) {
     if (r) return r;
     int v = 1;
     if (prec == RRG_PREC_FP64) {
-        if (g == 2) v = resident(direct_sym64_kernel<2, true, false>, Sym64<2, true, false>::smem);
-        else v = resident(direct_sym64_kernel<4, true, false>, Sym64<4, true, false>::smem);
+        if (g == 2) v = pair_blocks_per_sm(direct_sym64_kernel<2, true, false>, Sym64<2, true, false>::smem);
+        else v = pair_blocks_per_sm(direct_sym64_kernel<4, true, false>, Sym64<4, true, false>::smem);
     } else if (prec == RRG_PREC_MIXED) {
-        if (g == 2) v = resident(direct_sym32_kernel<1, true, false, false, true>, Sym32<1, true, false, false, true>::smem);
-        else v = resident(direct_sym32_kernel<2, true, false, false, true>, Sym32<2, true, false, false, true>::smem);
+        if (g == 2) v = pair_blocks_per_sm(direct_sym32_kernel<1, true, false, false, true>, Sym32<1, true, false, false, true>::smem);
+        else v = pair_blocks_per_sm(direct_sym32_kernel<2, true, false, false, true>, Sym32<2, true, false, false, true>::smem);
     } else {
-        if (g == 2) v = resident(direct_sym32_kernel<1, true, false, true, false>, Sym32<1, true, false, true, false>::smem);
-        else if (g == 4) v = resident(direct_sym32_kernel<2, true, false, true, false>, Sym32<2, true, false, true, false>::smem);
-        else v = resident(direct_sym32_kernel<4, true, false, true, false>, Sym32<4, true, false, true, false>::smem);
+        if (g == 2) v = pair_blocks_per_sm(direct_sym32_kernel<1, true, false, true, false>, Sym32<1, true, false, true, false>::smem);
+        else if (g == 4) v = pair_blocks_per_sm(direct_sym32_kernel<2, true, false, true, false>, Sym32<2, true, false, true, false>::smem);
+        else v = pair_blocks_per_sm(direct_sym32_kernel<4, true, false, true, false>, Sym32<4, true, false, true, false>::smem);
     }
     r = v;
     return r;
@@ -650,7 +597,7 @@ SymPlan plan_for(int prec, int64_t n, bool umass, int sms) {
     double t_best = 0.0;
     for (int g = 2; g <= (prec == RRG_PREC_FP32 ? 8 : 4); g *= 2) {
         const int per_sm = resident_blocks(prec, g);
-        const SymPlan p = make_plan(n, g, sms * per_sm);
+        const SymPlan p = make_pair_plan(n, g, sms * per_sm);
         const double unit = g / pair_rate(prec, g, umass);  // per block of a full SM, x per_sm
         const double units = static_cast<double>(p.rounds) / 8;
         double t = per_sm * unit * std::max(1.0, units / (static_cast<double>(sms) * per_sm));
@@ -673,7 +620,7 @@ size_t slot_bytes(int prec) {
 // (116); at 6,000 33 (25) and FP64 77 (64), the units being too few to fill the SMs. Up to
 // 131,072 particles the slots stay below 600 MB.
 size_t direct_sym_scratch_bytes(int prec, int64_t n, bool umass, int sms) {
-    if (n <= 31 * kBS || n > 131072) return 0;
+    if (!pair_plan_range(n)) return 0;
     const SymPlan pl = plan_for(prec, n, umass, sms);
     return slot_bytes(prec) * (static_cast<size_t>(n) * static_cast<size_t>(pl.tiles - 1 + pl.islots) +
                                static_cast<size_t>(pl.blocks) * kBS);
