@@ -31,7 +31,7 @@ CUFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-fvisib
 CXXFLAGS = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-I", str(INCLUDE), "-I",
             str(CSRC), "-I", "/usr/local/cuda/include"]
 
-LIB_SOURCES = ["direct.cu", "direct_sym.cu", "integrate.cu", "pm.cu", "context.cu", "adjoint.cu", "host_io.cpp",
+LIB_SOURCES = ["direct.cu", "direct_sym.cu", "direct_small.cu", "integrate.cu", "pm.cu", "context.cu", "adjoint.cu", "host_io.cpp",
                "run.cpp", "noalloc.cu", "sort.cu", "ensemble.cu", "pm_adjoint.cu",
                "wave_solve.cu"]
 

@@ -69,6 +69,21 @@ __device__ __forceinline__ float rsqrt_sfu(float x) {
     return y;
 }
 
+// FP64 reciprocal square root without branches, for pair loops (x >= 0): the SFU's approximation y
+// (PTX rsqrt.approx.ftz.f64, at least 20 bits) refined once by the binomial series of
+// x^-1/2 = y (1 - e)^-1/2, e = 1 - x y^2, to second order: y (1 + e / 2 + 3 e^2 / 8), whose next
+// term is below 2^-57. Within 2 ulp of the exact value; CUDA's rsqrt branches for special values,
+// which keeps a loop's independent pairs from overlapping. x above 1e300 (infinity included) counts
+// as 1e300: the cube of the result is 0 there and the result itself far below any other term.
+__device__ __forceinline__ double rsqrt_pair(double x) {
+    // (positive doubles compare as their high words; 0x7E37E43C is that of 1e300)
+    x = __hiloint2double(min(__double2hiint(x), 0x7E37E43C), __double2loint(x));
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
 // Error-free transformations for double-float arithmetic (Knuth TwoSum, Dekker Fast2Sum).
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     s = __fadd_rn(a, b);

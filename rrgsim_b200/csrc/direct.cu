@@ -16,6 +16,7 @@
 
 #include "direct_epi.cuh"
 #include "kernels.cuh"
+#include "wave_cells.cuh"
 
 namespace rrg {
 namespace {
@@ -46,6 +47,7 @@ __global__ void __launch_bounds__(kBS, 2) direct_f32_kernel(const F32Params p) {
     const int tid = threadIdx.x;
     const int64_t n = p.n;
     const int64_t ibase = static_cast<int64_t>(blockIdx.x) * (kBS * IPT);
+    pdl_next();  // (the finish may start and wait)
 
     float xi[IPT], yi[IPT], zi[IPT], hi[IPT];
     float xl[IPT], yl[IPT], zl[IPT];
@@ -195,6 +197,7 @@ __global__ void __launch_bounds__(kBS, 2) direct_f32x2_kernel(const F32Params p)
     const int tid = threadIdx.x;
     const int64_t n = p.n;
     const int64_t ibase = static_cast<int64_t>(blockIdx.x) * (kBS * IPT);
+    pdl_next();  // (the finish may start and wait)
 
     float2 nx[G], ny[G], nz[G], hs[G];
 #pragma unroll
@@ -321,6 +324,7 @@ __global__ void __launch_bounds__(kBS, 2) direct_f32jp_kernel(const F32Params p)
     const int tid = threadIdx.x;
     const int64_t n = p.n;
     const int64_t ibase = static_cast<int64_t>(blockIdx.x) * (kBS * G);
+    pdl_next();  // (the finish may start and wait)
 
     float2 nx[G], ny[G], nz[G], hs[G];
 #pragma unroll
@@ -428,29 +432,48 @@ __global__ void __launch_bounds__(kBS, 2) direct_f32jp_kernel(const F32Params p)
     }
 }
 
-// Fixed-order FP64 reduction of the split partials, then the epilogue.
+// Fixed-order FP64 reduction of the split partials, then the epilogue: four lanes per particle, a
+// quarter of the splits each (N = 4,096 with 16 splits: a thread per particle made 16 blocks of
+// serial loads, 4.8 us). Launched with programmatic dependence, so that its blocks are in place when
+// the force kernel ends. The force kernels are not: blocks that start beside those of the launch
+// before share its SMs and leave others idle (N = 8,192 52 us against 33). N = 4,096, 16 splits, us
+// per step: 15.1 -> 12.8.
+constexpr int kFinishThreads = 128;
+__device__ __forceinline__ double over_quad(double v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+
 template <bool MIXED>
-__global__ void direct_f32_finish(const F32Params p, int splits) {
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= p.n) return;
+__global__ void __launch_bounds__(kFinishThreads) direct_f32_finish(const F32Params p, int splits) {
+    const int64_t i = (static_cast<int64_t>(blockIdx.x) * kFinishThreads + threadIdx.x) >> 2;
+    pdl_next();
+    pdl_wait();
     double sx = 0, sy = 0, sz = 0, sp = 0;
-    for (int s = 0; s < splits; ++s) {
-        const V4<float> h = p.part_hi[static_cast<int64_t>(s) * p.n + i];
-        sx += h.x; sy += h.y; sz += h.z; sp += h.w;
-        if constexpr (MIXED) {
-            const V4<float> l = p.part_lo[static_cast<int64_t>(s) * p.n + i];
-            sx += l.x; sy += l.y; sz += l.z; sp += l.w;
+    if (i < p.n) {
+#pragma unroll 4
+        for (int s = threadIdx.x & 3; s < splits; s += 4) {
+            const V4<float> h = p.part_hi[static_cast<int64_t>(s) * p.n + i];
+            sx += h.x; sy += h.y; sz += h.z; sp += h.w;
+            if constexpr (MIXED) {
+                const V4<float> l = p.part_lo[static_cast<int64_t>(s) * p.n + i];
+                sx += l.x; sy += l.y; sz += l.z; sp += l.w;
+            }
         }
     }
+    sx = over_quad(sx);
+    sy = over_quad(sy);
+    sz = over_quad(sz);
+    sp = over_quad(sp);
+    if (i >= p.n || (threadIdx.x & 3) != 0) return;
     apply_epi<float, MIXED>(p.epi, i, static_cast<float>(sx), static_cast<float>(sy),
                             static_cast<float>(sz), static_cast<float>(-sp), p.want_pot,
                             p.posm, p.poslo);
 }
 
 // ----------------------------------------------------------------------------------------------
-// FP64: one i per thread. The reciprocal square root is CUDA's rsqrt (within 1 ulp): 1 / sqrt
-// spent most of the FP64 pipe on its two Newton sequences (N = 8,192: 177 us per evaluation
-// against 116 with rsqrt).
+// FP64: one i per thread. The reciprocal square root is rsqrt_pair: 1 / sqrt spent most of the FP64
+// pipe on its two Newton sequences (N = 7,936: 177 us per evaluation against 109).
 // ----------------------------------------------------------------------------------------------
 struct F64Params {
     const V4<double>* posm;
@@ -471,6 +494,7 @@ __global__ void __launch_bounds__(kBS) direct_f64_kernel(const F64Params p) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * kBS + tid;
     V4<double> pi = v4<double>(0, 0, 0, 0);
     double h = p.uniform_h;
+    pdl_next();  // (the finish may start and wait)
     if (i < p.n) {
         pi = p.posm[i];
         if constexpr (!USOFT) h = p.hsoft[i];
@@ -494,7 +518,7 @@ __global__ void __launch_bounds__(kBS) direct_f64_kernel(const F64Params p) {
             const V4<double> pj = s_pos[k];
             const double dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
             const double hs = USOFT ? (h + h) : (h + s_h[k]);
-            const double inv = rsqrt(dx * dx + dy * dy + dz * dz + hs);
+            const double inv = rsqrt_pair(dx * dx + dy * dy + dz * dz + hs);
             const double kk = pj.w * (inv * inv * inv);
             ax += dx * kk;
             ay += dy * kk;
@@ -510,14 +534,23 @@ __global__ void __launch_bounds__(kBS) direct_f64_kernel(const F64Params p) {
     }
 }
 
-__global__ void direct_f64_finish(const F64Params p, int splits) {
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= p.n) return;
+__global__ void __launch_bounds__(kFinishThreads) direct_f64_finish(const F64Params p, int splits) {
+    const int64_t i = (static_cast<int64_t>(blockIdx.x) * kFinishThreads + threadIdx.x) >> 2;
+    pdl_next();
+    pdl_wait();
     double sx = 0, sy = 0, sz = 0, sp = 0;
-    for (int s = 0; s < splits; ++s) {
-        const V4<double> h = p.part[static_cast<int64_t>(s) * p.n + i];
-        sx += h.x; sy += h.y; sz += h.z; sp += h.w;
+    if (i < p.n) {
+#pragma unroll 4
+        for (int s = threadIdx.x & 3; s < splits; s += 4) {
+            const V4<double> h = p.part[static_cast<int64_t>(s) * p.n + i];
+            sx += h.x; sy += h.y; sz += h.z; sp += h.w;
+        }
     }
+    sx = over_quad(sx);
+    sy = over_quad(sy);
+    sz = over_quad(sz);
+    sp = over_quad(sp);
+    if (i >= p.n || (threadIdx.x & 3) != 0) return;
     apply_epi<double, false>(p.epi, i, sx, sy, sz, -sp, p.want_pot, p.posm, nullptr);
 }
 
@@ -634,11 +667,18 @@ size_t direct_scratch_bytes(int prec, int64_t n, int splits) {
 
 void launch_direct(const DirectLaunch& L) {
     RRG_REQUIRE(L.n > 0, RRG_ERR_INVALID, "direct sum: n must be positive");
-    if (L.sym_scratch) {
+    if (L.variant == 0 && env_variant() == 0) {
         int dev = 0;
         RRG_CUDA(cudaGetDevice(&dev));
-        launch_direct_sym(L, num_sms(dev));
-        return;
+        const int sms = num_sms(dev);
+        if (direct_small_applies(L.n, sms)) {
+            launch_direct_small(L, sms);
+            return;
+        }
+        if (L.sym_scratch) {
+            launch_direct_sym(L, sms);
+            return;
+        }
     }
     const int splits = L.splits > 0 ? L.splits : 1;
     const int64_t tiles = (L.n + kBS - 1) / kBS;
@@ -675,7 +715,8 @@ void launch_direct(const DirectLaunch& L) {
         }
         RRG_LAUNCHED();
         if (real_splits > 1) {
-            direct_f64_finish<<<div_up(L.n, 256), 256, 0, L.stream>>>(p, real_splits);
+            launch_pdl(direct_f64_finish, div_up(4 * L.n, kFinishThreads), kFinishThreads, 0,
+                       L.stream, p, real_splits);
             RRG_LAUNCHED();
         }
         return;
@@ -746,8 +787,9 @@ void launch_direct(const DirectLaunch& L) {
     }
     RRG_LAUNCHED();
     if (real_splits > 1) {
-        if (mixed) direct_f32_finish<true><<<div_up(L.n, 256), 256, 0, L.stream>>>(p, real_splits);
-        else direct_f32_finish<false><<<div_up(L.n, 256), 256, 0, L.stream>>>(p, real_splits);
+        auto* finish = mixed ? direct_f32_finish<true> : direct_f32_finish<false>;
+        launch_pdl(finish, div_up(4 * L.n, kFinishThreads), kFinishThreads, 0, L.stream, p,
+                   real_splits);
         RRG_LAUNCHED();
     }
 }

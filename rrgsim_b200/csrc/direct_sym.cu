@@ -32,6 +32,7 @@
 #include "direct_epi.cuh"
 #include "kernels.cuh"
 #include "pair_plan.cuh"
+#include "wave_cells.cuh"
 
 namespace rrg {
 namespace {
@@ -180,6 +181,7 @@ __global__ void __launch_bounds__(kBS, 2)
         return make_float2(rsqrt_sfu(r2.x), rsqrt_sfu(r2.y));
     };
 
+    pdl_next();  // (the finish may start and wait)
     load_i();
     int64_t base = pl.first_unit(a);
     fetch(static_cast<int64_t>(a) * pl.g + (u0 - base));
@@ -301,11 +303,12 @@ __global__ void __launch_bounds__(kBS, 2)
 }
 
 // ----------------------------------------------------------------------------------------------
-// FP64: G i-particles per thread. The reciprocal square root is CUDA's rsqrt (within 1 ulp)
-// instead of 1 / sqrt, whose square root and division each cost a Newton sequence on the FP64
-// pipe, the bound of this kernel. Per evaluation on B200, ordered pairs with 1 / sqrt -> ordered
-// pairs with rsqrt (direct_f64_kernel) -> here, us: N = 8,192 177 -> 116 -> 89; 20,011
-// 869 -> 538 -> 400 (relative error of the forces against 64-bit sums 4.0e-16 -> 3.5e-16).
+// FP64: G i-particles per thread. The reciprocal square root is rsqrt_pair instead of 1 / sqrt,
+// whose square root and division each cost a Newton sequence on the FP64 pipe, the bound of this
+// kernel; without a branch the pairs of a thread overlap. Per evaluation on B200, ordered pairs with
+// 1 / sqrt -> each pair once with CUDA's rsqrt -> with rsqrt_pair, us: N = 8,192 177 -> 89 -> 84;
+// 20,011 869 -> 400 -> 381; 32,768 2211 -> 982 -> 940 (relative error of the forces against 64-bit
+// sums at 20,011 4.0e-16 -> 3.5e-16).
 // ----------------------------------------------------------------------------------------------
 template <int G, bool USOFT, bool POT>
 struct Sym64 {
@@ -378,9 +381,10 @@ __global__ void __launch_bounds__(kBS, 2) direct_sym64_kernel(const SymParams<do
         dy = pj.y - yi[g];
         dz = pj.z - zi[g];
         const double s = USOFT ? hi[g] : hi[g] + hj;
-        return rsqrt(dx * dx + dy * dy + dz * dz + s);
+        return rsqrt_pair(dx * dx + dy * dy + dz * dz + s);
     };
 
+    pdl_next();  // (the finish may start and wait)
     load_i();
     int64_t base = pl.first_unit(a);
     fetch(static_cast<int64_t>(a) * pl.g + (u0 - base));
@@ -488,6 +492,8 @@ __global__ void __launch_bounds__(128) direct_sym_finish(const SymParams<R, S> p
                                                          const EpiDev<R> epi, bool want_pot) {
     const SymPlan& pl = p.plan;
     const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    pdl_next();
+    pdl_wait();
     if (k >= pl.n) return;
     const int a = static_cast<int>(k / (kBS * pl.g));
     const int cnt = pl.last_block(a) - pl.first_block(a) + 1;
@@ -616,8 +622,8 @@ size_t slot_bytes(int prec) {
 
 }  // namespace
 
-// From 32 j-tiles on: at N = 8,192 FP32 takes 34 us (ordered pairs 38), MIXED 47 (65), FP64 89
-// (116); at 6,000 33 (25) and FP64 77 (64), the units being too few to fill the SMs. Up to
+// From 32 j-tiles on: at N = 8,192 FP32 takes 34 us (ordered pairs 38), MIXED 47 (65), FP64 84
+// (109); at 6,000 33 (25) and FP64 77 (64), the units being too few to fill the SMs. Up to
 // 131,072 particles the slots stay below 600 MB.
 size_t direct_sym_scratch_bytes(int prec, int64_t n, bool umass, int sms) {
     if (!pair_plan_range(n)) return 0;
@@ -646,7 +652,8 @@ void launch_direct_sym(const DirectLaunch& L, int sms) {
         if (pl.g == 2) dispatch64<2>(usoft, L.want_pot, p, L.stream);
         else dispatch64<4>(usoft, L.want_pot, p, L.stream);
         RRG_LAUNCHED();
-        direct_sym_finish<double, double, false><<<bl, 128, 0, L.stream>>>(p, make_epi<double>(L.epi), L.want_pot);
+        launch_pdl(direct_sym_finish<double, double, false>, bl, 128, 0, L.stream, p,
+                   make_epi<double>(L.epi), L.want_pot);
         RRG_LAUNCHED();
         return;
     }
@@ -669,7 +676,8 @@ void launch_direct_sym(const DirectLaunch& L, int sms) {
         if (pl.g == 2) dispatch32<1, true>(usoft, L.want_pot, umass, p, L.stream);
         else dispatch32<2, true>(usoft, L.want_pot, umass, p, L.stream);
         RRG_LAUNCHED();
-        direct_sym_finish<float, double, true><<<bl, 128, 0, L.stream>>>(p, make_epi<float>(L.epi), L.want_pot);
+        launch_pdl(direct_sym_finish<float, double, true>, bl, 128, 0, L.stream, p,
+                   make_epi<float>(L.epi), L.want_pot);
     } else {
         SymParams<float, float> p{};
         fill(p);
@@ -677,7 +685,8 @@ void launch_direct_sym(const DirectLaunch& L, int sms) {
         else if (pl.g == 4) dispatch32<2, false>(usoft, L.want_pot, umass, p, L.stream);
         else dispatch32<4, false>(usoft, L.want_pot, umass, p, L.stream);
         RRG_LAUNCHED();
-        direct_sym_finish<float, float, false><<<bl, 128, 0, L.stream>>>(p, make_epi<float>(L.epi), L.want_pot);
+        launch_pdl(direct_sym_finish<float, float, false>, bl, 128, 0, L.stream, p,
+                   make_epi<float>(L.epi), L.want_pot);
     }
     RRG_LAUNCHED();
 }

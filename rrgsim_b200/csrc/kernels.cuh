@@ -53,6 +53,9 @@ void launch_direct(const DirectLaunch& L);
 // are the faster ones (launch_direct takes this path when sym_scratch is given).
 size_t direct_sym_scratch_bytes(int prec, int64_t n, bool umass, int sms);
 void launch_direct_sym(const DirectLaunch& L, int sms);
+// One launch, no splits (direct_small.cu), while its blocks of 32 particles fit one per SM.
+bool direct_small_applies(int64_t n, int sms);
+void launch_direct_small(const DirectLaunch& L, int sms);
 
 // VJP of a(x, m) (FP32): out_i = (d<lam,a>/dx_i, d<lam,a>/dm_i).
 void launch_direct_vjp_f32(const void* posm, const void* hsoft, float uniform_hsoft, int64_t n,
