@@ -429,8 +429,8 @@ RRG_API rrg_status rrg_ensemble_step_sequential(rrg_ensemble* e, int nsteps, int
 RRG_API rrg_status rrg_ensemble_synchronize(rrg_ensemble* e);
 /* Downloads the state (any pointer may be NULL), in the order given at creation. */
 RRG_API rrg_status rrg_ensemble_get(rrg_ensemble* e, double* pos, double* vel, double* acc);
-/* The tile variant (1: 2 i-particles per thread, 2: 4), j-chunk, work items and the timed
- * force evaluation the autotuner settled on. */
+/* The tile variant (1: 2 i-particles per thread, 2: 4; 3 and 4: each pair evaluated once, 4 and 8),
+ * j-chunk, work items (3 and 4: blocks) and the timed force evaluation the autotuner settled on. */
 RRG_API rrg_status rrg_ensemble_tuning(const rrg_ensemble* e, int* variant, int* jchunk,
                                        int* num_items, double* force_ms);
 

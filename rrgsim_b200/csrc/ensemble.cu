@@ -8,6 +8,12 @@
 // resident CTAs through an atomic counter. Small galaxies then no longer leave most of the GPU
 // idle, and the whole ensemble step is two launches. Each item writes its partial sums; a
 // finish pass adds them in a fixed order (deterministic) and applies the leapfrog epilogue.
+//
+// The other form of the force launch evaluates each unordered pair once (direct_sym.cu): the units
+// of all galaxies, galaxy after galaxy, are cut into one equal run of rounds per resident block.
+// The autotuner times both. Per step, ordered -> each pair once: 24 galaxies of 1,024 to 16,384
+// particles 491 -> 418 us, 64 of 1,024 to 65,536 12.7 -> 9.5 ms, 4 of 512 to 4,096 37.5 -> 30.5 us.
+// Bound: the FP32 pipe.
 #include <algorithm>
 #include <cmath>
 #include <string>
@@ -15,6 +21,8 @@
 
 #include "host_io.h"
 #include "kernels.cuh"
+#include "pair_plan.cuh"
+#include "wave_cells.cuh"
 
 namespace rrg {
 namespace {
@@ -59,6 +67,7 @@ __global__ void __launch_bounds__(kBS, 2) ens_forces_kernel(const EnsForceParams
     float* const fxy = reinterpret_cast<float*>(s_xy);
     float* const fzm = reinterpret_cast<float*>(s_zm);
     const int q0 = tid >> 1, e0 = tid & 1;
+    pdl_next();  // (the finish may start and wait)
     for (;;) {
         __syncthreads();  // previous item fully done with s_item and the tiles
         if (tid == 0) s_item = static_cast<int>(atomicAdd(p.counter, 1u));
@@ -136,6 +145,201 @@ __global__ void __launch_bounds__(kBS, 2) ens_forces_kernel(const EnsForceParams
     }
 }
 
+// ----------------------------------------------------------------------------------------------
+// Each unordered pair once. A galaxy's units are numbered from unit0; its slots (direct_sym.cu:
+// js [tiles - 1][n], is [islots][n]) start at record `slots`, js2 [blocks][kBS] is common.
+// ----------------------------------------------------------------------------------------------
+struct EnsPairGalaxy {
+    int64_t off, unit0, slots;
+    int32_t n, nt, tiles;
+    float h2, m;
+};
+
+struct EnsPairParams {
+    const V4<float>* posm;
+    const EnsPairGalaxy* gal;
+    int ngal, g, blocks;
+    int64_t rounds;
+    V4<float>* part;
+    V4<float>* js2;
+
+    __host__ __device__ int64_t run_start(int64_t b) const { return b * rounds / blocks; }
+    __host__ __device__ int block_of(int64_t round) const {
+        return static_cast<int>(((round + 1) * blocks - 1) / rounds);
+    }
+    __host__ __device__ int64_t first_unit(const EnsPairGalaxy& y, int64_t a) const {
+        return y.unit0 + a * y.nt - static_cast<int64_t>(g) * (a * (a - 1) / 2);
+    }
+    __host__ __device__ int first_block(const EnsPairGalaxy& y, int64_t a) const {
+        return block_of(8 * first_unit(y, a));
+    }
+    __host__ __device__ int last_block(const EnsPairGalaxy& y, int64_t a) const {
+        return block_of(8 * (first_unit(y, a) + y.nt - a * g) - 1);
+    }
+};
+
+// G2 packed pairs of i-particles per thread; direct_sym32_kernel's pair loop with a galaxy's
+// softening and (UMASS) mass.
+template <int G2, bool UMASS>
+__global__ void __launch_bounds__(kBS, 2) ens_pair_kernel(const EnsPairParams p) {
+    __shared__ float4 s_p[kBS];
+    __shared__ V4<float> s_j[kBS];
+    __shared__ float s_i[2 * G2 * 3][kBS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_next();  // (the finish may start and wait)
+    const int64_t q0 = p.run_start(blockIdx.x), q1 = p.run_start(blockIdx.x + 1);  // rounds
+    const int64_t u0 = q0 / kPairWarps, u1 = (q1 + kPairWarps - 1) / kPairWarps;     // units
+    // the galaxy and i-tile of the first unit
+    int lo = 0, hi = p.ngal - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (p.gal[mid].unit0 <= u0) lo = mid;
+        else hi = mid - 1;
+    }
+    int gi = lo;
+    EnsPairGalaxy y = p.gal[gi];
+    int a = 0;
+    while (a + 1 < y.tiles && p.first_unit(y, a + 1) <= u0) ++a;
+
+    float2 nx[G2], ny[G2], nz[G2], mi[G2], hs;
+    auto load_i = [&]() {
+        hs = dup2(y.h2);
+#pragma unroll
+        for (int g = 0; g < G2; ++g) {
+            V4<float> pi[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int i = a * (kBS * 2 * G2) + (2 * g + e) * kBS + tid;
+                pi[e] = i < y.n ? p.posm[y.off + i] : v4<float>(kPad, kPad, kPad, 0.f);
+            }
+            nx[g] = make_float2(-pi[0].x, -pi[1].x);
+            ny[g] = make_float2(-pi[0].y, -pi[1].y);
+            nz[g] = make_float2(-pi[0].z, -pi[1].z);
+            mi[g] = make_float2(pi[0].w, pi[1].w);
+        }
+#pragma unroll
+        for (int k = 0; k < 2 * G2 * 3; ++k) s_i[k][tid] = 0.f;
+    };
+    auto flush_i = [&]() {
+        const int slot = static_cast<int>(blockIdx.x) - p.first_block(y, a);
+        const float um = UMASS ? y.m : 1.f;
+#pragma unroll
+        for (int q = 0; q < 2 * G2; ++q) {
+            const int i = a * (kBS * 2 * G2) + q * kBS + tid;
+            if (i >= y.n) continue;
+            p.part[y.slots + static_cast<int64_t>(y.tiles - 1 + slot) * y.n + i] = v4<float>(
+                um * s_i[3 * q][tid], um * s_i[3 * q + 1][tid], um * s_i[3 * q + 2][tid], 0.f);
+        }
+    };
+    load_i();
+    int64_t base = p.first_unit(y, a);
+    for (int64_t u = u0; u < u1; ++u) {
+        if (u >= base + (y.nt - static_cast<int64_t>(a) * p.g)) {
+            flush_i();
+            if (++a == y.tiles) {
+                y = p.gal[++gi];
+                a = 0;
+            }
+            base = p.first_unit(y, a);
+            load_i();
+        }
+        const int t = static_cast<int>(a * p.g + (u - base));
+        const int r0 = u == u0 ? static_cast<int>(q0 - u0 * kPairWarps) : 0;
+        const int r1 = u + 1 == u1 ? static_cast<int>(q1 - u * kPairWarps) : kPairWarps;
+        const int j = t * kBS + tid;
+        const V4<float> pj = j < y.n ? p.posm[y.off + j] : v4<float>(kPad, kPad, kPad, 0.f);
+        __syncthreads();  // the tile before is done with (its j sums are stored)
+        s_p[tid] = make_float4(pj.x, pj.y, pj.z, pj.w);
+        s_j[tid] = v4<float>(0.f, 0.f, 0.f, 0.f);
+        __syncthreads();
+        float2 tx[G2], ty[G2], tz[G2];
+#pragma unroll
+        for (int g = 0; g < G2; ++g) tx[g] = ty[g] = tz[g] = make_float2(0.f, 0.f);
+        if (t < (a + 1) * p.g) {
+            // the i-tile's own j-tiles: i alone, every ordered pair
+#pragma unroll 4
+            for (int k = 32 * r0; k < 32 * r1; ++k) {
+                const float4 q = s_p[k];
+#pragma unroll
+                for (int g = 0; g < G2; ++g) {
+                    const float2 dx = __fadd2_rn(dup2(q.x), nx[g]);
+                    const float2 dy = __fadd2_rn(dup2(q.y), ny[g]);
+                    const float2 dz = __fadd2_rn(dup2(q.z), nz[g]);
+                    const float2 r2 =
+                        __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, hs)));
+                    const float2 inv = make_float2(rsqrt_sfu(r2.x), rsqrt_sfu(r2.y));
+                    const float2 minv = UMASS ? inv : __fmul2_rn(dup2(q.w), inv);
+                    const float2 kk = __fmul2_rn(minv, __fmul2_rn(inv, inv));
+                    tx[g] = __ffma2_rn(dx, kk, tx[g]);
+                    ty[g] = __ffma2_rn(dy, kk, ty[g]);
+                    tz[g] = __ffma2_rn(dz, kk, tz[g]);
+                }
+            }
+        } else {
+            for (int r = r0; r < r1; ++r) {
+                const int c = ((warp + r) & (kPairWarps - 1)) * 32;
+                const int from = (lane + 1) & 31;
+                float cx = 0.f, cy = 0.f, cz = 0.f;
+#pragma unroll 4
+                for (int s = 0; s < 32; ++s) {
+                    const float4 q = s_p[c + ((lane + s) & 31)];
+                    float2 jx = make_float2(cx, 0.f), jy = make_float2(cy, 0.f),
+                           jz = make_float2(cz, 0.f);
+#pragma unroll
+                    for (int g = 0; g < G2; ++g) {
+                        const float2 dx = __fadd2_rn(dup2(q.x), nx[g]);
+                        const float2 dy = __fadd2_rn(dup2(q.y), ny[g]);
+                        const float2 dz = __fadd2_rn(dup2(q.z), nz[g]);
+                        const float2 r2 =
+                            __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, hs)));
+                        const float2 inv = make_float2(rsqrt_sfu(r2.x), rsqrt_sfu(r2.y));
+                        const float2 inv2 = __fmul2_rn(inv, inv);
+                        float2 ki, kj;
+                        if constexpr (UMASS) {
+                            ki = kj = __fmul2_rn(inv, inv2);
+                        } else {
+                            ki = __fmul2_rn(__fmul2_rn(dup2(q.w), inv), inv2);
+                            kj = __fmul2_rn(__fmul2_rn(mi[g], inv), inv2);
+                        }
+                        tx[g] = __ffma2_rn(dx, ki, tx[g]);
+                        ty[g] = __ffma2_rn(dy, ki, ty[g]);
+                        tz[g] = __ffma2_rn(dz, ki, tz[g]);
+                        jx = __ffma2_rn(dx, kj, jx);
+                        jy = __ffma2_rn(dy, kj, jy);
+                        jz = __ffma2_rn(dz, kj, jz);
+                    }
+                    cx = __shfl_sync(0xffffffffu, half_sum(jx), from);
+                    cy = __shfl_sync(0xffffffffu, half_sum(jy), from);
+                    cz = __shfl_sync(0xffffffffu, half_sum(jz), from);
+                }
+                V4<float> v = s_j[c + lane];
+                v.x += cx;
+                v.y += cy;
+                v.z += cz;
+                s_j[c + lane] = v;
+                __syncthreads();  // the next warp to add to this chunk comes after
+            }
+            if (j < y.n) {
+                const float um = UMASS ? y.m : 1.f;
+                const V4<float> v = s_j[tid];
+                V4<float>* const to = r0 == 0 ? p.part + y.slots + static_cast<int64_t>(a) * y.n + j
+                                              : p.js2 + static_cast<int64_t>(blockIdx.x) * kBS + tid;
+                *to = v4<float>(-um * v.x, -um * v.y, -um * v.z, 0.f);
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < G2; ++g) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                s_i[3 * (2 * g + e)][tid] += e ? tx[g].y : tx[g].x;
+                s_i[3 * (2 * g + e) + 1][tid] += e ? ty[g].y : ty[g].x;
+                s_i[3 * (2 * g + e) + 2][tid] += e ? tz[g].y : tz[g].x;
+            }
+        }
+    }
+    flush_i();
+}
+
 struct EnsFinishParams {
     int64_t ntot;
     const int32_t* gid;
@@ -150,18 +354,42 @@ struct EnsFinishParams {
     int mode;  // EPI_STORE, EPI_CORRECT, EPI_CORRECT_PREDICT
 };
 
-// Fixed-order FP64 sum of a particle's partials + the leapfrog epilogue (as apply_epi).
-__global__ void __launch_bounds__(256) ens_finish_kernel(const EnsFinishParams p) {
+// Fixed-order FP64 sum of a particle's partials (PAIRS: its slots) + the leapfrog epilogue (as
+// apply_epi).
+template <bool PAIRS>
+__global__ void __launch_bounds__(128) ens_finish_kernel(const EnsFinishParams p,
+                                                         const EnsPairParams pr) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    pdl_next();
+    pdl_wait();
     if (i >= p.ntot) return;
-    const EnsGalaxy gg = p.gal[p.gid[i]];
-    const int64_t li = i - gg.off;
     double sx = 0, sy = 0, sz = 0;
-    for (int s = 0; s < gg.splits; ++s) {
-        const V4<float> v = p.part[gg.part_off + static_cast<int64_t>(s) * gg.n + li];
+    auto add = [&](const V4<float>& v) {
         sx += v.x;
         sy += v.y;
         sz += v.z;
+    };
+    if constexpr (PAIRS) {
+        const EnsPairGalaxy y = pr.gal[p.gid[i]];
+        const int k = static_cast<int>(i - y.off), t = k / kBS, a = t / pr.g;
+        const V4<float>* const js = pr.part + y.slots + k;
+#pragma unroll 4
+        for (int s = 0; s < a; ++s) {
+            add(js[static_cast<int64_t>(s) * y.n]);
+            // the second part of a unit that two runs share
+            const int64_t q = 8 * (pr.first_unit(y, s) + t - static_cast<int64_t>(s) * pr.g);
+            const int b = pr.block_of(q + 7);
+            if (pr.run_start(b) > q) add(pr.js2[static_cast<int64_t>(b) * kBS + (k & (kBS - 1))]);
+        }
+        const int cnt = pr.last_block(y, a) - pr.first_block(y, a) + 1;
+#pragma unroll 4
+        for (int s = 0; s < cnt; ++s) add(js[static_cast<int64_t>(y.tiles - 1 + s) * y.n]);
+    } else {
+        const EnsGalaxy gg = p.gal[p.gid[i]];
+        const int64_t li = i - gg.off;
+#pragma unroll 4
+        for (int s = 0; s < gg.splits; ++s)
+            add(p.part[gg.part_off + static_cast<int64_t>(s) * gg.n + li]);
     }
     const float ax = static_cast<float>(sx), ay = static_cast<float>(sy),
                 az = static_cast<float>(sz);
@@ -243,9 +471,12 @@ struct rrg_ensemble {
     std::vector<float> h2;
     std::vector<float> gmass;  // per-galaxy particle mass (all equal within every galaxy)
     bool umass = false;
-    DevBuf posm[2], vel, acc, u, gid, gal, items, part, counter;
+    DevBuf posm[2], vel, acc, u, gid, gal, items, part, counter, widened;
     int cur = 0;
-    int variant = 1;      // 1: G = 1 (2 i per thread), 2: G = 2 (4 i per thread)
+    // 1: G = 1 (2 i per thread), 2: G = 2 (4 i per thread); each pair once: 3: 4 i, 4: 8 i per thread
+    int variant = 1;
+    DevBuf pair_gal;
+    EnsPairParams pairs{};
     int jchunk = 4096;
     int num_items = 0;
     int grid = 0;
@@ -308,7 +539,67 @@ void build_worklist(rrg_ensemble* e, int variant, int jchunk) {
     drop_ens_graphs(e);
 }
 
+// The schedule of the kernels that evaluate each pair once, with g i-particles per thread.
+void build_pairs(rrg_ensemble* e, int variant) {
+    const int g = variant == 4 ? 8 : 4;
+    EnsPairParams p{};
+    p.ngal = e->ngal;
+    p.g = g;
+    std::vector<EnsPairGalaxy> gal(e->ngal);
+    int64_t units = 0;
+    for (int k = 0; k < e->ngal; ++k) {
+        EnsPairGalaxy& y = gal[k];
+        y.off = e->offs[k];
+        y.unit0 = units;
+        y.n = static_cast<int32_t>(e->counts[k]);
+        y.nt = (y.n + kBS - 1) / kBS;
+        y.tiles = (y.nt + g - 1) / g;
+        y.h2 = e->h2[k];
+        y.m = e->gmass[k];
+        units = p.first_unit(y, y.tiles - 1) + y.nt - static_cast<int64_t>(y.tiles - 1) * g;
+    }
+    p.rounds = 8 * units;
+    const int per_sm = variant == 4 ? (e->umass ? pair_blocks_per_sm(ens_pair_kernel<4, true>, 0)
+                                                : pair_blocks_per_sm(ens_pair_kernel<4, false>, 0))
+                                    : (e->umass ? pair_blocks_per_sm(ens_pair_kernel<2, true>, 0)
+                                                : pair_blocks_per_sm(ens_pair_kernel<2, false>, 0));
+    p.blocks = static_cast<int>(std::min<int64_t>(num_sms(e->device) * per_sm, units));
+    int64_t records = 0;
+    for (EnsPairGalaxy& y : gal) {
+        int islots = 1;
+        for (int a = 0; a < y.tiles; ++a)
+            islots = std::max(islots, p.last_block(y, a) - p.first_block(y, a) + 1);
+        y.slots = records;
+        records += static_cast<int64_t>(y.tiles - 1 + islots) * y.n;
+    }
+    e->pair_gal.alloc(sizeof(EnsPairGalaxy) * gal.size());
+    e->part.alloc(sizeof(V4<float>) * static_cast<size_t>(records + static_cast<int64_t>(p.blocks) * kBS));
+    RRG_CUDA(cudaMemcpy(e->pair_gal.p, gal.data(), sizeof(EnsPairGalaxy) * gal.size(),
+                        cudaMemcpyHostToDevice));
+    p.gal = e->pair_gal.as<EnsPairGalaxy>();
+    p.part = e->part.as<V4<float>>();
+    p.js2 = p.part + records;
+    e->pairs = p;
+    e->variant = variant;
+    e->jchunk = kBS;
+    e->num_items = p.blocks;
+    drop_ens_graphs(e);
+}
+
 void launch_forces(rrg_ensemble* e, const void* posm) {
+    if (e->variant >= 3) {
+        EnsPairParams p = e->pairs;
+        p.posm = static_cast<const V4<float>*>(posm);
+        if (e->variant == 4) {
+            if (e->umass) ens_pair_kernel<4, true><<<p.blocks, kBS, 0, e->stream>>>(p);
+            else ens_pair_kernel<4, false><<<p.blocks, kBS, 0, e->stream>>>(p);
+        } else {
+            if (e->umass) ens_pair_kernel<2, true><<<p.blocks, kBS, 0, e->stream>>>(p);
+            else ens_pair_kernel<2, false><<<p.blocks, kBS, 0, e->stream>>>(p);
+        }
+        RRG_LAUNCHED();
+        return;
+    }
     RRG_CUDA(cudaMemsetAsync(e->counter.p, 0, sizeof(unsigned int), e->stream));
     EnsForceParams p;
     p.posm = static_cast<const V4<float>*>(posm);
@@ -340,7 +631,8 @@ void launch_finish(rrg_ensemble* e, int mode, const void* posm, void* pos_out) {
     f.u = e->u.as<V4<float>>();
     f.dt = static_cast<float>(e->dt);
     f.mode = mode;
-    ens_finish_kernel<<<div_up(e->ntot, 256), 256, 0, e->stream>>>(f);
+    auto* finish = e->variant >= 3 ? ens_finish_kernel<true> : ens_finish_kernel<false>;
+    launch_pdl(finish, div_up(e->ntot, 128), 128, 0, e->stream, f, e->pairs);
     RRG_LAUNCHED();
 }
 
@@ -395,16 +687,22 @@ void run_steps(rrg_ensemble* e, int nsteps) {
     count_launches(1 + 2 * nsteps);
 }
 
-// Times one force evaluation per (variant, j-chunk) candidate and keeps the fastest.
+// Times one force evaluation per candidate (tile variant and j-chunk; each pair once) and keeps the
+// fastest.
 void autotune(rrg_ensemble* e) {
     cudaEvent_t a, b;
     RRG_CUDA(cudaEventCreate(&a));
     RRG_CUDA(cudaEventCreate(&b));
     float best = 1e30f;
     int bv = 1, bj = 4096;
-    for (int v : {1, 2}) {
+    for (int v : {1, 2, 3, 4}) {
         for (int j : {1024, 2048, 4096, 8192, 16384}) {
-            build_worklist(e, v, j);
+            if (v >= 3) {
+                if (j != 1024) break;  // (no j-chunk)
+                build_pairs(e, v);
+            } else {
+                build_worklist(e, v, j);
+            }
             launch_forces(e, e->posm[e->cur].p);  // warm
             RRG_CUDA(cudaEventRecord(a, e->stream));
             for (int r = 0; r < 2; ++r) launch_forces(e, e->posm[e->cur].p);
@@ -421,7 +719,8 @@ void autotune(rrg_ensemble* e) {
     }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
-    build_worklist(e, bv, bj);
+    if (bv >= 3) build_pairs(e, bv);
+    else build_worklist(e, bv, bj);
     e->tuned_ms = best / 2;
 }
 
@@ -579,17 +878,20 @@ RRG_API rrg_status rrg_ensemble_step_sequential(rrg_ensemble* e, int nsteps, int
 
 RRG_API rrg_status rrg_ensemble_get(rrg_ensemble* e, double* pos, double* vel, double* acc) {
     ENS_ENTRY(e, {
-        std::vector<V4<float>> hp(e->ntot), hv(e->ntot), ha(e->ntot);
-        const size_t vb = sizeof(V4<float>) * e->ntot;
+        // widened on the device, straight into the caller's arrays (131,000 particles: converting
+        // in host loops from three staging vectors took 5.7 ms)
+        const size_t each = 3 * static_cast<size_t>(e->ntot);
+        if (e->widened.bytes < 3 * each * sizeof(double)) e->widened.alloc(3 * each * sizeof(double));
+        double* d = e->widened.as<double>();
+        launch_unpack_state(RRG_PREC_FP32, e->ntot, nullptr, e->posm[e->cur].p, nullptr, e->vel.p,
+                            e->acc.p, nullptr, pos ? d : nullptr, vel ? d + each : nullptr,
+                            acc ? d + 2 * each : nullptr, nullptr, e->stream);
+        double* const out[3] = {pos, vel, acc};
+        for (int k = 0; k < 3; ++k)
+            if (out[k])
+                RRG_CUDA(cudaMemcpyAsync(out[k], d + k * each, each * sizeof(double),
+                                         cudaMemcpyDeviceToHost, e->stream));
         RRG_CUDA(cudaStreamSynchronize(e->stream));
-        RRG_CUDA(cudaMemcpy(hp.data(), e->posm[e->cur].p, vb, cudaMemcpyDeviceToHost));
-        RRG_CUDA(cudaMemcpy(hv.data(), e->vel.p, vb, cudaMemcpyDeviceToHost));
-        RRG_CUDA(cudaMemcpy(ha.data(), e->acc.p, vb, cudaMemcpyDeviceToHost));
-        for (int64_t i = 0; i < e->ntot; ++i) {
-            if (pos) { pos[3 * i] = hp[i].x; pos[3 * i + 1] = hp[i].y; pos[3 * i + 2] = hp[i].z; }
-            if (vel) { vel[3 * i] = hv[i].x; vel[3 * i + 1] = hv[i].y; vel[3 * i + 2] = hv[i].z; }
-            if (acc) { acc[3 * i] = ha[i].x; acc[3 * i + 1] = ha[i].y; acc[3 * i + 2] = ha[i].z; }
-        }
     })
 }
 

@@ -1,0 +1,41 @@
+"""The ensemble's force forms (ordered pairs, each pair once) against the FP64 oracle."""
+import numpy as np
+import pytest
+
+import oracle as orc
+import rrgsim_b200 as rg
+from helpers import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ngal,nmin,nmax", [(1, 1, 1), (3, 200, 700), (9, 3, 5000)])
+@pytest.mark.parametrize("masses", ["equal", "spread"])
+def test_every_form_of_the_forces_matches_the_oracle(ngal, nmin, nmax, masses):
+    """Galaxies of a particle to several i-tiles, equal masses or not: the accelerations that the
+    autotuned form (each pair once, or ordered pairs) leaves after two steps against the FP64
+    oracle's direct sum at the same positions, bar 1e-5 (median)."""
+    rng = np.random.default_rng(ngal)
+    counts = np.unique(np.linspace(nmin, nmax, ngal).astype(np.int64))
+    pos, vel, m, s2 = [], [], [], []
+    for k, n in enumerate(counts):
+        p, v = rg.generate_plummer(k + 1, int(n), 1.0, 1.0, 20.0)
+        pos.append(p)
+        vel.append(v)
+        w = np.full(n, 1.0 / n)
+        m.append(w if masses == "equal" else w * rng.uniform(0.5, 1.5, n))
+        s2.append((0.01 * (k + 1)) ** 2)
+    P, V, M = np.vstack(pos), np.vstack(vel), np.concatenate(m)
+    with rg.Ensemble(counts, P, V, M, np.array(s2), 1e-3, autotune=True) as e:
+        e.step(2)
+        got = e.get()
+    at = 0
+    for k, n in enumerate(counts):
+        p = got["pos"][at:at + n]
+        ref = orc.direct_acc(p, M[at:at + n], np.full(n, s2[k]))
+        a = got["acc"][at:at + n]
+        if n == 1:
+            np.testing.assert_array_equal(a, 0.0)
+        else:
+            assert np.median(rel_err(a, ref)) <= 1e-5
+        at += n

@@ -46,27 +46,3 @@ def test_l2_window_follows_the_context_stream():
     assert _window(cudart, s2_.cuda_stream).num_bytes == w.num_bytes
     c.close()  # and leaves the caller's stream with it
     assert _window(cudart, s2_.cuda_stream).num_bytes == 0
-
-
-def test_l2_set_aside_belongs_to_the_persistent_solve_grids():
-    """Grids without the persistent solve put no window on the stream, and the last context with
-    one gives the process's set-aside back."""
-    torch = pytest.importorskip("torch")
-    from cuda.bindings import runtime as cudart
-    limit = cudart.cudaLimit.cudaLimitPersistingL2CacheSize
-    pos, vel, m, s2 = disk(1000, seed=5)
-    for prec, nx in (("fp32", 40), ("fp32", 160), ("fp64", 64)):
-        s = torch.cuda.Stream()
-        with rg.Context(0, prec) as c:
-            c.load_particles(pos, vel, m, s2)
-            c.set_stream(s.cuda_stream)
-            c.init_grid(rg.GridInfo.from_values(nx, 16.0 / nx, 0.2))
-            assert _window(cudart, s.cuda_stream).num_bytes == 0
-    with rg.Context(0, "fp32") as c:
-        c.load_particles(pos, vel, m, s2)
-        c.init_grid(rg.GridInfo.from_values(64, 0.25, 0.2))
-        err, held = cudart.cudaDeviceGetLimit(limit)
-        assert err == cudart.cudaError_t.cudaSuccess
-        c.init_grid(rg.GridInfo.from_values(40, 0.4, 0.2))  # another grid: the window goes
-    err, after = cudart.cudaDeviceGetLimit(limit)
-    assert err == cudart.cudaError_t.cudaSuccess and (held == 0 or after < held)
