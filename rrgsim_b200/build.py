@@ -33,7 +33,7 @@ CXXFLAGS = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-I", str(INCLU
 
 LIB_SOURCES = ["direct.cu", "direct_sym.cu", "direct_small.cu", "integrate.cu", "pm.cu", "context.cu", "adjoint.cu", "host_io.cpp",
                "run.cpp", "noalloc.cu", "sort.cu", "ensemble.cu", "pm_adjoint.cu",
-               "wave_solve.cu"]
+               "wave_solve.cu", "wave_march.cu"]
 
 
 def _headers() -> list[Path]:

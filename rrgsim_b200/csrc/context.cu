@@ -349,7 +349,29 @@ bool solve_step_fused(rrg_ctx* c, const WaveCoef& w, int iterations, bool store_
         WaveCoef wi = w;
         wi.K_F = 1.0;
         int cur = first ? 1 : 0;
-        for (int k = first ? 1 : 0; k < (staged ? iterations : iterations - 1); ++k) {
+        int left = (staged ? iterations : iterations - 1) - (first ? 1 : 0);
+        if (!staged && left >= 3 && wave_march_applies(nx)) {
+            // three substeps per launch, to and fro between the increments and two free grids:
+            // the rest of the field buffer and the level before phi0. After an odd number of
+            // launches the increments end there, the last but one in the latter, which the last
+            // substep overwrites cell by cell. (PM step with 4M particles on 256^3, 20 substeps:
+            // 1075 -> 901 us.)
+            const int n = left / 3;
+            left -= 3 * n;
+            float* spare[2] = {a4 + 3 * nc, c->phi[1 - c->phi_cur].as<float>()};
+            const int to = n % 2 == 1 && left % 2 == 1 ? 1 : 0;
+            float *p[2] = {d[cur], d[1 - cur]}, *q[2] = {spare[to], spare[1 - to]};
+            for (int k = 0; k < n; ++k) {
+                launch_wave_march(nx, p[0], p[1], g, q[0], q[1], w.K_MAIN, w.K_ACTUAL, w.K_OLD,
+                                  1.0, c->stream);
+                std::swap(p[0], q[0]);
+                std::swap(p[1], q[1]);
+            }
+            d[0] = p[0];
+            d[1] = p[1];
+            cur = 0;
+        }
+        for (int k = 0; k < left; ++k) {
             launch_wave_step(c->prec, nx, d[cur], d[1 - cur], g, wi, nullptr, c->stream);
             cur = 1 - cur;
         }

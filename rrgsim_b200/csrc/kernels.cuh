@@ -138,6 +138,13 @@ void launch_wave_step(int prec, int nx, const void* phi, void* phi_old_inout, co
 // P <- km L6(C) + ka C + beta P, F += kf C.
 void launch_wave_adjoint_step(int prec, int nx, const void* C, void* P, void* F, double km,
                               double ka, double beta, double kf, cudaStream_t s);
+// Three substeps on a periodic FP32 grid (wave_march.cu): out = level 3, out_old = level 2, from
+// cur = level 0 and old = the level before it. The outputs are other buffers than the inputs; the
+// same bits as three launch_wave_step. wave_march_applies: on grids that do not stay in L2.
+bool wave_march_applies(int nx);
+void launch_wave_march(int nx, const float* cur, const float* old, const float* src, float* out,
+                       float* out_old, double km, double ka, double ko, double kf,
+                       cudaStream_t s);
 // a = -grad phi on the grid (rm_p2mesh.cu:238-290): acc4[c] = (ax, ay, az, phi[c]).
 void launch_gradient(int prec, int nx, double dx, const void* phi, void* acc4, cudaStream_t s);
 // One damped-wave update of four x-cells (wave_diss_iteration, wave.cu:106-193, periodic box,

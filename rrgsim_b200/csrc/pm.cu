@@ -429,7 +429,8 @@ __device__ __forceinline__ void block_max_to(double dmax, double amax, int tid,
 // the substep before it ends (no load is ahead of the wait).
 //
 // Bound: launch and L2 latency up to ~100^3, L2 bandwidth to ~160^3, HBM beyond (256^3: 268 MB in
-// 38.9 us, 1.05 of the copy peak, part of it L2 hits). Per substep in a graph on B200, us: one-cell
+// 38.9 us, 1.05 of the copy peak, part of it L2 hits; the fused FP32 solves take three substeps per
+// launch there, wave_march.cu). Per substep in a graph on B200, us: one-cell
 // columns (FP64, and rows that do not tile a warp) or float4 rows, chunks of up to 8 planes, normal
 // launches -> vectors everywhere and programmatic launches -> loads a plane ahead, 2 planes: FP32
 // 33^3 2.61 -> 2.05 -> 1.5, 64^3 2.39 -> 2.13 -> 1.72, 96^3 4.68 -> 3.05 -> 2.64, 128^3 4.59 -> 4.35
