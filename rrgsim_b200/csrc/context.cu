@@ -515,23 +515,6 @@ void alloc_step_partial(rrg_ctx* c) {
                               sizeof(double));
 }
 
-// `count` substeps on the full levels, the last one with the maxima of the steady check when
-// maxbits is given: one persistent launch where that applies (periodic FP32 / MIXED grids of 32,
-// 64 or 128 cells: 3.3 us per substep at 128^3 against 4.7 and a launch each), from the count on
-// at which its start (the levels and the source into the SMs and back, ~10 us) is paid.
-void wave_substeps(rrg_ctx* c, const WaveCoef& w, int count, unsigned long long* maxbits) {
-    if (count >= 8 && c->prec != RRG_PREC_FP64 && c->bc_type == RRG_BC_PERIODIC &&
-        !c->keep_layer &&
-        launch_wave_relax(c->grid.nx, count, c->phi[0].as<float>(), c->phi[1].as<float>(),
-                          c->phi_cur, c->src.as<float>(), w, maxbits,
-                          c->wsync.as<unsigned int>(), c->wsync.bytes, c->stream)) {
-        c->wave_solve_used = true;
-        if (count % 2 == 1) c->phi_cur = 1 - c->phi_cur;
-        return;
-    }
-    for (int k = 0; k < count; ++k) wave_substep(c, w, k + 1 == count ? maxbits : nullptr);
-}
-
 // Steady-state controlled relaxation (solve_wave_equation, wave.cu:230-297). Host-synchronous
 // only on check iterations.
 int solve_wave(rrg_ctx* c, int max_iterations, double* last_rel) {
@@ -546,20 +529,57 @@ int solve_wave(rrg_ctx* c, int max_iterations, double* last_rel) {
     double rel = -1.0;
     int it = 0;
     bool synced = false;
+    const int64_t every = c->wave.steady_check_step;
+    auto read = [&](void* to, const void* from, size_t bytes) {
+        RRG_CUDA(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, c->stream));
+        RRG_CUDA(cudaStreamSynchronize(c->stream));
+        synced = true;
+    };
     while (it < max_iterations) {
-        // up to and with the next substep that checks, or to the end
-        const int64_t every = c->wave.steady_check_step;
+        const int left = max_iterations - it;
+        // the next substep that checks
         const int64_t next = std::max<int64_t>(1, (it + every - 1) / every) * every;
         const bool check = next < max_iterations;
-        const int count = static_cast<int>(check ? next + 1 : max_iterations) - it;
-        if (check) RRG_CUDA(cudaMemsetAsync(c->maxbits.p, 0, 16, c->stream));
-        wave_substeps(c, w, count, check ? c->maxbits.as<unsigned long long>() : nullptr);
+        // the rest in one persistent launch, checks included, where that applies (periodic FP32 /
+        // MIXED grids of 32, 64 or 128 cells) and its start (the levels and the source into the
+        // SMs and back, ~10 us) is paid
+        if (left >= 8 && c->prec != RRG_PREC_FP64 && c->bc_type == RRG_BC_PERIODIC &&
+            !c->keep_layer) {
+            auto* checks = c->maxbits.as<RelaxCheck>();
+            auto* result = reinterpret_cast<RelaxResult*>(checks + kRelaxChecks);
+            const RelaxControl control{check ? static_cast<int>(next) - it : left,
+                                       static_cast<int>(every), hold, c->wave.steady_hold_steps,
+                                       c->wave.tolerance};
+            RRG_CUDA(cudaMemsetAsync(checks, 0, kRelaxBytes, c->stream));
+            if (launch_wave_relax(c->grid.nx, left, c->phi[0].as<float>(), c->phi[1].as<float>(),
+                                  c->phi_cur, c->src.as<float>(), w, control, checks, result,
+                                  c->wsync.as<unsigned int>(), c->wsync.bytes, c->stream)) {
+                c->wave_solve_used = true;
+                RelaxResult r{rel, left, hold};
+                if (check) {
+                    read(&r, result, sizeof r);
+                    if (r.done == 0) {
+                        check_wave_solve(c);
+                        throw Error(RRG_ERR_CUDA, "wave solve: the relaxation did not run");
+                    }
+                }
+                it += r.done;
+                if (r.done % 2 == 1) c->phi_cur = 1 - c->phi_cur;
+                rel = r.rel;
+                hold = r.hold;
+                if (check && hold >= c->wave.steady_hold_steps) break;
+                continue;
+            }
+        }
+        // up to and with the next substep that checks, or to the end
+        const int count = check ? static_cast<int>(next) + 1 - it : left;
+        unsigned long long* maxbits = check ? c->maxbits.as<unsigned long long>() : nullptr;
+        if (check) RRG_CUDA(cudaMemsetAsync(maxbits, 0, 16, c->stream));
+        for (int k = 0; k < count; ++k) wave_substep(c, w, k + 1 == count ? maxbits : nullptr);
         it += count;
         if (check) {
             unsigned long long bits[2];
-            RRG_CUDA(cudaMemcpyAsync(bits, c->maxbits.p, 16, cudaMemcpyDeviceToHost, c->stream));
-            RRG_CUDA(cudaStreamSynchronize(c->stream));
-            synced = true;
+            read(bits, maxbits, 16);
             double d, a;
             std::memcpy(&d, &bits[0], 8);
             std::memcpy(&a, &bits[1], 8);
@@ -1117,7 +1137,7 @@ RRG_API rrg_status rrg_init_grid(rrg_ctx* ctx, const rrg_grid_info* grid) {
         ctx->acc4.alloc(nc * v4b(ctx));
         ctx->src.alloc(nc * ctx->rsz);
         apply_l2_window(ctx);
-        ctx->maxbits.alloc(16);
+        ctx->maxbits.alloc(kRelaxBytes);
         ctx->wsync.alloc(wave_solve_sync_bytes(grid->nx));
         for (Buf* b : {&ctx->mg[0], &ctx->mg[1], &ctx->src, &ctx->phi[0], &ctx->phi[1],
                        &ctx->acc4, &ctx->maxbits, &ctx->wsync})

@@ -261,13 +261,32 @@ bool launch_wave_solve(int nx, int iterations, float* phi0, float* phi1, int cur
                        const unsigned long long* mg, unsigned long long* mg_zero, int shift_s,
                        double dx, double rho_sub, const WaveCoef& w, float* src, float4* acc4,
                        unsigned int* sync, size_t sync_bytes, cudaStream_t s);
-// `iterations` substeps on the full levels (the operator path) in the same persistent kernel's
-// other form, the source read from src: the same bits as launch_wave_step x iterations. maxbits
-// != nullptr: the last substep's max|dphi|, max|phi| folded into maxbits[0..1] as
-// launch_wave_step does. Returns false, launching nothing, where it does not apply.
+// Up to `iterations` substeps on the full levels (the operator path) in the same persistent kernel's
+// other form, the source read from src: the same bits as launch_wave_step x the substeps run. The
+// substeps control.first, control.first + control.every, ... (from 0; none from `iterations` on) are
+// steady checks: max|dphi| / (max|phi| + 1e-30) below the tolerance hold_steps times in a row (hold
+// of them before this launch) ends the run, and so does the last of kRelaxChecks checks. `checks` and
+// `result` must be zeroed; result->done == 0 afterwards: the launch failed. Returns false, launching
+// nothing, where it does not apply.
+constexpr int kRelaxChecks = 128;
+struct RelaxCheck {
+    unsigned long long dmax, amax;  // bit patterns of doubles
+    unsigned int arrived, pad[3];
+};
+struct RelaxResult {
+    double rel;  // of the last check, -1 without one
+    int done;    // substeps run
+    int hold;
+};
+constexpr size_t kRelaxBytes = kRelaxChecks * sizeof(RelaxCheck) + sizeof(RelaxResult);
+struct RelaxControl {
+    int first, every, hold, hold_steps;
+    double tolerance;
+};
 bool launch_wave_relax(int nx, int iterations, float* phi0, float* phi1, int cur,
-                       const float* src, const WaveCoef& w, unsigned long long* maxbits,
-                       unsigned int* sync, size_t sync_bytes, cudaStream_t s);
+                       const float* src, const WaveCoef& w, const RelaxControl& control,
+                       RelaxCheck* checks, RelaxResult* result, unsigned int* sync,
+                       size_t sync_bytes, cudaStream_t s);
 // Trilinear gather of acc4 to particles (rm_mesh2p.cu:48-114).
 void launch_interp(int prec, int64_t n, const void* posm, const void* poslo, const GridDev& g,
                    const void* acc4, void* acc, cudaStream_t s);

@@ -58,9 +58,11 @@
 // much as the 20 one-deep ones.
 //
 // The operator path (setup relaxation, rrg_solve_wave_equation) runs the same kernel on the full
-// levels (FULL): the substeps between two steady checks in one launch, the check's maxima from
-// the registers of the last one. 300 substeps with their nine checks at 128^3: 2.19 ms one launch
-// per substep (4.7 us each and their launches) -> 1.32 ms.
+// levels (FULL), steady checks included: the checking substep's maxima go from the registers to
+// one word pair per check while the faces are exchanged, and when every block's have arrived each
+// block takes the same decision. 300 substeps with their nine checks at 128^3: 2.19 ms one launch
+// per substep (4.7 us each and their launches), 1.32 ms one launch per check that the host waits
+// for, 1.12 ms now (1,500 substeps with 50 checks, deposit and downloads: 10.8, 6.6, 5.6 ms).
 //
 // All blocks must be resident together: the launch is cooperative and the host checks capacity
 // first. Every wait is bounded; one that runs out sets the error word and the block leaves (the
@@ -136,8 +138,12 @@ struct SolveArgs {
     double kf_d, km_d, kao_d;         // K_F, K_MAIN, K_ACTUAL + K_OLD - 1 for the increments' source
     float* src;                     // nullptr, or where the source is also stored
     float4* acc4;                   // nullptr: no gradient
-    unsigned long long* maxbits;    // FULL: nullptr, or where max|dphi|, max|phi| of the last
-                                    // substep are folded in
+    // FULL, the steady check: the substeps first_check, first_check + every, ... (from 0) check;
+    // hold passes so far of hold_steps in a row below the tolerance
+    RelaxCheck* checks;             // kRelaxChecks of them, zeroed
+    RelaxResult* result;
+    int first_check, every, hold, hold_steps;
+    double tolerance;
     unsigned int* sync;             // sync_bytes_for(blocks), zeroed before the first launch
 };
 
@@ -153,6 +159,7 @@ __global__ void __launch_bounds__(kThreads, 2) wave_solve_kernel(const SolveArgs
     float4* const srcs = zh + S::zhN;         // [ZC][kThreads]
     __shared__ int fail_s;
     __shared__ unsigned int base_s;
+    __shared__ double dmax_s[kThreads / 32], amax_s[kThreads / 32], rel_s;
 
     volatile unsigned int* const err = a.sync + kErrWord;
     unsigned int* const counters = a.sync + (blockIdx.y * gridDim.x + blockIdx.x) * kCounterStride;
@@ -341,6 +348,10 @@ __global__ void __launch_bounds__(kThreads, 2) wave_solve_kernel(const SolveArgs
         for (int i = tid; i < S::zhN; i += kThreads) zh[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         __syncthreads();
     }
+    int done = a.iterations;  // (FULL: fewer when the check stops the run)
+    unsigned int check_at = a.first_check;  // (t + every may pass INT_MAX)
+    int hold = a.hold, nchecks = 0;
+    double rel = -1.0;
     for (int t = 0; t < a.iterations; ++t) {
         const bool last = t + 1 == a.iterations;
         float4 zm = zh[r * W + q];
@@ -362,15 +373,77 @@ __global__ void __launch_bounds__(kThreads, 2) wave_solve_kernel(const SolveArgs
             store_faces(e0 + t + 1, k, cur[k]);
         }
         const unsigned int e = e0 + t + 1;
+        const bool check = FULL && static_cast<unsigned int>(t) == check_at;
+        if (check) {
+            // this substep's max |dphi| and max |phi|, differences in FP64 as
+            // wave_periodic_vec_kernel takes them
+            double dmax = 0.0;
+            float amax = 0.f;
+#pragma unroll
+            for (int k = 0; k < ZC; ++k) {
+                const float4 c = cur[k], o = old[k];
+                dmax = fmax(dmax, fmax(fmax(fabs(double(c.x) - double(o.x)), fabs(double(c.y) - double(o.y))),
+                                       fmax(fabs(double(c.z) - double(o.z)), fabs(double(c.w) - double(o.w)))));
+                amax = fmaxf(amax, fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(c.z), fabsf(c.w))));
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                dmax = fmax(dmax, __shfl_down_sync(0xffffffffu, dmax, o));
+                amax = fmaxf(amax, __shfl_down_sync(0xffffffffu, amax, o));
+            }
+            if (lane == 0) {
+                dmax_s[tid >> 5] = dmax;
+                amax_s[tid >> 5] = static_cast<double>(amax);
+            }
+        }
         publish(e);  // (its barrier also ends this substep's reads of the tile and halo)
         // (the last exchange gives the gradient its halo; it also keeps every block's final
         // writes after its neighbours' reads of phi0's halo, even without a gradient)
+        if (check && tid == 32) {  // (a warp that does not poll)
+            double d = dmax_s[0], m = amax_s[0];
+            for (int i = 1; i < kThreads / 32; ++i) {
+                d = fmax(d, dmax_s[i]);
+                m = fmax(m, amax_s[i]);
+            }
+            // (non-negative doubles compare as their bit patterns)
+            RelaxCheck* const ck = a.checks + nchecks;
+            atomicMax(&ck->dmax, static_cast<unsigned long long>(__double_as_longlong(d)));
+            atomicMax(&ck->amax, static_cast<unsigned long long>(__double_as_longlong(m)));
+            __threadfence();
+            atomicAdd(&ck->arrived, 1u);
+        }
         if (!exchange(e)) return;
+        if (check) {
+            // every block's maxima (they arrive during the exchange); all blocks decide alike
+            RelaxCheck* const ck = a.checks + nchecks;
+            if (tid == 0) {
+                const long long t0 = clock64();
+                for (unsigned int polls = 1; ld_acquire(&ck->arrived) != static_cast<unsigned int>(nblocks); ++polls) {
+                    if (clock64() - t0 > kWaitCycles || ((polls & 255u) == 0 && *err != 0)) {
+                        fail_s = 1;
+                        atomicExch(a.sync + kErrWord, 1u);
+                        break;
+                    }
+                }
+                const double d = __longlong_as_double(static_cast<long long>(__ldcg(&ck->dmax)));
+                const double m = __longlong_as_double(static_cast<long long>(__ldcg(&ck->amax)));
+                rel_s = d / (m + 1e-30);
+            }
+            __syncthreads();
+            if (fail_s) return;
+            rel = rel_s;
+            hold = rel < a.tolerance ? hold + 1 : 0;
+            if (hold >= a.hold_steps || ++nchecks == kRelaxChecks) {
+                done = t + 1;
+                break;
+            }
+            check_at += a.every;
+        }
     }
 
     // ---- the levels to global memory (only this thread reads them in this launch) ---------
     {
-        const bool fin0 = (a.cur ^ (a.iterations & 1)) == 0;
+        const bool fin0 = (a.cur ^ (done & 1)) == 0;
         float4* fin = reinterpret_cast<float4*>(fin0 ? a.phi0 : a.phi1);
         float4* prv = reinterpret_cast<float4*>(fin0 ? a.phi1 : a.phi0);
 #pragma unroll
@@ -381,29 +454,7 @@ __global__ void __launch_bounds__(kThreads, 2) wave_solve_kernel(const SolveArgs
     }
 
     if constexpr (FULL) {
-        if (a.maxbits == nullptr) return;
-        // the last substep's max |dphi| and max |phi|, differences in FP64 as
-        // wave_periodic_vec_kernel takes them
-        double dmax = 0.0;
-        float amax = 0.f;
-#pragma unroll
-        for (int k = 0; k < ZC; ++k) {
-            const float4 c = cur[k], o = old[k];
-            dmax = fmax(dmax, fmax(fmax(fabs(double(c.x) - double(o.x)), fabs(double(c.y) - double(o.y))),
-                                   fmax(fabs(double(c.z) - double(o.z)), fabs(double(c.w) - double(o.w)))));
-            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(c.z), fabsf(c.w))));
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            dmax = fmax(dmax, __shfl_down_sync(0xffffffffu, dmax, o));
-            amax = fmaxf(amax, __shfl_down_sync(0xffffffffu, amax, o));
-        }
-        if (lane == 0) {
-            // (non-negative doubles compare as their bit patterns)
-            atomicMax(a.maxbits, static_cast<unsigned long long>(__double_as_longlong(dmax)));
-            atomicMax(a.maxbits + 1, static_cast<unsigned long long>(
-                                         __double_as_longlong(static_cast<double>(amax))));
-        }
+        if (me == 0 && tid == 0) *a.result = RelaxResult{rel, done, hold};
         return;
     }
     // ---- gradient of the final level (its halo is in place): central inside, one-sided at
@@ -451,7 +502,7 @@ __global__ void __launch_bounds__(kThreads, 2) wave_solve_kernel(const SolveArgs
             for (int i = 0; i < 4; ++i) o[i * 32 + lane] = st[i * 32 + lane];
         }
     }
-    // the counter ends at e0 + iterations in every block: the next launch starts from there
+    // the counter ends at e0 + done in every block: the next launch starts from there
 }
 
 
@@ -1010,8 +1061,9 @@ bool launch_wave_solve(int nx, int iterations, float* phi0, float* phi1, int cur
 }
 
 bool launch_wave_relax(int nx, int iterations, float* phi0, float* phi1, int cur,
-                       const float* src, const WaveCoef& w, unsigned long long* maxbits,
-                       unsigned int* sync, size_t sync_bytes, cudaStream_t s) {
+                       const float* src, const WaveCoef& w, const RelaxControl& control,
+                       RelaxCheck* checks, RelaxResult* result, unsigned int* sync,
+                       size_t sync_bytes, cudaStream_t s) {
     if (!wave_solve_applicable(nx) || iterations < 1 || (nx == 128 && use_tb())) return false;
     SolveArgs a{};
     a.phi0 = phi0;
@@ -1023,7 +1075,13 @@ bool launch_wave_relax(int nx, int iterations, float* phi0, float* phi1, int cur
     a.ko = static_cast<float>(w.K_OLD);
     a.kf = static_cast<float>(w.K_F);
     a.src = const_cast<float*>(src);
-    a.maxbits = maxbits;
+    a.checks = checks;
+    a.result = result;
+    a.first_check = control.first;
+    a.every = control.every;
+    a.hold = control.hold;
+    a.hold_steps = control.hold_steps;
+    a.tolerance = control.tolerance;
     a.sync = sync;
     return launch_persistent(nx, true, false, a, sync_bytes, s);
 }
