@@ -3,7 +3,7 @@
 // damped-wave substeps (wave_diss_iteration, wave.cu:106-193), then the gradient
 // (calc_acceleration_field_, rm_p2mesh.cu:238-290).
 //
-// Decomposition: a block of 256 threads owns RB = 256 / W rows (y) x ZC planes (z) of whole
+// Decomposition: a block of 256 threads owns RB = 256 / W rows (y) x ZC (8 or 2) planes (z) of whole
 // x-rows, W = nx / 4 float4 per row; a thread owns one float4 column (four x-cells of one row,
 // all ZC planes) and keeps its current and previous level in registers and its source in
 // shared memory for the whole solve. The x neighbours are warp shuffles (a warp holds whole
@@ -80,7 +80,10 @@ namespace rrg {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kZC = 8;                          // planes per block
+// planes per block: 8 on 128^3 (256 blocks, two per SM); 2 on 64^3 and 32^3, where 8 leave most
+// SMs idle (32 and 4 blocks): a solve of 20 substeps on 64^3 69.9 -> 47.8 us, 32^3 60.1 -> 45.2.
+constexpr int kZC = 8;
+constexpr int planes_of(int W) { return W == 32 ? kZC : 2; }
 constexpr long long kWaitCycles = 1ll << 28;    // ~0.14 s at 1.9 GHz per wait at most
 constexpr int kCounterStride = 32;              // a block's epoch counter: 128 bytes apart
 constexpr int kErrWord = 16383;                 // in the first 64 KB: counters, error word
@@ -96,14 +99,17 @@ size_t sync_bytes_for(int64_t nblocks) {
 template <int W>
 struct Shape {
     static constexpr int nx = 4 * W;
+    static constexpr int ZC = planes_of(W);           // planes per block
     static constexpr int RB = kThreads / W;           // rows per block
-    static constexpr int Hy = kZC * W;                // float4 of a y face (ZC slots of W)
+    static constexpr int Hy = ZC * W;                // float4 of a y face (ZC slots of W)
     static constexpr int Hz = RB * W;                 // float4 of a z face (RB slots) = 256
     static constexpr int Hn = 2 * Hy + 2 * Hz;        // a block's halo: y-, y+, z-, z+
     static constexpr int NH = (Hn + kThreads - 1) / kThreads;  // halo float4 per thread
-    static constexpr int tileN = kZC * (RB + 2) * W;  // y tile: rows y0 - 1 .. y0 + RB
+    static constexpr int tileN = ZC * (RB + 2) * W;  // y tile: rows y0 - 1 .. y0 + RB
     static constexpr int zhN = 2 * RB * W;            // z halo planes z0 - 1 and z0 + ZC
-    static constexpr size_t smem = (tileN + zhN + kZC * kThreads) * sizeof(float4);
+    // the source, [ZC][kThreads]; the gradient stages four float4 per thread in it
+    static constexpr int srcN = (ZC > 4 ? ZC : 4) * kThreads;
+    static constexpr size_t smem = (tileN + zhN + srcN) * sizeof(float4);
 };
 
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
@@ -152,11 +158,11 @@ struct SolveArgs {
 template <int W, bool FULL>
 __global__ void __launch_bounds__(kThreads, 2) wave_solve_kernel(const SolveArgs a) {
     using S = Shape<W>;
-    constexpr int nx = S::nx, RB = S::RB, ZC = kZC;
+    constexpr int nx = S::nx, RB = S::RB, ZC = S::ZC;
     extern __shared__ __align__(16) float4 sm[];
     float4* const tile = sm;                  // [ZC][RB + 2][W]
     float4* const zh = sm + S::tileN;         // [2][RB][W]
-    float4* const srcs = zh + S::zhN;         // [ZC][kThreads]
+    float4* const srcs = zh + S::zhN;         // [ZC][kThreads], srcN
     __shared__ int fail_s;
     __shared__ unsigned int base_s;
     __shared__ double dmax_s[kThreads / 32], amax_s[kThreads / 32], rel_s;
@@ -948,7 +954,7 @@ void launch_cooperative(cudaLaunchConfig_t& cfg, bool full, const SolveArgs& a) 
 
 int64_t block_count(int nx) {
     const int W = nx / 4, RB = kThreads / W;
-    return static_cast<int64_t>(nx / RB) * (nx / kZC);
+    return static_cast<int64_t>(nx / RB) * (nx / planes_of(W));
 }
 
 }  // namespace
@@ -972,7 +978,7 @@ namespace {
 bool launch_persistent(int nx, bool full, bool tbk, const SolveArgs& a, size_t sync_bytes,
                        cudaStream_t s) {
     const int W = nx / 4, RB = (tbk ? tb::T : kThreads) / W;
-    const dim3 grid(nx / RB, nx / kZC);
+    const dim3 grid(nx / RB, nx / planes_of(W));
     const int64_t nblocks = static_cast<int64_t>(grid.x) * grid.y;
     RRG_REQUIRE(nblocks * kCounterStride < kErrWord &&
                     sync_bytes >= (tbk ? sync_bytes_tb(nblocks) : sync_bytes_for(nblocks)),
