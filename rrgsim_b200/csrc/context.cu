@@ -284,12 +284,9 @@ void wave_source(rrg_ctx* c, bool zero_other) {
     // reads mg[mg_cur]; clears mg[1 - mg_cur] when asked (the next deposit target)
     const double rho_sub = (c->bc_type == RRG_BC_PERIODIC) ? c->rho_mean : 0.0;
     launch_wave_source(c->prec, c->grid.nx, c->mg[c->mg_cur].as<unsigned long long>(),
-                       c->shift_s, c->grid.dx, rho_sub, 1.0, c->src.p, false, c->stream);
-    if (zero_other) {
-        // cleared with a memset node: the source kernel must not touch the deposit it reads
-        RRG_CUDA(cudaMemsetAsync(c->mg[1 - c->mg_cur].p, 0, c->mg[1 - c->mg_cur].bytes,
-                                 c->stream));
-    }
+                       c->shift_s, c->grid.dx, rho_sub, 1.0, c->src.p,
+                       zero_other ? c->mg[1 - c->mg_cur].as<unsigned long long>() : nullptr,
+                       c->stream);
     c->src_dirty = false;
     c->src_valid = true;
 }

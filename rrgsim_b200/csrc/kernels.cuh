@@ -126,10 +126,10 @@ void launch_cic_deposit(int prec, int64_t n, const void* posm, const void* poslo
                         const GridDev& g, int shift_s, unsigned long long* grid,
                         cudaStream_t s);
 // Wave source from the fixed-point mass: src = 4 pi G (m 2^-S / dx^3 - rho_mean) [* K_F when
-// uniform], stored in R; optionally zeroes the fixed-point grid.
+// uniform], stored in R; zero_grid (mgrid itself or another fixed-point grid), if given, is cleared.
 void launch_wave_source(int prec, int nx, const unsigned long long* mgrid, int shift_s,
-                        double dx, double rho_mean, double scale, void* src, bool zero_grid,
-                        cudaStream_t s);
+                        double dx, double rho_mean, double scale, void* src,
+                        unsigned long long* zero_grid, cudaStream_t s);
 // One damped-wave substep (wave.cu:106-193): phi_old_inout <- phi_new.
 // If maxbits != nullptr also folds max|phi_new - phi| and max|phi_new| into maxbits[0..1].
 void launch_wave_step(int prec, int nx, const void* phi, void* phi_old_inout, const void* src,

@@ -232,13 +232,14 @@ __global__ void __launch_bounds__(256) cic_kernel(int64_t n, const void* __restr
 // FP64 divides by dx^3 as the reference does; FP32, whose source is rounded to float anyway,
 // multiplies by the host's 1 / dx^3 (an FP64 division per cell made this pass instruction-bound).
 template <typename R>
-__global__ void wave_source_kernel(int64_t ncells, unsigned long long* __restrict__ mgrid,
+__global__ void wave_source_kernel(int64_t ncells, const unsigned long long* mgrid,
                                    double inv_scale, double dx3, double inv_dx3, double rho_sub,
-                                   double mult, R* __restrict__ src, bool zero_grid) {
+                                   double mult, R* src, unsigned long long* zero_grid) {
     const int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    pdl_wait();
     if (c >= ncells) return;
     const unsigned long long q = mgrid[c];
-    if (zero_grid) mgrid[c] = 0ull;
+    if (zero_grid) zero_grid[c] = 0ull;  // (mgrid itself, or the next deposit's grid)
     if constexpr (sizeof(R) == 8) {
         const double mass = static_cast<double>(q) * inv_scale;
         const double rho = mass / dx3 - rho_sub;
@@ -254,21 +255,25 @@ __global__ void wave_source_kernel(int64_t ncells, unsigned long long* __restric
 // Bound: HBM at 256^3 (32 to 36 B per cell); below, the FP64 arithmetic of g.
 template <int V, bool FIRST>
 __global__ void __launch_bounds__(256) wave_inc_prep_kernel(
-    int nx, const unsigned long long* __restrict__ mg, unsigned long long* __restrict__ mg_zero,
-    double inv_scale, double inv_dx3, double rho_sub, const float* __restrict__ phi0,
-    const float* __restrict__ phi_prev, double kf, double km, double kao, float ko,
-    float* __restrict__ g, float* __restrict__ d, float* __restrict__ d_old,
-    float* __restrict__ src) {
+    int nx, const unsigned long long* mg, unsigned long long* mg_zero,
+    double inv_scale, double inv_dx3, double rho_sub, const float* phi0,
+    const float* phi_prev, double kf, double km, double kao, float ko,
+    float* g, float* d, float* d_old,
+    float* src) {
     using C = Cells<float, V>;
     const int W = nx / V;
     const int64_t u = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t units = static_cast<int64_t>(W) * nx * nx;
-    if (u >= units) return;
+    if (u >= units) {  // (every block waits)
+        pdl_wait();
+        return;
+    }
     const int q = static_cast<int>(u % W);
     const int64_t row = u / W;
     const int y = static_cast<int>(row % nx), z = static_cast<int>(row / nx);
     const int64_t plane = static_cast<int64_t>(nx) * nx;
     const int64_t c = row * nx + q * V;
+    pdl_wait();
     auto cells = [&](int64_t at) { return *reinterpret_cast<const C*>(phi0 + at); };
     const C p = cells(c), pp = *reinterpret_cast<const C*>(phi_prev + c);
     const float l = phi0[row * nx + (q == 0 ? nx : q * V) - 1];
@@ -646,101 +651,98 @@ __global__ void __launch_bounds__(kTX* kTY, 2) wave_step_kernel(
 // Gradient (calc_acceleration_field_, rm_p2mesh.cu:238-290): central differences inside,
 // one-sided at the faces, a = -dphi / dx. Output cell (ax, ay, az, phi).
 // ----------------------------------------------------------------------------------------------
-template <typename R>
-__global__ void __launch_bounds__(kTX* kTY) gradient_kernel(int nx, R coef,
-                                                            const R* __restrict__ phi,
-                                                            V4<R>* __restrict__ acc4) {
-    const int x = blockIdx.x * kTX + threadIdx.x;
-    const int y = blockIdx.y * kTY + threadIdx.y;
-    const int z = blockIdx.z;
-    if (x >= nx || y >= nx) return;
-    const int64_t sx = 1, sy = nx, sz = static_cast<int64_t>(nx) * nx;
-    const int64_t c = x + y * sy + z * sz;
-    const R pc = phi[c];
-    R dx, dy, dz;
-    if (x == 0) dx = phi[c + sx] - pc;
-    else if (x == nx - 1) dx = pc - phi[c - sx];
-    else dx = R(0.5) * (phi[c + sx] - phi[c - sx]);
-    if (y == 0) dy = phi[c + sy] - pc;
-    else if (y == nx - 1) dy = pc - phi[c - sy];
-    else dy = R(0.5) * (phi[c + sy] - phi[c - sy]);
-    if (z == 0) dz = phi[c + sz] - pc;
-    else if (z == nx - 1) dz = pc - phi[c - sz];
-    else dz = R(0.5) * (phi[c + sz] - phi[c - sz]);
-    acc4[c] = v4<R>(dx * coef, dy * coef, dz * coef, pc);
-}
-
-// FP32 gradient with four x-cells per thread (float4 rows, as wave_periodic_vec_kernel): x +- 1
-// by warp shuffles (a scalar load where a warp ends inside a row), rows y +- 1 as coalesced
-// float4 loads, the z neighbours from a register pipeline over ZC planes, and the four
-// (ax, ay, az, phi) cells written as four float4 stores. Same expressions, faces one-sided, as
-// gradient_kernel. Needs nx % 4 == 0 and nx % ZC == 0.
-template <int ZC, int BS>
-__global__ void __launch_bounds__(BS) gradient_x4_kernel(int nx, float coef,
-                                                         const float* __restrict__ phi,
-                                                         float4* __restrict__ acc4) {
-    const int W = nx >> 2;
-    const int plane4 = W * nx;
+// V consecutive x-cells per thread and ZC planes, as wave_periodic_vec_kernel: x +- 1 by warp
+// shuffles (a scalar load where a warp ends inside a row), rows y +- 1 as coalesced vector loads a
+// plane ahead, the z neighbours in registers. A warp's 32 V cells are consecutive in memory: they
+// are staged in shared memory and stored 512 contiguous bytes per instruction (64-byte strides
+// before: 256^3 78 -> 54 us, 0.95 of the copy peak).
+// Bound: launch and L2 latency on small grids, HBM on large ones (FP32 20 B, FP64 40 B per cell).
+//
+// This kernel, the source, the increments' preparation and the particle pass are launched with
+// programmatic dependence but do not let the kernel after them start early (no pdl_next): a chain
+// in which every kernel does lets the waiting blocks of many substeps pile up on the SMs. PM steps,
+// us, normal launches / programmatic / programmatic and early starts: FP32 48^3 38.3 / 38.1 / 45.5,
+// 96^3 71.4 / 68.6 / 68.2, 160^3 227 / 216 / 218, 256^3 905 / 872 / 876; FP64 33^3 38.5 / 37.0 / 40.
+constexpr int kGradThreads = 128;
+template <typename R, int V, int ZC>
+__global__ void __launch_bounds__(kGradThreads) gradient_vec_kernel(int nx, R coef, const R* phi,
+                                                                    V4<R>* acc4) {
+    using C = Cells<R, V>;
+    constexpr int U = V * static_cast<int>(sizeof(V4<R>)) / 16;  // 16-byte units of a thread's cells
+    constexpr int cellU = static_cast<int>(sizeof(V4<R>)) / 16;
+    __shared__ float4 stage[kGradThreads / 32][32 * U];
+    const int W = nx / V, plane = nx * nx, units = W * nx;
     const int tid = threadIdx.x, lane = tid & 31;
-    const int g = blockIdx.x * BS + tid;
-    const bool valid = g < plane4;
-    const int y = g / W, q = g - (g / W) * W;
+    const int g = blockIdx.x * kGradThreads + tid;  // unit within a plane
+    const bool valid = g < units;
+    const int y = valid ? g / W : 0, q = valid ? g - y * W : 0;
+    const int at = y * nx + q * V;
     // (a neighbour across the row's end is not used: the faces are one-sided)
-    const bool lload = lane == 0 && q > 0, rload = lane == 31 && q < W - 1;
-    const float4* phi4 = reinterpret_cast<const float4*>(phi);
+    const bool lload = valid && lane == 0 && q > 0, rload = valid && lane == 31 && q < W - 1;
+    const int aym = y > 0 ? at - nx : at, ayp = y < nx - 1 ? at + nx : at;
     const int z0 = blockIdx.y * ZC;
-    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 pv[ZC + 2];  // phi at z0 - 1 ... z0 + ZC (clamped to the box; faces are one-sided)
+    float4* const st = stage[tid >> 5];
+    // the warp's cells of a plane: from cell first on, count 16-byte units
+    const int first = (g - lane) * V, count = min(32, units - (g - lane)) * U;
+    pdl_wait();
+    C pv[ZC + 2];  // phi at z0 - 1 ... z0 + ZC (clamped to the box; faces are one-sided)
 #pragma unroll
-    for (int k = 0; k < ZC + 2; ++k) {
-        const int z = min(max(z0 - 1 + k, 0), nx - 1);
-        pv[k] = valid ? __ldg(phi4 + g + z * plane4) : zero4;
-    }
-    const int gym = y > 0 ? g - W : g;
-    const int gyp = y < nx - 1 ? g + W : g;
-    const int x = 4 * q;
+    for (int k = 0; k < ZC + 2; ++k)
+        pv[k] = load_cells<R, V>(phi + (at + min(max(z0 - 1 + k, 0), nx - 1) * plane));
+    struct Plane {
+        C ym, yp;
+        R l, r;
+    };
+    auto fetch = [&](int z) -> Plane {
+        Plane p{};
+        if (valid && z < nx) {
+            const int zb = z * plane;
+            if (lload) p.l = load_cells<R, 1>(phi + (at - 1 + zb)).v[0];
+            if (rload) p.r = load_cells<R, 1>(phi + (at + V + zb)).v[0];
+            p.ym = load_cells<R, V>(phi + (aym + zb));
+            p.yp = load_cells<R, V>(phi + (ayp + zb));
+        }
+        return p;
+    };
+    // central inside, one-sided at the first and the last node
+    auto diff = [&](int i, R m, R c, R p) {
+        return i == 0 ? p - c : i == nx - 1 ? c - m : R(0.5) * (p - m);
+    };
+    Plane next = fetch(z0);
 #pragma unroll
     for (int k = 0; k < ZC; ++k) {
         const int z = z0 + k;
-        const float4 c = pv[k + 1];
-        float lft = __shfl_up_sync(0xffffffffu, c.w, 1);
-        float rgt = __shfl_down_sync(0xffffffffu, c.x, 1);
-        if (!valid) continue;
-        const int rowbase = z * nx * nx + y * nx;
-        if (lload) lft = __ldg(phi + rowbase + x - 1);
-        if (rload) rgt = __ldg(phi + rowbase + x + 4);
-        // x: central inside, one-sided at x = 0 and x = nx - 1
-        const float d0 = x == 0 ? c.y - c.x : 0.5f * (c.y - lft);
-        const float d1 = 0.5f * (c.z - c.x);
-        const float d2 = 0.5f * (c.w - c.y);
-        const float d3 = x + 4 == nx ? c.w - c.z : 0.5f * (rgt - c.z);
-        // y
-        float4 ey;
-        if (y == 0) {
-            const float4 yp = __ldg(phi4 + gyp + z * plane4);
-            ey = make_float4(yp.x - c.x, yp.y - c.y, yp.z - c.z, yp.w - c.w);
-        } else if (y == nx - 1) {
-            const float4 ym = __ldg(phi4 + gym + z * plane4);
-            ey = make_float4(c.x - ym.x, c.y - ym.y, c.z - ym.z, c.w - ym.w);
-        } else {
-            const float4 yp = __ldg(phi4 + gyp + z * plane4);
-            const float4 ym = __ldg(phi4 + gym + z * plane4);
-            ey = make_float4(0.5f * (yp.x - ym.x), 0.5f * (yp.y - ym.y), 0.5f * (yp.z - ym.z),
-                             0.5f * (yp.w - ym.w));
+        if (z >= nx) break;
+        const Plane p = next;
+        if (k + 1 < ZC) next = fetch(z + 1);
+        const C c = pv[k + 1];
+        R lft = __shfl_up_sync(0xffffffffu, c.v[V - 1], 1);
+        R rgt = __shfl_down_sync(0xffffffffu, c.v[0], 1);
+        if (lload) lft = p.l;
+        if (rload) rgt = p.r;
+        __syncwarp();  // (the plane before has been read from the stage)
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            const R l = i == 0 ? lft : c.v[i > 0 ? i - 1 : 0];
+            const R r = i == V - 1 ? rgt : c.v[i < V - 1 ? i + 1 : 0];
+            const V4<R> o = v4<R>(diff(q * V + i, l, c.v[i], r) * coef,
+                                  diff(y, p.ym.v[i], c.v[i], p.yp.v[i]) * coef,
+                                  diff(z, pv[k].v[i], c.v[i], pv[k + 2].v[i]) * coef, c.v[i]);
+            const float4* const o4 = reinterpret_cast<const float4*>(&o);
+#pragma unroll
+            for (int j = 0; j < cellU; ++j) {
+                const int slot = lane * U + i * cellU + j;
+                st[slot ^ ((slot >> 3) & 7)] = o4[j];  // (no bank conflicts on either side)
+            }
         }
-        // z
-        const float4 zm = pv[k], zp = pv[k + 2];
-        float4 ez;
-        if (z == 0) ez = make_float4(zp.x - c.x, zp.y - c.y, zp.z - c.z, zp.w - c.w);
-        else if (z == nx - 1) ez = make_float4(c.x - zm.x, c.y - zm.y, c.z - zm.z, c.w - zm.w);
-        else
-            ez = make_float4(0.5f * (zp.x - zm.x), 0.5f * (zp.y - zm.y), 0.5f * (zp.z - zm.z),
-                             0.5f * (zp.w - zm.w));
-        float4* o = acc4 + (static_cast<size_t>(z) * nx + y) * nx + x;
-        o[0] = make_float4(d0 * coef, ey.x * coef, ez.x * coef, c.x);
-        o[1] = make_float4(d1 * coef, ey.y * coef, ez.y * coef, c.y);
-        o[2] = make_float4(d2 * coef, ey.z * coef, ez.z * coef, c.z);
-        o[3] = make_float4(d3 * coef, ey.w * coef, ez.w * coef, c.w);
+        __syncwarp();
+        float4* const to =
+            reinterpret_cast<float4*>(acc4 + (static_cast<size_t>(z) * plane + first));
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const int slot = j * 32 + lane;
+            if (slot < count) to[slot] = st[slot ^ ((slot >> 3) & 7)];
+        }
     }
 }
 
@@ -899,6 +901,7 @@ __global__ void __launch_bounds__(kPmThreads, 6) pm_particle_kernel(PmParticleAr
     V4<R>* accp = static_cast<V4<R>*>(a.acc);
     V4<R>* u = static_cast<V4<R>*>(a.u);
     const R dt = static_cast<R>(a.dt);
+    pdl_wait();
     double x = 0, y = 0, z = 0, m = 0;
     if (active) load_pos<R>(a.posm, MIXED ? lo : nullptr, i, x, y, z, m);
 
@@ -1003,25 +1006,23 @@ __global__ void __launch_bounds__(kPmThreads, 6) pm_particle_kernel(PmParticleAr
 
 template <typename R, bool MIXED>
 void dispatch_pm(const PmParticleArgs& a, int mode, double scale, cudaStream_t s) {
-    const int b = div_up(a.n, 256);
+    auto go = [&](auto* kernel) { launch_pdl(kernel, div_up(a.n, 256), 256, 0, s, a, scale); };
     switch (mode) {
         case PM_INTERP_CORRECT | PM_WRITE_SYNC:
-            pm_particle_kernel<R, MIXED, PM_INTERP_CORRECT | PM_WRITE_SYNC><<<b, 256, 0, s>>>(a, scale);
+            go(pm_particle_kernel<R, MIXED, PM_INTERP_CORRECT | PM_WRITE_SYNC>);
             break;
         case PM_PREDICT_DEPOSIT:
-            pm_particle_kernel<R, MIXED, PM_PREDICT_DEPOSIT><<<b, 256, 0, s>>>(a, scale);
+            go(pm_particle_kernel<R, MIXED, PM_PREDICT_DEPOSIT>);
             break;
         case PM_INTERP_CORRECT | PM_PREDICT_DEPOSIT:
-            pm_particle_kernel<R, MIXED, PM_INTERP_CORRECT | PM_PREDICT_DEPOSIT><<<b, 256, 0, s>>>(a, scale);
+            go(pm_particle_kernel<R, MIXED, PM_INTERP_CORRECT | PM_PREDICT_DEPOSIT>);
             break;
         case PM_INTERP_CORRECT | PM_PREDICT_DEPOSIT | PM_WRITE_SYNC:
-            pm_particle_kernel<R, MIXED, PM_INTERP_CORRECT | PM_PREDICT_DEPOSIT | PM_WRITE_SYNC>
-                <<<b, 256, 0, s>>>(a, scale);
+            go(pm_particle_kernel<R, MIXED, PM_INTERP_CORRECT | PM_PREDICT_DEPOSIT | PM_WRITE_SYNC>);
             break;
         case PM_INTERP_CORRECT | PM_PREDICT_DEPOSIT | PM_WRITE_SYNC | PM_SUMS:
-            pm_particle_kernel<R, MIXED,
-                               PM_INTERP_CORRECT | PM_PREDICT_DEPOSIT | PM_WRITE_SYNC | PM_SUMS>
-                <<<b, 256, 0, s>>>(a, scale);
+            go(pm_particle_kernel<R, MIXED,
+                                  PM_INTERP_CORRECT | PM_PREDICT_DEPOSIT | PM_WRITE_SYNC | PM_SUMS>);
             break;
         default:
             throw Error(RRG_ERR_INVALID, "pm particle pass: unsupported mode");
@@ -1046,20 +1047,17 @@ void launch_cic_deposit(int prec, int64_t n, const void* posm, const void* poslo
 }
 
 void launch_wave_source(int prec, int nx, const unsigned long long* mgrid, int shift_s,
-                        double dx, double rho_mean, double scale, void* src, bool zero_grid,
-                        cudaStream_t s) {
+                        double dx, double rho_mean, double scale, void* src,
+                        unsigned long long* zero_grid, cudaStream_t s) {
     const int64_t nc = static_cast<int64_t>(nx) * nx * nx;
     const double inv_scale = ldexp(1.0, -shift_s);
-    auto* mg = const_cast<unsigned long long*>(mgrid);
     const double dx3 = dx * dx * dx;
     if (prec == RRG_PREC_FP64)
-        wave_source_kernel<double><<<div_up(nc, 256), 256, 0, s>>>(
-            nc, mg, inv_scale, dx3, 1.0 / dx3, rho_mean, scale, static_cast<double*>(src),
-            zero_grid);
+        launch_pdl(wave_source_kernel<double>, div_up(nc, 256), 256, 0, s, nc, mgrid, inv_scale,
+                   dx3, 1.0 / dx3, rho_mean, scale, static_cast<double*>(src), zero_grid);
     else
-        wave_source_kernel<float><<<div_up(nc, 256), 256, 0, s>>>(
-            nc, mg, inv_scale, dx3, 1.0 / dx3, rho_mean, scale, static_cast<float*>(src),
-            zero_grid);
+        launch_pdl(wave_source_kernel<float>, div_up(nc, 256), 256, 0, s, nc, mgrid, inv_scale,
+                   dx3, 1.0 / dx3, rho_mean, scale, static_cast<float*>(src), zero_grid);
     RRG_LAUNCHED();
 }
 
@@ -1070,10 +1068,9 @@ void launch_wave_inc_prep(int nx, bool first, const unsigned long long* mg,
     const int V = nx % 4 == 0 ? 4 : nx % 2 == 0 ? 2 : 1;
     const int64_t units = static_cast<int64_t>(nx / V) * nx * nx;
     auto go = [&](auto* kernel) {
-        kernel<<<div_up(units, 256), 256, 0, s>>>(
-            nx, mg, mg_zero, ldexp(1.0, -shift_s), 1.0 / (dx * dx * dx), rho_sub, phi0, phi_prev,
-            w.K_F, w.K_MAIN, w.K_ACTUAL + w.K_OLD - 1.0, static_cast<float>(w.K_OLD), g, d, d_old,
-            src);
+        launch_pdl(kernel, div_up(units, 256), 256, 0, s, nx, mg, mg_zero, ldexp(1.0, -shift_s),
+                   1.0 / (dx * dx * dx), rho_sub, phi0, phi_prev, w.K_F, w.K_MAIN,
+                   w.K_ACTUAL + w.K_OLD - 1.0, static_cast<float>(w.K_OLD), g, d, d_old, src);
         RRG_LAUNCHED();
     };
     if (first) {
@@ -1262,27 +1259,31 @@ void launch_wave_step(int prec, int nx, const void* phi, void* phi_old_inout, co
     RRG_LAUNCHED();
 }
 
+namespace {
+
+template <typename R, int V>
+void launch_gradient_vec(int nx, double coef, const void* phi, void* acc4, cudaStream_t s) {
+    constexpr int ZC = 2;
+    const dim3 grid(div_up(static_cast<int64_t>(nx / V) * nx, kGradThreads), div_up(nx, ZC));
+    launch_pdl(gradient_vec_kernel<R, V, ZC>, grid, kGradThreads, 0, s, nx, static_cast<R>(coef),
+               static_cast<const R*>(phi), static_cast<V4<R>*>(acc4));
+    RRG_LAUNCHED();
+}
+
+}  // namespace
+
 void launch_gradient(int prec, int nx, double dx, const void* phi, void* acc4, cudaStream_t s) {
     const double coef = -1.0 / dx;
-    const int W4 = nx / 4;
-    if (prec != RRG_PREC_FP64 && nx >= 8 && nx % 4 == 0) {
-        dim3 g4(div_up(static_cast<int64_t>(W4) * nx, 128), nx / 4);
-        gradient_x4_kernel<4, 128><<<g4, 128, 0, s>>>(nx, static_cast<float>(coef),
-                                                      static_cast<const float*>(phi),
-                                                      static_cast<float4*>(acc4));
-        RRG_LAUNCHED();
-        return;
+    const bool f64 = prec == RRG_PREC_FP64;
+    const int V = cells_per_thread(nx, f64);
+    if (f64) {
+        if (V == 2) launch_gradient_vec<double, 2>(nx, coef, phi, acc4, s);
+        else launch_gradient_vec<double, 1>(nx, coef, phi, acc4, s);
+    } else {
+        if (V == 4) launch_gradient_vec<float, 4>(nx, coef, phi, acc4, s);
+        else if (V == 2) launch_gradient_vec<float, 2>(nx, coef, phi, acc4, s);
+        else launch_gradient_vec<float, 1>(nx, coef, phi, acc4, s);
     }
-    dim3 grid(div_up(nx, kTX), div_up(nx, kTY), nx);
-    dim3 block(kTX, kTY);
-    if (prec == RRG_PREC_FP64)
-        gradient_kernel<double><<<grid, block, 0, s>>>(nx, coef, static_cast<const double*>(phi),
-                                                       static_cast<V4<double>*>(acc4));
-    else
-        gradient_kernel<float><<<grid, block, 0, s>>>(nx, static_cast<float>(coef),
-                                                      static_cast<const float*>(phi),
-                                                      static_cast<V4<float>*>(acc4));
-    RRG_LAUNCHED();
 }
 
 void launch_interp(int prec, int64_t n, const void* posm, const void* poslo, const GridDev& g,

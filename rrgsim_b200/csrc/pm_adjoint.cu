@@ -326,8 +326,9 @@ void pm_step(rrg_pm_adjoint* P, cudaStream_t s) {
     a.mgrid = static_cast<unsigned long long*>(P->mg.p);
     a.dt = P->dt;
     launch_pm_particles(a, PM_PREDICT_DEPOSIT, s);
-    launch_wave_source(P->prec, P->grid.nx, static_cast<unsigned long long*>(P->mg.p), P->shift_s,
-                       P->grid.dx, P->rho_mean, 1.0, P->src.p, true, s);
+    auto* mg = static_cast<unsigned long long*>(P->mg.p);
+    launch_wave_source(P->prec, P->grid.nx, mg, P->shift_s, P->grid.dx, P->rho_mean, 1.0, P->src.p,
+                       mg, s);
     for (int k = 0; k < P->substeps; ++k) {
         // phi[1] current, phi[0] previous: the new level overwrites phi[0], then roles swap
         launch_wave_step(P->prec, P->grid.nx, P->phi[1].p, P->phi[0].p, P->src.p, P->wc, nullptr, s);

@@ -68,7 +68,7 @@
 // first. Every wait is bounded; one that runs out sets the error word and the block leaves (the
 // step's results are then invalid), and later launches return at once until the host, which
 // turns the word into an error, clears the sync memory. The arithmetic is that of
-// wave_source_kernel<float>, wave_periodic_vec_kernel and gradient_x4_kernel, expression for
+// wave_source_kernel<float>, wave_periodic_vec_kernel and gradient_vec_kernel, expression for
 // expression, so the results are the same bits.
 #include <algorithm>
 #include <cstdlib>
@@ -868,7 +868,7 @@ __global__ void __launch_bounds__(tb::T, 1) wave_solve_tb_kernel(const SolveArgs
         }
     }
 
-    // ---- gradient of the final level (gradient_x4_kernel's expressions) -------------------
+    // ---- gradient of the final level (gradient_vec_kernel's expressions) -------------------
     if (a.acc4 != nullptr) {
         const int x = 4 * q, y = y0 + r;
 #pragma unroll
