@@ -187,8 +187,10 @@ __global__ void __launch_bounds__(kBS, 2) vjp_f32x2_kernel(const VjpParams<float
         }
         float2 tAx = z2, tAy = z2, tAz = z2, tBx = z2, tBy = z2, tBz = z2, tM = z2;
         float2 tFx = z2, tFy = z2, tFz = z2;
+        // (a chunk may be shorter than a tile; what is staged past its end adds nothing)
+        const int cnt = static_cast<int>(min(static_cast<int64_t>(kBS), (je - j0 + 3) & ~int64_t(3)));
 #pragma unroll 4
-        for (int q = 0; q < kBS; ++q) {
+        for (int q = 0; q < cnt; ++q) {
             const float4 xy = s_xy[q], zm = s_zm[q], lxy = s_lxy[q], lzh = s_lzh[q];
             const float2 px = make_float2(xy.x, xy.y), py = make_float2(xy.z, xy.w);
             const float2 pz = make_float2(zm.x, zm.y);
@@ -544,8 +546,9 @@ struct VjpSymParams {
     R uniform_h;
     int64_t n;
     int tiles;
+    int parts;     // of a tile pair: 256 / parts j each, 1 to 8
     const V4<R>* lam;
-    V4<R>* slots;  // [tiles][tiles][256]
+    V4<R>* slots;  // [tiles][tiles][parts][256]
 };
 
 
@@ -558,7 +561,9 @@ __global__ void __launch_bounds__(kBS) vjp_sym_kernel(const VjpSymParams<R> p) {
     const int tid = threadIdx.x, lane = tid & 31;
     // upper-triangular (with diagonal) row-major tile-pair index -> (a, b)
     const int T = p.tiles;
-    const int64_t t = blockIdx.x;
+    const int64_t t = blockIdx.x / p.parts;
+    const int part = static_cast<int>(blockIdx.x) - static_cast<int>(t) * p.parts;
+    const int len = kBS / p.parts, q0 = part * len;  // this block's j in the tile
     auto S = [T](int64_t a) { return a * T - a * (a - 1) / 2; };
     const double B2 = 2.0 * T + 1.0;
     int64_t a = static_cast<int64_t>(floor((B2 - sqrt(B2 * B2 - 8.0 * static_cast<double>(t))) * 0.5));
@@ -616,7 +621,7 @@ __global__ void __launch_bounds__(kBS) vjp_sym_kernel(const VjpSymParams<R> p) {
     };
     if (!sym) {
 #pragma unroll 2
-        for (int q = 0; q < kBS; ++q) {
+        for (int q = q0; q < q0 + len; ++q) {
             R jx, jy, jz, jm;
             pair(q, jx, jy, jz, jm);
         }
@@ -625,7 +630,7 @@ __global__ void __launch_bounds__(kBS) vjp_sym_kernel(const VjpSymParams<R> p) {
         // j = 32 c + (l + t) mod 32 and adds to the sums that lane l + 1 held for it, so after
         // 32 steps lane l holds its warp's sums for j = 32 c + l (one shuffle per sum and step,
         // and one shared add per chunk, instead of a warp reduction per j)
-        for (int c = 0; c < kBS / 32; ++c) {
+        for (int c = q0 / 32; c < (q0 + len) / 32; ++c) {
             R ax = 0, ay = 0, az = 0, am = 0;
 #pragma unroll 4
             for (int t = 0; t < 32; ++t) {
@@ -643,51 +648,80 @@ __global__ void __launch_bounds__(kBS) vjp_sym_kernel(const VjpSymParams<R> p) {
             atomicAdd(&s_acc[c * 32 + lane][3], am);
         }
     }
-    p.slots[(a * T + b) * kBS + tid] = v4<R>(gx, gy, gz, gm);
+    p.slots[((a * T + b) * p.parts + part) * kBS + tid] = v4<R>(gx, gy, gz, gm);
     if (sym) {
         __syncthreads();
-        p.slots[(b * T + a) * kBS + tid] =
-            v4<R>(s_acc[tid][0], s_acc[tid][1], s_acc[tid][2], s_acc[tid][3]);
+        if (tid >= q0 && tid < q0 + len)  // (every j of the tile is in one part)
+            p.slots[(b * T + a) * p.parts * kBS + tid] =
+                v4<R>(s_acc[tid][0], s_acc[tid][1], s_acc[tid][2], s_acc[tid][3]);
     }
 }
 
+// A block of (32, 8) threads takes 32 particles of one tile, warp w every eighth of their sums;
+// warp 0 adds the eight in order.
+constexpr int kFinWarps = 8;
 template <typename R>
-__global__ void vjp_sym_finish(int64_t n, int T, const V4<R>* __restrict__ slots,
-                               V4<R>* __restrict__ out, int accumulate, const AdjUpd<R> upd) {
-    const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= n) return;
+__global__ void __launch_bounds__(32 * kFinWarps)
+vjp_sym_finish(int64_t n, int T, int parts, const V4<R>* __restrict__ slots, V4<R>* __restrict__ out,
+               int accumulate, const AdjUpd<R> upd) {
+    __shared__ double sh[kFinWarps][4][32];
+    const int lane = threadIdx.x, w = threadIdx.y;
+    const int64_t k = static_cast<int64_t>(blockIdx.x) * 32 + lane;
     const int64_t a = k / kBS, l = k % kBS;
-    double sx = 0, sy = 0, sz = 0, sm = 0;
-    for (int b = 0; b < T; ++b) {
-        const V4<R> v = slots[(a * T + b) * kBS + l];
-        sx += v.x;
-        sy += v.y;
-        sz += v.z;
-        sm += v.w;
+    double v[4] = {};
+    if (k < n) {
+        // the tiles before (one sum each, in their first part), then the parts of the others
+        const V4<R>* const from = slots + a * T * parts * kBS + l;
+        const int count = static_cast<int>(a + (T - a) * parts);
+#pragma unroll 4
+        for (int i = w; i < count; i += kFinWarps) {
+            const V4<R> q = from[(i < a ? i * parts : a * parts + (i - a)) * kBS];
+            v[0] += q.x;
+            v[1] += q.y;
+            v[2] += q.z;
+            v[3] += q.w;
+        }
     }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) sh[w][c][lane] = v[c];
+    __syncthreads();
+    if (w != 0 || k >= n) return;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        for (int i = 1; i < kFinWarps; ++i) v[c] += sh[i][c][lane];
     if (accumulate) {
         const V4<R> o = out[k];
-        sx += o.x;
-        sy += o.y;
-        sz += o.z;
-        sm += o.w;
+        v[0] += o.x;
+        v[1] += o.y;
+        v[2] += o.z;
+        v[3] += o.w;
     }
-    const V4<R> r = v4<R>(static_cast<R>(sx), static_cast<R>(sy), static_cast<R>(sz),
-                          static_cast<R>(sm));
+    const V4<R> r = v4<R>(static_cast<R>(v[0]), static_cast<R>(v[1]), static_cast<R>(v[2]),
+                          static_cast<R>(v[3]));
     out[k] = r;
     if (upd.V) adjoint_update_at(k, r.x, r.y, r.z, upd);
 }
 
+// Parts of a tile pair: 1, 2, 4 or 8, the most that keep the blocks within four per SM. Whole pairs
+// leave SMs idle below ~8,000 particles (N = 2,000: 36 blocks). Product and finish, us, whole pairs ->
+// parts: N = 1,000 56.6 -> 12.1, 2,000 57.3 -> 18.5, 5,000 100 -> 76.6, 8,000 (whole) 195 -> 191.
+int vjp_sym_parts(int64_t n, int sms) {
+    const int64_t T = (n + kBS - 1) / kBS, blocks = T * (T + 1) / 2;
+    int parts = 1;
+    while (parts < 8 && 2 * parts * blocks <= 4 * static_cast<int64_t>(sms)) parts *= 2;
+    return parts;
+}
+
 template <typename R>
-size_t vjp_sym_slot_bytes(int64_t n) {
+size_t vjp_sym_slot_bytes(int64_t n, int sms) {
     const int64_t T = (n + kBS - 1) / kBS;
-    return sizeof(V4<R>) * static_cast<size_t>(T * T * kBS);
+    return sizeof(V4<R>) * static_cast<size_t>(T * T * vjp_sym_parts(n, sms) * kBS);
 }
 
 template <typename R>
 void vjp_sym_launch(const void* posm, const void* hsoft, double uniform_h, int64_t n,
                     const void* lam, void* out, bool accumulate, void* slots,
-                    cudaStream_t stream, const AdjUpd<R>& upd = AdjUpd<R>()) {
+                    int sms, cudaStream_t stream, const AdjUpd<R>& upd = AdjUpd<R>()) {
     const int T = static_cast<int>((n + kBS - 1) / kBS);
     VjpSymParams<R> p;
     p.posm = static_cast<const V4<R>*>(posm);
@@ -695,45 +729,90 @@ void vjp_sym_launch(const void* posm, const void* hsoft, double uniform_h, int64
     p.uniform_h = static_cast<R>(uniform_h);
     p.n = n;
     p.tiles = T;
+    p.parts = vjp_sym_parts(n, sms);
     p.lam = static_cast<const V4<R>*>(lam);
     p.slots = static_cast<V4<R>*>(slots);
-    const unsigned blocks = static_cast<unsigned>(static_cast<int64_t>(T) * (T + 1) / 2);
+    const unsigned blocks = static_cast<unsigned>(static_cast<int64_t>(T) * (T + 1) / 2 * p.parts);
     if (hsoft) vjp_sym_kernel<R, false><<<blocks, kBS, 0, stream>>>(p);
     else vjp_sym_kernel<R, true><<<blocks, kBS, 0, stream>>>(p);
     RRG_LAUNCHED();
-    vjp_sym_finish<R><<<div_up(n, 256), 256, 0, stream>>>(n, T, p.slots, static_cast<V4<R>*>(out),
-                                                          accumulate ? 1 : 0, upd);
+    vjp_sym_finish<R><<<div_up(n, 32), dim3(32, kFinWarps), 0, stream>>>(
+        n, T, p.parts, p.slots, static_cast<V4<R>*>(out), accumulate ? 1 : 0, upd);
     RRG_LAUNCHED();
 }
 
-template <typename R>
-__global__ void vjp_finish(const VjpParams<R> p, int splits, const AdjUpd<R> upd) {
-    const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= p.n) return;
-    double sx = 0, sy = 0, sz = 0, sm = 0;
-    for (int s = 0; s < splits; ++s) {
-        const V4<R> v = p.part[static_cast<int64_t>(s) * p.n + k];
-        sx += v.x;
-        sy += v.y;
-        sz += v.z;
-        sm += v.w;
+// Sums of a particle's split partials in FP64 and a fixed order: a block of (32, 8) threads takes
+// 32 particles, warp w the splits w, w + 8, ..., and warp 0 adds the eight sums in order. f: the
+// force partials', with FORCE. True for the threads (of warp 0) that hold a particle's sums.
+template <bool FORCE>
+__device__ __forceinline__ bool vjp_part_sum(const VjpParams<float>& p, int splits, int64_t k,
+                                             double s[4], double f[3]) {
+    constexpr int NV = FORCE ? 7 : 4;
+    __shared__ double sh[kFinWarps][NV][32];
+    const int lane = threadIdx.x, w = threadIdx.y;
+    double v[NV] = {};
+    if (k < p.n) {
+#pragma unroll 4
+        for (int i = w; i < splits; i += kFinWarps) {
+            const int64_t o = static_cast<int64_t>(i) * p.n + k;
+            const V4<float> q = p.part[o];
+            v[0] += q.x;
+            v[1] += q.y;
+            v[2] += q.z;
+            v[3] += q.w;
+            if constexpr (FORCE) {
+                const V4<float> a = p.part_a[o];
+                v[4] += a.x;
+                v[5] += a.y;
+                v[6] += a.z;
+            }
+        }
     }
+#pragma unroll
+    for (int c = 0; c < NV; ++c) sh[w][c][lane] = v[c];
+    __syncthreads();
+    if (w != 0 || k >= p.n) return false;
+#pragma unroll
+    for (int c = 0; c < NV; ++c)
+        for (int i = 1; i < kFinWarps; ++i) v[c] += sh[i][c][lane];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) s[c] = v[c];
+    if constexpr (FORCE) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f[c] = v[4 + c];
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(32 * kFinWarps) vjp_finish(const VjpParams<float> p, int splits,
+                                                             const AdjUpd<float> upd) {
+    const int64_t k = static_cast<int64_t>(blockIdx.x) * 32 + threadIdx.x;
+    double s[4];
+    if (!vjp_part_sum<false>(p, splits, k, s, nullptr)) return;
     if (p.accumulate) {
-        const V4<R> o = p.out[k];
-        sx += o.x;
-        sy += o.y;
-        sz += o.z;
-        sm += o.w;
+        const V4<float> o = p.out[k];
+        s[0] += o.x;
+        s[1] += o.y;
+        s[2] += o.z;
+        s[3] += o.w;
     }
-    const V4<R> r = v4<R>(static_cast<R>(sx), static_cast<R>(sy), static_cast<R>(sz),
-                          static_cast<R>(sm));
+    const V4<float> r = v4<float>(static_cast<float>(s[0]), static_cast<float>(s[1]),
+                                  static_cast<float>(s[2]), static_cast<float>(s[3]));
     p.out[k] = r;
     if (upd.V) adjoint_update_at(k, r.x, r.y, r.z, upd);
 }
 
-// j-split count of the paired FP32 VJP: the smallest whose block count fills whole waves of
-// resident blocks to within 2% of the best achievable (the rule of the forward kernels).
-int vjp_f32x2_splits(int64_t n, int sms) {
+// j-chunks of the ordered FP32 VJP. Where 256-particle chunks fill less than one wave of resident
+// blocks (up to ~6,000 particles): the shortest multiple of 32 that stays within a wave. Beyond:
+// whole tiles, the fewest chunks whose blocks fill whole waves to within 2% of the best achievable
+// (the rule of the forward kernels). Product with force and its finish, us, whole tiles and one thread
+// per particle in the finish -> here: N = 600 62.4 -> 7.8, 1,000 43.4 -> 8.1, 2,000 44.3 -> 12.0,
+// 3,000 27.6 -> 16.5, 4,000 29.2 -> 25.6, 6,000 51.9 -> 44.8.
+struct VjpChunks {
+    int64_t chunk;
+    int splits;
+};
+VjpChunks vjp_f32x2_chunks(int64_t n, int sms) {
     static int resident = 0;
     if (!resident) {
         int nb = 0;
@@ -749,6 +828,9 @@ int vjp_f32x2_splits(int64_t n, int sms) {
     const int64_t kblocks = (n + 2 * kBS - 1) / (2 * kBS);
     const int64_t tiles = (n + kBS - 1) / kBS;
     const int64_t slots = static_cast<int64_t>(sms) * resident;
+    for (int64_t c = 32; c <= kBS; c += 32)
+        if (kblocks * ((n + c - 1) / c) <= slots)
+            return {c, static_cast<int>((n + c - 1) / c)};
     double best = 0, eff[65] = {};
     const int64_t top = std::min<int64_t>(tiles, 64);
     for (int64_t sp = 1; sp <= top; ++sp) {
@@ -757,9 +839,10 @@ int vjp_f32x2_splits(int64_t n, int sms) {
         eff[sp] = static_cast<double>(total) / static_cast<double>(waves * slots);
         best = std::max(best, eff[sp]);
     }
-    for (int64_t sp = 1; sp <= top; ++sp)
-        if (eff[sp] >= best - 0.02) return static_cast<int>(sp);
-    return 1;
+    int64_t sp = 1;
+    while (eff[sp] < best - 0.02) ++sp;
+    const int64_t per = (tiles + sp - 1) / sp;
+    return {per * kBS, static_cast<int>((tiles + per - 1) / per)};
 }
 
 size_t vjp_f32x2_part_bytes(int64_t n, int splits) {
@@ -773,17 +856,15 @@ void adjoint_update_launch(int64_t n, const void* X, const AdjUpd<float>& upd, c
 // mgrad = false: no mass gradient (the w slot gets 0, or keeps its value when accumulating).
 void vjp_f32x2_launch(const void* posm, const void* hsoft, double uniform_h, double uniform_m,
                       int64_t n, const void* lam, void* out, bool accumulate, void* part,
-                      int splits, cudaStream_t stream,
+                      const VjpChunks& chunks, cudaStream_t stream,
                       const AdjUpd<float>& upd = AdjUpd<float>(), bool mgrad = true) {
-    const int64_t tiles = (n + kBS - 1) / kBS;
-    const int64_t tiles_per = (tiles + splits - 1) / splits;
-    const int real = static_cast<int>((tiles + tiles_per - 1) / tiles_per);
+    const int real = chunks.splits;
     VjpParams<float> p;
     p.posm = static_cast<const V4<float>*>(posm);
     p.hsoft = static_cast<const float*>(hsoft);
     p.uniform_h = static_cast<float>(uniform_h);
     p.n = n;
-    p.jchunk = tiles_per * kBS;
+    p.jchunk = chunks.chunk;
     p.lam = static_cast<const V4<float>*>(lam);
     p.out = static_cast<V4<float>*>(out);
     p.part = static_cast<V4<float>*>(part);
@@ -811,7 +892,7 @@ void vjp_f32x2_launch(const void* posm, const void* hsoft, double uniform_h, dou
 #undef RRG_VJP2
     RRG_LAUNCHED();
     if (real > 1) {
-        vjp_finish<float><<<div_up(n, 256), 256, 0, stream>>>(p, real, upd);
+        vjp_finish<<<div_up(n, 32), dim3(32, kFinWarps), 0, stream>>>(p, real, upd);
         RRG_LAUNCHED();
     } else if (upd.V) {
         adjoint_update_launch(n, out, upd, stream);
@@ -862,28 +943,18 @@ __global__ void reverse_init_kernel(int64_t n, const V4<float>* __restrict__ x,
 
 // Finish of a FORCE pass at x_m: X += sum of the VJP partials (fixed order, FP64), a(x_m) from
 // the force partials, w -= dt a, x_{m-1} = x_m - dt w, then the adjoint update of step m - 1.
-__global__ void vjp_reverse_finish(const VjpParams<float> p, int splits, const AdjUpd<float> upd,
-                                   const RevStep r) {
-    const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= p.n) return;
-    double sx = 0, sy = 0, sz = 0, sm = 0, ax = 0, ay = 0, az = 0;
-    for (int s = 0; s < splits; ++s) {
-        const int64_t o = static_cast<int64_t>(s) * p.n + k;
-        const V4<float> v = p.part[o];
-        sx += v.x;
-        sy += v.y;
-        sz += v.z;
-        sm += v.w;
-        const V4<float> a = p.part_a[o];
-        ax += a.x;
-        ay += a.y;
-        az += a.z;
-    }
+__global__ void __launch_bounds__(32 * kFinWarps) vjp_reverse_finish(const VjpParams<float> p,
+                                                                     int splits,
+                                                                     const AdjUpd<float> upd,
+                                                                     const RevStep r) {
+    const int64_t k = static_cast<int64_t>(blockIdx.x) * 32 + threadIdx.x;
+    double s[4], f[3];
+    if (!vjp_part_sum<true>(p, splits, k, s, f)) return;
     const V4<float> o = p.out[k];
-    const V4<float> X = v4<float>(static_cast<float>(sx + o.x), static_cast<float>(sy + o.y),
-                                  static_cast<float>(sz + o.z), static_cast<float>(sm + o.w));
+    const V4<float> X = v4<float>(static_cast<float>(s[0] + o.x), static_cast<float>(s[1] + o.y),
+                                  static_cast<float>(s[2] + o.z), static_cast<float>(s[3] + o.w));
     p.out[k] = X;
-    reverse_step_at(k, ax, ay, az, r);
+    reverse_step_at(k, f[0], f[1], f[2], r);
     if (upd.V) adjoint_update_at(k, X.x, X.y, X.z, upd);
 }
 
@@ -891,19 +962,17 @@ __global__ void vjp_reverse_finish(const VjpParams<float> p, int splits, const A
 // the reverse update of (w, positions) and the adjoint update upd. part / part_a hold
 // [splits][n] V4 each.
 void vjp_reverse_launch(const void* hsoft, double uniform_h, double uniform_m, int64_t n,
-                        const void* lam, void* out, void* part, void* part_a, int splits,
-                        cudaStream_t stream, const AdjUpd<float>& upd, const RevStep& r,
+                        const void* lam, void* out, void* part, void* part_a,
+                        const VjpChunks& chunks, cudaStream_t stream, const AdjUpd<float>& upd, const RevStep& r,
                         bool mgrad) {
-    const int64_t tiles = (n + kBS - 1) / kBS;
-    const int64_t tiles_per = (tiles + splits - 1) / splits;
-    const int real = static_cast<int>((tiles + tiles_per - 1) / tiles_per);
+    const int real = chunks.splits;
     RRG_REQUIRE(part && part_a, RRG_ERR_STATE, "vjp: missing partials");
     VjpParams<float> p;
     p.posm = r.x;
     p.hsoft = static_cast<const float*>(hsoft);
     p.uniform_h = static_cast<float>(uniform_h);
     p.n = n;
-    p.jchunk = tiles_per * kBS;
+    p.jchunk = chunks.chunk;
     p.lam = static_cast<const V4<float>*>(lam);
     p.out = static_cast<V4<float>*>(out);
     p.part = static_cast<V4<float>*>(part);
@@ -929,7 +998,7 @@ void vjp_reverse_launch(const void* hsoft, double uniform_h, double uniform_m, i
 #undef RRG_VJPF_M
 #undef RRG_VJPF
     RRG_LAUNCHED();
-    vjp_reverse_finish<<<div_up(n, 256), 256, 0, stream>>>(p, real, upd, r);
+    vjp_reverse_finish<<<div_up(n, 32), dim3(32, kFinWarps), 0, stream>>>(p, real, upd, r);
     RRG_LAUNCHED();
 }
 
@@ -1138,12 +1207,12 @@ void launch_direct_vjp_f32(const void* posm, const void* hsoft, float uniform_hs
                            const void* lam, void* out, cudaStream_t stream) {
     int dev = 0;
     RRG_CUDA(cudaGetDevice(&dev));
-    const int splits = vjp_f32x2_splits(n, num_sms(dev));
+    const VjpChunks chunks = vjp_f32x2_chunks(n, num_sms(dev));
     void* part = nullptr;
-    const size_t pb = vjp_f32x2_part_bytes(n, splits);
+    const size_t pb = vjp_f32x2_part_bytes(n, chunks.splits);
     if (pb) RRG_CUDA(cudaMallocAsync(&part, pb, stream));
     try {
-        vjp_f32x2_launch(posm, hsoft, uniform_hsoft, -1.0, n, lam, out, false, part, splits,
+        vjp_f32x2_launch(posm, hsoft, uniform_hsoft, -1.0, n, lam, out, false, part, chunks,
                          stream);
     } catch (...) {
         if (part) cudaFreeAsync(part, stream);
@@ -1180,7 +1249,7 @@ struct rrg_adjoint {
     ABuf mflags;            // uniform-mass check: mismatch flag, mass bits
     int splits = 1;
     bool force_sym = false;  // scratch holds the pair slots of the symmetric direct sum
-    int vjp_splits = 1;
+    VjpChunks vjp_chunks{};
     double uniform_m = -1;  // >= 0 while every particle of the last forward has this mass
     bool mass_grad = true;  // compute dL/dm (the w slot of the position gradient)
     bool forward_done = false;
@@ -1259,14 +1328,14 @@ AdjUpd<R> step_update(rrg_adjoint* A, int m) {
 void vjp(rrg_adjoint* A, const void* x, int m, cudaStream_t s) {
     if (A->prec == RRG_PREC_FP64)
         vjp_sym_launch<double>(x, A->hsoft.p, A->uniform_h, A->n, A->c.p, A->X.p, true,
-                               A->sym_slots.p, s, step_update<double>(A, m));
+                               A->sym_slots.p, A->sms, s, step_update<double>(A, m));
     else if (A->vjp_pairs)
         vjp_pair_launch(x, A->hsoft.p, A->uniform_h, A->uniform_m, A->n, A->c.p, A->X.p, true,
                         A->vjp_part.p, A->sms, s, step_update<float>(A, m), nullptr,
                         A->mass_grad);
     else
         vjp_f32x2_launch(x, A->hsoft.p, A->uniform_h, A->uniform_m, A->n, A->c.p, A->X.p, true,
-                         A->vjp_part.p, A->vjp_splits, s, step_update<float>(A, m),
+                         A->vjp_part.p, A->vjp_chunks, s, step_update<float>(A, m),
                          A->mass_grad);
 }
 
@@ -1320,9 +1389,10 @@ RRG_API rrg_status rrg_dev_direct_vjp(const void* posm, const void* hsoft, doubl
             return RRG_OK;
         }
         void* slots = nullptr;
-        RRG_CUDA(cudaMallocAsync(&slots, vjp_sym_slot_bytes<double>(n), s));
+        const int sms = num_sms(dev);
+        RRG_CUDA(cudaMallocAsync(&slots, vjp_sym_slot_bytes<double>(n, sms), s));
         try {
-            vjp_sym_launch<double>(posm, hsoft, uniform_hsoft, n, lam, out, false, slots, s);
+            vjp_sym_launch<double>(posm, hsoft, uniform_hsoft, n, lam, out, false, slots, sms, s);
         } catch (...) {
             cudaFreeAsync(slots, s);
             throw;
@@ -1376,6 +1446,7 @@ RRG_API rrg_status rrg_adjoint_create(int device, int precision, int64_t n, doub
         for (ABuf* b : {&A->x, &A->x2, &A->v, &A->a, &A->u, &A->X, &A->V, &A->c, &A->g, &A->xN})
             b->alloc(vb(A));
         const int sms = num_sms(device);
+        A->sms = sms;
         A->splits = direct_choose_splits(precision, n, sms);
         const size_t sb = direct_scratch_bytes(precision, n, A->splits);
         // (whether the masses are equal is known only in the forward pass)
@@ -1391,9 +1462,8 @@ RRG_API rrg_status rrg_adjoint_create(int device, int precision, int64_t n, doub
         }
         if (!A->force_sym && sb) A->scratch.alloc(sb);
         if (precision == RRG_PREC_FP64) {
-            A->sym_slots.alloc(vjp_sym_slot_bytes<double>(n));
+            A->sym_slots.alloc(vjp_sym_slot_bytes<double>(n, sms));
         } else {
-            A->sms = sms;
             if (const size_t pairs = vjp_pair_bytes(n, sms)) {
                 try {
                     A->vjp_part.alloc(pairs);
@@ -1403,10 +1473,10 @@ RRG_API rrg_status rrg_adjoint_create(int device, int precision, int64_t n, doub
                 }
             }
             if (!A->vjp_pairs) {
-                A->vjp_splits = vjp_f32x2_splits(n, sms);
+                A->vjp_chunks = vjp_f32x2_chunks(n, sms);
                 // the reverse steps write partials even with one split
                 const size_t pb = sizeof(V4<float>) * static_cast<size_t>(n) *
-                                  static_cast<size_t>(std::max(1, A->vjp_splits));
+                                  static_cast<size_t>(A->vjp_chunks.splits);
                 A->vjp_part.alloc(pb);
                 A->vjp_part_a.alloc(pb);
             }
@@ -1537,7 +1607,7 @@ RRG_API rrg_status rrg_adjoint_backward(rrg_adjoint* A, const void* gx_final,
                                         step_update<float>(A, m - 1), &r, A->mass_grad);
                     else
                         vjp_reverse_launch(A->hsoft.p, A->uniform_h, A->uniform_m, A->n, A->c.p,
-                                           A->X.p, A->vjp_part.p, A->vjp_part_a.p, A->vjp_splits,
+                                           A->X.p, A->vjp_part.p, A->vjp_part_a.p, A->vjp_chunks,
                                            s, step_update<float>(A, m - 1), r, A->mass_grad);
                 }
             }
