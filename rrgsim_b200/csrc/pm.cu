@@ -64,9 +64,11 @@ __device__ __forceinline__ void cic_axis(double x, double dmin, double inv_dx, i
 // cell make long runs, but as they drift from the sorted order a warp's cells interleave. A warp
 // holding more than four runs therefore first sorts its (cell, lane) pairs with a bitonic
 // network of full-warp shuffles (15 compare-exchange steps) and takes each lane's values along.
-// Each of the 8 corner values is then summed over its run by a segmented warp scan (five
-// full-warp shuffles), and the run's last lane adds the eight sums with 64-bit atomics: one set
-// of atomics per distinct cell in the warp. Values fit in 27 bits (the scale S is chosen so that
+// Each of the 8 corner values is then summed over its run by a segmented warp scan (a full-warp
+// shuffle per doubling of the longest run), and the run's last lane adds the eight sums with 64-bit
+// atomics at fixed offsets from the cell: one set of atomics per distinct cell in the warp. (Always
+// five scan steps, and the corners taken from the cell's coordinates by divisions: 120.0 against
+// 116.2 us per PM step with 1M particles on 128^3; the pass issues 70 % of its cycles.) Values fit in 27 bits (the scale S is chosen so that
 // m_max 2^S <= 2^26), so a warp's sum fits 32 bits; integer sums are exact in any order, so the
 // grid does not depend on how particles fall into runs. (Grouping lanes with __match_any_sync and
 // summing each group with __reduce_add_sync cost more: every distinct group mask in a warp is a
@@ -171,27 +173,26 @@ __device__ __forceinline__ void cic_deposit_warp(bool active, double x, double y
     } else {
         const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));  // the run's first lane
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            unsigned v = q[c];
+        for (int c = 0; c < 8; ++c) sum[c] = q[c];
+        // distance d only while some run has more than d lanes (d lanes in a row that are no heads)
+        unsigned longer = ~heads;
+        for (int d = 1; longer != 0u; d <<= 1) {
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const unsigned t = __shfl_up_sync(0xffffffffu, v, d);
-                if (lane - d >= first) v += t;
+            for (int c = 0; c < 8; ++c) {
+                const unsigned t = __shfl_up_sync(0xffffffffu, sum[c], d);
+                if (lane - d >= first) sum[c] += t;
             }
-            sum[c] = v;  // at the run's last lane: the run's total
+            longer &= longer >> d;
         }
+        // (at the run's last lane: the run's total)
     }
     if (key >= 0 && tail) {
-        // the run's cell and its corners (clamped as cic_axis clamps)
-        const int a0 = key % nx, b0 = (key / nx) % nx, c0 = key / nx2;
-        const int a1 = min(a0 + 1, nx - 1), b1 = min(b0 + 1, nx - 1), c1 = min(c0 + 1, nx - 1);
-        const int ii[8] = {a0, a1, a0, a1, a0, a1, a0, a1};
-        const int jj[8] = {b0, b0, b1, b1, b0, b0, b1, b1};
-        const int kk[8] = {c0, c0, c0, c0, c1, c1, c1, c1};
+        // the run's cell and its corners (cic_axis keeps i0 <= nx - 2: no corner is clamped)
+        unsigned long long* const at = grid + key;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
             if (sum[c] != 0u)
-                atomicAdd(grid + (kk[c] * nx + jj[c]) * nx + ii[c],
+                atomicAdd(at + ((c & 1) + (c & 2 ? nx : 0) + (c & 4 ? nx2 : 0)),
                           static_cast<unsigned long long>(sum[c]));
         }
     }
