@@ -139,7 +139,7 @@ void launch_wave_step(int prec, int nx, const void* phi, void* phi_old_inout, co
 void launch_wave_adjoint_step(int prec, int nx, const void* C, void* P, void* F, double km,
                               double ka, double beta, double kf, cudaStream_t s);
 // Three substeps on a periodic FP32 grid (wave_march.cu): out = level 3, out_old = level 2, from
-// cur = level 0 and old = the level before it. The outputs are other buffers than the inputs; the
+// cur = level 0 and old = the level before it (null: zero). The outputs are other buffers than the inputs; the
 // same bits as three launch_wave_step. wave_march_applies: on grids that do not stay in L2.
 bool wave_march_applies(int nx);
 void launch_wave_march(int nx, const float* cur, const float* old, const float* src, float* out,
@@ -230,7 +230,8 @@ __device__ __forceinline__ float4 f4_add(const float4 a, const float4 b) {
 // kernels do not apply, and RRG_WAVE_PERSIST=0) then runs launch_wave_step on (d, d_old, g) with
 // K_F = 1, and finish writes phi0 + d_final and phi0 + d_before into fin and prv (either may be
 // phi0 itself). FP32 grids, periodic, uniform.
-// first: the first substep as well (d_old then holds level 1 of the increments, d level 0).
+// first: the first substep as well (d_old then holds level 1 of the increments, d level 0, which is
+// zero and not stored where d is null).
 void launch_wave_inc_prep(int nx, bool first, const unsigned long long* mg,
                           unsigned long long* mg_zero, int shift_s, double dx, double rho_sub,
                           const float* phi0, const float* phi_prev, const WaveCoef& w, float* g,

@@ -252,7 +252,8 @@ __global__ void wave_source_kernel(int64_t ncells, const unsigned long long* mgr
 
 // The incremental solve's preparation (wave_inc_source), V consecutive x-cells per thread.
 // FIRST: also the first substep, which needs no neighbours (the increments start at zero):
-// d_1 = K_OLD d_old + g, stored over d_old's place, with level 0 of the increments (zero) in d.
+// d_1 = K_OLD d_old + g, stored over d_old's place, with level 0 of the increments (zero) in d
+// (null: not stored).
 // Bound: HBM at 256^3 (32 to 36 B per cell); below, the FP64 arithmetic of g.
 template <int V, bool FIRST>
 __global__ void __launch_bounds__(256) wave_inc_prep_kernel(
@@ -309,7 +310,7 @@ __global__ void __launch_bounds__(256) wave_inc_prep_kernel(
         os.v[i] = static_cast<float>(sd);
     }
     *reinterpret_cast<C*>(g + c) = og;
-    *reinterpret_cast<C*>(d + c) = od;
+    if (d) *reinterpret_cast<C*>(d + c) = od;
     *reinterpret_cast<C*>(d_old + c) = oo;
     if (src) *reinterpret_cast<C*>(src + c) = os;
 }

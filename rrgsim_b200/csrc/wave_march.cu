@@ -39,7 +39,7 @@ constexpr int kStages = 6;               // planes in shared memory, copied kAhe
 constexpr int kAhead = kStages - 2;      // one before is still read, the one overwritten is not
 
 struct MarchArgs {
-    const float* cur;   // level 0 and the one before it
+    const float* cur;   // level 0 and the one before it (null: zero)
     const float* old;
     const float* src;
     float* out;         // level 3 and level 2
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(16 * kMaxRows, 1) wave_march_kernel(const Marc
             for (int r = 0; r < 2; ++r) {
                 const uint32_t to = sm0 + 8u * (sc + 32 * r);
                 copy8(to, a.cur + (zc * plane + at[r]));
-                copy8(to + 8u * buf, a.old + (zo * plane + at[r]));
+                if (a.old) copy8(to + 8u * buf, a.old + (zo * plane + at[r]));
                 copy8(to + 16u * buf, a.src + (zo * plane + at[r]));
             }
             zo = zc;
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(16 * kMaxRows, 1) wave_march_kernel(const Marc
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 v[0][f][r] = sm[so + me + 32 * r];
-                old[r] = sm[so + buf + me + 32 * r];
+                old[r] = a.old ? sm[so + buf + me + 32 * r] : zero;
                 g[f][r] = sm[so + 2 * buf + me + 32 * r];
             }
             // level k on plane p - k, from level k - 1 on planes p - k - 1 .. p - k + 1
