@@ -1083,8 +1083,10 @@ RRG_API rrg_status rrg_get_particles(rrg_ctx* ctx, double* pos, double* vel, dou
         const int64_t n = ctx->n;
         ensure_download(ctx, static_cast<size_t>(n) * 10 * sizeof(double));
         double* d = ctx->dl.as<double>();
-        launch_unpack_state(ctx->prec, n, ctx->sorted ? ctx->id.as<int32_t>() : nullptr,
-                            ctx->P(), ctx->L(), ctx->vel.p, ctx->acc.p, ctx->pot.p,
+        // (the sort's destinations are not needed between sorts)
+        uint32_t* slot = ctx->sorted ? ctx->sort_dest.as<uint32_t>() : nullptr;
+        if (slot) launch_inverse(n, ctx->id.as<int32_t>(), slot, ctx->stream);
+        launch_unpack_state(ctx->prec, n, slot, ctx->P(), ctx->L(), ctx->vel.p, ctx->acc.p, ctx->pot.p,
                             pos ? d : nullptr, vel ? d + 3 * n : nullptr,
                             acc ? d + 6 * n : nullptr, grav ? d + 9 * n : nullptr, ctx->stream);
         if (pos) RRG_CUDA(cudaMemcpyAsync(pos, d, 3 * n * 8, cudaMemcpyDeviceToHost, ctx->stream));

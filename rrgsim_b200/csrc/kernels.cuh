@@ -101,8 +101,10 @@ void launch_check_state(int64_t n, const double* pos3, const double* vel3, const
 void launch_pack_state(int prec, int64_t n, const double* pos3, const double* vel3,
                        const double* mass, const double* soft2, void* posm, void* poslo,
                        void* vel, void* hsoft, cudaStream_t s);
-// Gathers back into the original order through id (sorted slot -> original index).
-void launch_unpack_state(int prec, int64_t n, const int32_t* id, const void* posm,
+// slot[id[s]] = s: where a particle of the original order sits
+void launch_inverse(int64_t n, const int32_t* id, uint32_t* slot, cudaStream_t s);
+// The state as doubles in the original order (slot: null, or from launch_inverse).
+void launch_unpack_state(int prec, int64_t n, const uint32_t* slot, const void* posm,
                          const void* poslo, const void* vel, const void* acc, const void* pot,
                          double* pos3, double* vel3, double* acc3, double* grav,
                          cudaStream_t s);
