@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kBS, 2) vjp_pair_kernel(const VjpPairParams p)
 // ----------------------------------------------------------------------------------------------
 // Symmetric VJP: the pair term is antisymmetric (T_jk = -T_kj for x-bar), so each unordered
 // pair of particles is evaluated once. Blocks run over tile pairs (a, b), a <= b, of 256
-// particles: threads own k in tile a, tile b sits in shared memory. For a < b the j-side sums
+// particles: threads own k in tile a (two each), tile b sits in shared memory. For a < b the j-side sums
 // (x-bar_j -= T, m-bar_j += f (lam_k . d)) travel along the warp with the j they belong to (one
 // shuffle per sum and step, see the kernel) and each warp adds its sums for a chunk of 32 j into
 // a shared accumulator; block (a, b) then writes its tile-a sums to slot [a][b] and its
@@ -552,8 +552,11 @@ struct VjpSymParams {
 };
 
 
+// Two k per thread (tile a = k0 + 128 e): each j read from shared memory and each travelling sum
+// serves two pairs (one k per thread was bound by shared memory as much as by the FP64 pipe).
+constexpr int kSymThreads = kBS / 2;
 template <typename R, bool USOFT>
-__global__ void __launch_bounds__(kBS) vjp_sym_kernel(const VjpSymParams<R> p) {
+__global__ void __launch_bounds__(kSymThreads) vjp_sym_kernel(const VjpSymParams<R> p) {
     __shared__ V4<R> s_pos[kBS];
     __shared__ V4<R> s_lam[kBS];
     __shared__ R s_h[USOFT ? 1 : kBS];
@@ -572,58 +575,63 @@ __global__ void __launch_bounds__(kBS) vjp_sym_kernel(const VjpSymParams<R> p) {
     while (a > 0 && S(a) > t) --a;
     const int64_t b = t - S(a) + a;
 
-    const int64_t k = a * kBS + tid;
-    V4<R> pk = v4<R>(R(1e18), R(1e18), R(1e18), R(0)), lk = v4<R>(0, 0, 0, 0);
-    R hk = p.uniform_h;
-    if (k < p.n) {
-        pk = p.posm[k];
-        lk = p.lam[k];
-        if constexpr (!USOFT) hk = p.hsoft[k];
+    V4<R> pk[2], lk[2];
+    R hk[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int l = tid + e * kSymThreads;
+        pk[e] = v4<R>(R(1e18), R(1e18), R(1e18), R(0));
+        lk[e] = v4<R>(0, 0, 0, 0);
+        hk[e] = p.uniform_h;
+        const int64_t k = a * kBS + l;
+        if (k < p.n) {
+            pk[e] = p.posm[k];
+            lk[e] = p.lam[k];
+            if constexpr (!USOFT) hk[e] = p.hsoft[k];
+        }
+        const int64_t j = b * kBS + l;
+        const bool in = j < p.n;
+        s_pos[l] = in ? p.posm[j] : v4<R>(R(1e18), R(1e18), R(1e18), R(0));
+        s_lam[l] = in ? p.lam[j] : v4<R>(0, 0, 0, 0);
+        if constexpr (!USOFT) s_h[l] = in ? p.hsoft[j] : R(1);
+        s_acc[l][0] = s_acc[l][1] = s_acc[l][2] = s_acc[l][3] = R(0);
     }
-    const int64_t j = b * kBS + tid;
-    if (j < p.n) {
-        s_pos[tid] = p.posm[j];
-        s_lam[tid] = p.lam[j];
-        if constexpr (!USOFT) s_h[tid] = p.hsoft[j];
-    } else {
-        s_pos[tid] = v4<R>(R(1e18), R(1e18), R(1e18), R(0));
-        s_lam[tid] = v4<R>(0, 0, 0, 0);
-        if constexpr (!USOFT) s_h[tid] = R(1);
-    }
-    s_acc[tid][0] = s_acc[tid][1] = s_acc[tid][2] = s_acc[tid][3] = R(0);
     __syncthreads();
     const bool sym = (a != b);
-    R gx = 0, gy = 0, gz = 0, gm = 0;
-    // one pair (k, j): its k-side terms into (gx, gy, gz, gm), its j-side ones returned
-    auto pair = [&](int q, R& jx, R& jy, R& jz, R& jm) {
+    R gx[2] = {}, gy[2] = {}, gz[2] = {}, gm[2] = {};
+    // one j against both k: the k-side terms into (gx, gy, gz, gm), the j-side ones added to v
+    auto pairs = [&](int q, R v[4]) {
         const V4<R> pj = s_pos[q];
         const V4<R> lj = s_lam[q];
-        const R dx = pj.x - pk.x, dy = pj.y - pk.y, dz = pj.z - pk.z;
-        const R s = USOFT ? (hk + hk) : (hk + s_h[q]);
-        const R r2 = dx * dx + dy * dy + dz * dz + s;
-        const R inv = inv_sqrt(r2);
-        const R inv2 = inv * inv;
-        const R f = inv * inv2;
-        const R g = R(-3) * f * inv2;
-        const R ux = pk.w * lj.x - pj.w * lk.x;
-        const R uy = pk.w * lj.y - pj.w * lk.y;
-        const R uz = pk.w * lj.z - pj.w * lk.z;
-        const R tt = g * (dx * ux + dy * uy + dz * uz);
-        const R Tx = f * ux + tt * dx, Ty = f * uy + tt * dy, Tz = f * uz + tt * dz;
-        gx += Tx;
-        gy += Ty;
-        gz += Tz;
-        gm -= f * (dx * lj.x + dy * lj.y + dz * lj.z);
-        jx = -Tx;
-        jy = -Ty;
-        jz = -Tz;
-        jm = f * (dx * lk.x + dy * lk.y + dz * lk.z);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const R dx = pj.x - pk[e].x, dy = pj.y - pk[e].y, dz = pj.z - pk[e].z;
+            const R s = USOFT ? (hk[e] + hk[e]) : (hk[e] + s_h[q]);
+            const R r2 = dx * dx + dy * dy + dz * dz + s;
+            const R inv = inv_sqrt(r2);
+            const R inv2 = inv * inv;
+            const R f = inv * inv2;
+            const R g = R(-3) * f * inv2;
+            const R ux = pk[e].w * lj.x - pj.w * lk[e].x;
+            const R uy = pk[e].w * lj.y - pj.w * lk[e].y;
+            const R uz = pk[e].w * lj.z - pj.w * lk[e].z;
+            const R tt = g * (dx * ux + dy * uy + dz * uz);
+            const R Tx = f * ux + tt * dx, Ty = f * uy + tt * dy, Tz = f * uz + tt * dz;
+            gx[e] += Tx;
+            gy[e] += Ty;
+            gz[e] += Tz;
+            gm[e] -= f * (dx * lj.x + dy * lj.y + dz * lj.z);
+            v[0] -= Tx;
+            v[1] -= Ty;
+            v[2] -= Tz;
+            v[3] += f * (dx * lk[e].x + dy * lk[e].y + dz * lk[e].z);
+        }
     };
     if (!sym) {
 #pragma unroll 2
         for (int q = q0; q < q0 + len; ++q) {
-            R jx, jy, jz, jm;
-            pair(q, jx, jy, jz, jm);
+            R v[4] = {};
+            pairs(q, v);
         }
     } else {
         // the j-side terms ride along the warp: in step t of a chunk of 32 j, lane l takes
@@ -631,29 +639,27 @@ __global__ void __launch_bounds__(kBS) vjp_sym_kernel(const VjpSymParams<R> p) {
         // 32 steps lane l holds its warp's sums for j = 32 c + l (one shuffle per sum and step,
         // and one shared add per chunk, instead of a warp reduction per j)
         for (int c = q0 / 32; c < (q0 + len) / 32; ++c) {
-            R ax = 0, ay = 0, az = 0, am = 0;
-#pragma unroll 4
+            R v[4] = {};
+#pragma unroll 2
             for (int t = 0; t < 32; ++t) {
-                R jx, jy, jz, jm;
-                pair(c * 32 + ((lane + t) & 31), jx, jy, jz, jm);
+                pairs(c * 32 + ((lane + t) & 31), v);
                 const int from = (lane + 1) & 31;
-                ax = __shfl_sync(0xffffffffu, ax + jx, from);
-                ay = __shfl_sync(0xffffffffu, ay + jy, from);
-                az = __shfl_sync(0xffffffffu, az + jz, from);
-                am = __shfl_sync(0xffffffffu, am + jm, from);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[k] = __shfl_sync(0xffffffffu, v[k], from);
             }
-            atomicAdd(&s_acc[c * 32 + lane][0], ax);
-            atomicAdd(&s_acc[c * 32 + lane][1], ay);
-            atomicAdd(&s_acc[c * 32 + lane][2], az);
-            atomicAdd(&s_acc[c * 32 + lane][3], am);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) atomicAdd(&s_acc[c * 32 + lane][k], v[k]);
         }
     }
-    p.slots[((a * T + b) * p.parts + part) * kBS + tid] = v4<R>(gx, gy, gz, gm);
+    V4<R>* const ks = p.slots + ((a * T + b) * p.parts + part) * kBS;
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+        ks[tid + e * kSymThreads] = v4<R>(gx[e], gy[e], gz[e], gm[e]);
     if (sym) {
         __syncthreads();
-        if (tid >= q0 && tid < q0 + len)  // (every j of the tile is in one part)
-            p.slots[(b * T + a) * p.parts * kBS + tid] =
-                v4<R>(s_acc[tid][0], s_acc[tid][1], s_acc[tid][2], s_acc[tid][3]);
+        for (int l = q0 + tid; l < q0 + len; l += kSymThreads)  // (every j of the tile is in one part)
+            p.slots[(b * T + a) * p.parts * kBS + l] =
+                v4<R>(s_acc[l][0], s_acc[l][1], s_acc[l][2], s_acc[l][3]);
     }
 }
 
@@ -702,13 +708,15 @@ vjp_sym_finish(int64_t n, int T, int parts, const V4<R>* __restrict__ slots, V4<
     if (upd.V) adjoint_update_at(k, r.x, r.y, r.z, upd);
 }
 
-// Parts of a tile pair: 1, 2, 4 or 8, the most that keep the blocks within four per SM. Whole pairs
-// leave SMs idle below ~8,000 particles (N = 2,000: 36 blocks). Product and finish, us, whole pairs ->
-// parts: N = 1,000 56.6 -> 12.1, 2,000 57.3 -> 18.5, 5,000 100 -> 76.6, 8,000 (whole) 195 -> 191.
+// Parts of a tile pair: 1, 2, 4 or 8, the most that keep the blocks within eight per SM. Whole pairs
+// leave SMs idle below ~8,000 particles (N = 2,000: 36 blocks) and fill the last ones badly above.
+// Product and finish, us, whole pairs and one k per thread -> parts -> two k per thread: N = 1,000
+// 56.6 -> 11.9 -> 13.2, 2,000 57.3 -> 18.7 -> 16.7, 3,000 - -> 42.1 -> 29.7, 5,000 100 -> 76.6 -> 59.6,
+// 6,500 - -> 146 -> 94.5, 8,000 195 -> 192 -> 138 (four blocks per SM: 5,000 61.2, 8,000 147).
 int vjp_sym_parts(int64_t n, int sms) {
     const int64_t T = (n + kBS - 1) / kBS, blocks = T * (T + 1) / 2;
     int parts = 1;
-    while (parts < 8 && 2 * parts * blocks <= 4 * static_cast<int64_t>(sms)) parts *= 2;
+    while (parts < 8 && 2 * parts * blocks <= 8 * static_cast<int64_t>(sms)) parts *= 2;
     return parts;
 }
 
@@ -733,8 +741,8 @@ void vjp_sym_launch(const void* posm, const void* hsoft, double uniform_h, int64
     p.lam = static_cast<const V4<R>*>(lam);
     p.slots = static_cast<V4<R>*>(slots);
     const unsigned blocks = static_cast<unsigned>(static_cast<int64_t>(T) * (T + 1) / 2 * p.parts);
-    if (hsoft) vjp_sym_kernel<R, false><<<blocks, kBS, 0, stream>>>(p);
-    else vjp_sym_kernel<R, true><<<blocks, kBS, 0, stream>>>(p);
+    if (hsoft) vjp_sym_kernel<R, false><<<blocks, kSymThreads, 0, stream>>>(p);
+    else vjp_sym_kernel<R, true><<<blocks, kSymThreads, 0, stream>>>(p);
     RRG_LAUNCHED();
     vjp_sym_finish<R><<<div_up(n, 32), dim3(32, kFinWarps), 0, stream>>>(
         n, T, p.parts, p.slots, static_cast<V4<R>*>(out), accumulate ? 1 : 0, upd);
