@@ -687,35 +687,38 @@ void run_steps(rrg_ensemble* e, int nsteps) {
     count_launches(1 + 2 * nsteps);
 }
 
-// Times one force evaluation per candidate (tile variant and j-chunk; each pair once) and keeps the
-// fastest.
+// Times one force evaluation per candidate (the pair forms, tile variants and j-chunks) and keeps the
+// fastest. An ordered variant is sampled at two j-chunks, and at the others only where one of the two
+// comes within 15 % of the best: creating an ensemble of 8 galaxies 11.7 -> 8.3 ms, 24 galaxies of up to
+// 16,384 particles 44 -> 31.
 void autotune(rrg_ensemble* e) {
     cudaEvent_t a, b;
     RRG_CUDA(cudaEventCreate(&a));
     RRG_CUDA(cudaEventCreate(&b));
     float best = 1e30f;
     int bv = 1, bj = 4096;
-    for (int v : {1, 2, 3, 4}) {
-        for (int j : {1024, 2048, 4096, 8192, 16384}) {
-            if (v >= 3) {
-                if (j != 1024) break;  // (no j-chunk)
-                build_pairs(e, v);
-            } else {
-                build_worklist(e, v, j);
-            }
-            launch_forces(e, e->posm[e->cur].p);  // warm
-            RRG_CUDA(cudaEventRecord(a, e->stream));
-            for (int r = 0; r < 2; ++r) launch_forces(e, e->posm[e->cur].p);
-            RRG_CUDA(cudaEventRecord(b, e->stream));
-            RRG_CUDA(cudaEventSynchronize(b));
-            float ms = 0.f;
-            RRG_CUDA(cudaEventElapsedTime(&ms, a, b));
-            if (ms < best) {
-                best = ms;
-                bv = v;
-                bj = j;
-            }
+    auto consider = [&](int v, int j) {
+        if (v >= 3) build_pairs(e, v);
+        else build_worklist(e, v, j);
+        launch_forces(e, e->posm[e->cur].p);  // warm
+        RRG_CUDA(cudaEventRecord(a, e->stream));
+        for (int r = 0; r < 2; ++r) launch_forces(e, e->posm[e->cur].p);
+        RRG_CUDA(cudaEventRecord(b, e->stream));
+        RRG_CUDA(cudaEventSynchronize(b));
+        float ms = 0.f;
+        RRG_CUDA(cudaEventElapsedTime(&ms, a, b));
+        if (ms < best) {
+            best = ms;
+            bv = v;
+            bj = j;
         }
+        return ms;
+    };
+    for (int v : {3, 4}) consider(v, 1024);  // (no j-chunk)
+    for (int v : {1, 2}) {
+        const float two = std::min(consider(v, 2048), consider(v, 8192));
+        if (two <= 1.15f * best)
+            for (int j : {1024, 4096, 16384}) consider(v, j);
     }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
