@@ -471,15 +471,17 @@ void apply_l2_window(rrg_ctx* c) {
     c->l2_stream = c->stream;
 }
 
-// After a synchronisation: the persistent solve's error word is set when a wait between its
-// thread blocks ran out, which leaves the steps since the last check invalid.
-void check_wave_solve(rrg_ctx* c) {
-    if (!c->wave_solve_used || !c->wsync.p) return;
-    unsigned int e = 0;
-    RRG_CUDA(cudaMemcpyAsync(&e, c->wsync.as<char>() + kWaveSyncErrOffset, 4,
-                             cudaMemcpyDeviceToHost, c->stream));
+// Synchronises the stream. The persistent solve's error word is set when a wait between its thread
+// blocks ran out, which leaves the steps since the last check invalid; it is fetched ahead of the
+// synchronisation, into pinned memory, so that looking at it costs no second one.
+void sync_checked(rrg_ctx* c) {
+    const bool look = c->wave_solve_used && c->wsync.p;
+    auto* e = reinterpret_cast<unsigned int*>(c->host_red + 15);
+    if (look)
+        RRG_CUDA(cudaMemcpyAsync(e, c->wsync.as<char>() + kWaveSyncErrOffset, 4,
+                                 cudaMemcpyDeviceToHost, c->stream));
     RRG_CUDA(cudaStreamSynchronize(c->stream));
-    if (e != 0) {
+    if (look && *e != 0) {
         RRG_CUDA(cudaMemsetAsync(c->wsync.p, 0, c->wsync.bytes, c->stream));
         RRG_CUDA(cudaStreamSynchronize(c->stream));
         throw Error(RRG_ERR_CUDA,
@@ -559,7 +561,7 @@ int solve_wave(rrg_ctx* c, int max_iterations, double* last_rel) {
                 if (check) {
                     read(&r, result, sizeof r);
                     if (r.done == 0) {
-                        check_wave_solve(c);
+                        sync_checked(c);
                         throw Error(RRG_ERR_CUDA, "wave solve: the relaxation did not run");
                     }
                 }
@@ -589,7 +591,7 @@ int solve_wave(rrg_ctx* c, int max_iterations, double* last_rel) {
             if (hold >= c->wave.steady_hold_steps) break;
         }
     }
-    if (synced) check_wave_solve(c);
+    if (synced) sync_checked(c);
     if (last_rel) *last_rel = rel;
     return it;
 }
@@ -939,8 +941,7 @@ RRG_API rrg_status rrg_set_stream(rrg_ctx* ctx, void* stream) {
 
 RRG_API rrg_status rrg_synchronize(rrg_ctx* ctx) {
     RRG_ENTRY(ctx, {
-        RRG_CUDA(cudaStreamSynchronize(ctx->stream));
-        check_wave_solve(ctx);
+        sync_checked(ctx);
         ctx->sums_ready = entry_sums_ready;
     })
 }
@@ -1096,8 +1097,7 @@ RRG_API rrg_status rrg_get_particles(rrg_ctx* ctx, double* pos, double* vel, dou
             RRG_CUDA(cudaMemcpyAsync(acc, d + 6 * n, 3 * n * 8, cudaMemcpyDeviceToHost, ctx->stream));
         if (grav)
             RRG_CUDA(cudaMemcpyAsync(grav, d + 9 * n, n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-        RRG_CUDA(cudaStreamSynchronize(ctx->stream));
-        check_wave_solve(ctx);
+        sync_checked(ctx);
         ctx->sums_ready = entry_sums_ready;
     })
 }
@@ -1404,11 +1404,11 @@ static void conservation_sums(rrg_ctx* ctx, bool com, bool ready, double* out) {
 }
 
 static void reduce_state(rrg_ctx* ctx, bool com, bool ready) {
-    conservation_sums(ctx, com, ready, ctx->red_out.as<double>());
-    RRG_CUDA(cudaMemcpyAsync(ctx->host_red, ctx->red_out.p, 12 * sizeof(double),
-                             cudaMemcpyDeviceToHost, ctx->stream));
-    RRG_CUDA(cudaStreamSynchronize(ctx->stream));
-    check_wave_solve(ctx);
+    // straight into pinned memory: no copy after the finishing kernel
+    void* out = nullptr;
+    RRG_CUDA(cudaHostGetDevicePointer(&out, ctx->host_red, 0));
+    conservation_sums(ctx, com, ready, static_cast<double*>(out));
+    sync_checked(ctx);
 }
 
 RRG_API rrg_status rrg_calc_conservation(rrg_ctx* ctx, rrg_conservation* out) {
@@ -1517,8 +1517,7 @@ RRG_API rrg_status rrg_solver_precalc(rrg_ctx* ctx) {
             e.pot = ctx->pot.p;
             direct(ctx, true, e);
         }
-        RRG_CUDA(cudaStreamSynchronize(ctx->stream));
-        check_wave_solve(ctx);
+        sync_checked(ctx);
     })
 }
 
