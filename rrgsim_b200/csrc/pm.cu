@@ -264,15 +264,18 @@ __global__ void __launch_bounds__(256) wave_inc_prep_kernel(
     float* src) {
     using C = Cells<float, V>;
     const int W = nx / V;
-    const int64_t u = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t units = static_cast<int64_t>(W) * nx * nx;
+    // (at most 2^30 units: 32-bit divisions; PM step with 64-bit ones 256^3 845 against 837 us)
+    const unsigned int u = blockIdx.x * 256u + threadIdx.x;
+    const unsigned int units = static_cast<unsigned int>(W) * nx * nx;
     if (u >= units) {  // (every block waits)
         pdl_wait();
         return;
     }
-    const int q = static_cast<int>(u % W);
-    const int64_t row = u / W;
-    const int y = static_cast<int>(row % nx), z = static_cast<int>(row / nx);
+    const unsigned int r0 = u / static_cast<unsigned int>(W);
+    const int q = static_cast<int>(u - r0 * W);
+    const int z = static_cast<int>(r0 / static_cast<unsigned int>(nx)),
+              y = static_cast<int>(r0) - z * nx;
+    const int64_t row = r0;
     const int64_t plane = static_cast<int64_t>(nx) * nx;
     const int64_t c = row * nx + q * V;
     pdl_wait();
