@@ -315,10 +315,13 @@ void gradient_after(rrg_ctx* c, int k) {
 // first increment, the plain source when store_src, the next deposit target cleared), the
 // substeps, the finish (the levels in full) and the gradient; the increments and their source
 // live in the field buffer (acc4: 4 floats per cell), which the gradient rewrites at the end.
-// False (nothing launched) on other grids and precisions: the caller launches the reference's
-// full-level form (wave_source + wave_substep x iterations + gradient).
+// False (nothing launched) on other grids and precisions, and for no substeps (the increments would
+// round the level before the current one): the caller launches the reference's full-level form
+// (wave_source + wave_substep x iterations + gradient).
 bool solve_step_fused(rrg_ctx* c, const WaveCoef& w, int iterations, bool store_src) {
-    if (c->prec == RRG_PREC_FP64 || c->bc_type != RRG_BC_PERIODIC || c->keep_layer) return false;
+    if (c->prec == RRG_PREC_FP64 || c->bc_type != RRG_BC_PERIODIC || c->keep_layer ||
+        iterations < 1)
+        return false;
     const int nx = c->grid.nx;
     if (launch_wave_solve(nx, iterations, c->phi[0].as<float>(), c->phi[1].as<float>(),
                           c->phi_cur, c->mg[c->mg_cur].as<unsigned long long>(),

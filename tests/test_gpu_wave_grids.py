@@ -67,3 +67,38 @@ def test_adjoint_on_other_rows_matches_autograd(nx, every):
         grads.append((xr.grad, vr.grad, mr.grad))
     for a, b in zip(*grads):
         assert float(torch.linalg.norm(a - b) / torch.linalg.norm(b)) <= 1e-6
+
+
+@pytest.mark.parametrize("prec", ["fp32", "mixed", "fp64"])
+@pytest.mark.parametrize("nx", [32, 33, 40, 96])
+@pytest.mark.parametrize("steps", [3, 4])
+def test_zero_substeps_leave_the_levels_alone(prec, nx, steps):
+    """Steps in a frozen potential: both levels keep their bits, and the particles follow the FP64
+    context's. Bars: four roundings a step of coordinates below 8 and of velocities below 2, with
+    the few roundings of the accelerations below them by dt."""
+    pos, vel, m, s2 = disk(3000, seed=nx)
+    g = rg.GridInfo.from_values(nx, 16.0 / nx, 0.0)
+    wp = rg.WaveParams.make(g.dx, diss_base=1.0 / (4 * g.dx), wave_speed=9.0, iterations=0,
+                            setup_iterations=0)
+    rng = np.random.default_rng(nx)
+    phi = f32(-1.0 + 0.01 * rng.standard_normal(nx ** 3))
+    before = f32(phi + 0.01 * rng.standard_normal(nx ** 3))
+    sim = rg.SimParams(time_max=1.0, dt_save=0.1, dt_dynamics=2e-3, saves_without_dump=0,
+                       use_wave_model=1)
+    got = {}
+    for p in (prec, "fp64"):
+        with rg.Context(0, p) as c:
+            c.load_particles(f32(pos), f32(vel), m, s2)
+            c.init_grid(g)
+            c.set_wave_params(wp)
+            c.solver_init(sim)
+            c.set_wave_state(phi, before)
+            c.resume()
+            c.sync_particles_and_grid()
+            c.calc_steps(steps)
+            cur, prev = c.get_wave_state()
+            got[p] = c.get_particles()
+        np.testing.assert_array_equal(cur, phi)
+        np.testing.assert_array_equal(prev, before)
+    assert np.max(np.abs(got[prec]["pos"] - got["fp64"]["pos"])) <= steps * 4 * 2.0 ** -24 * 8
+    assert np.max(np.abs(got[prec]["vel"] - got["fp64"]["vel"])) <= steps * 4 * 2.0 ** -24 * 2
