@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(kSymThreads) vjp_sym_kernel(const VjpSymParams
         if (k < p.n) {
             pk[e] = p.posm[k];
             lk[e] = p.lam[k];
-            if constexpr (!USOFT) hk[e] = p.hsoft[k];
+            if constexpr (!USOFT) hk[e] = pair_soft(p.hsoft[k]);
         }
         const int64_t j = b * kBS + l;
         const bool in = j < p.n;
@@ -734,7 +734,7 @@ void vjp_sym_launch(const void* posm, const void* hsoft, double uniform_h, int64
     VjpSymParams<R> p;
     p.posm = static_cast<const V4<R>*>(posm);
     p.hsoft = static_cast<const R*>(hsoft);
-    p.uniform_h = static_cast<R>(uniform_h);
+    p.uniform_h = pair_soft(static_cast<R>(uniform_h));
     p.n = n;
     p.tiles = T;
     p.parts = vjp_sym_parts(n, sms);

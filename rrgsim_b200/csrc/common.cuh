@@ -69,19 +69,30 @@ __device__ __forceinline__ float rsqrt_sfu(float x) {
     return y;
 }
 
-// FP64 reciprocal square root without branches, for pair loops (x >= 0): the SFU's approximation y
+// FP64 reciprocal square root without branches, for pair loops (x > 0): the SFU's approximation y
 // (PTX rsqrt.approx.ftz.f64, at least 20 bits) refined once by the binomial series of
 // x^-1/2 = y (1 - e)^-1/2, e = 1 - x y^2, to second order: y (1 + e / 2 + 3 e^2 / 8), whose next
 // term is below 2^-57. Within 2 ulp of the exact value; CUDA's rsqrt branches for special values,
-// which keeps a loop's independent pairs from overlapping. x above 1e300 (infinity included) counts
-// as 1e300: the cube of the result is 0 there and the result itself far below any other term.
+// which keeps a loop's independent pairs from overlapping. e takes infinity as a finite number, so
+// that the result there is y = 0; NaN and negative x give NaN. Below the smallest normal number,
+// which y flushes, e is -infinity and the result +infinity. At x = 0 e would be NaN: callers lift
+// the softening of a pair off zero (pair_soft) by the smallest positive number, which any distance
+// but 0 swallows. (One integer operation, off the FP64 pipe. With 0 handled here, the direct sum of
+// 20,011 particles took 2.4 % longer by a second clamp and 4 % by a select on the result.)
 __device__ __forceinline__ double rsqrt_pair(double x) {
-    // (positive doubles compare as their high words; 0x7E37E43C is that of 1e300)
-    x = __hiloint2double(min(__double2hiint(x), 0x7E37E43C), __double2loint(x));
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
+    // (positive doubles compare as their high words; 0x7FEFFFFF is that of the largest finite ones)
+    const double c = __hiloint2double(min(__double2hiint(x), 0x7FEFFFFF), __double2loint(x));
+    const double e = fma(-(c * y), y, 1.0);
     return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// A particle's softening for pairs: FP64 zero becomes the smallest positive number (rsqrt_pair).
+template <typename R>
+__host__ __device__ __forceinline__ R pair_soft(R h) {
+    if constexpr (sizeof(R) == 8) return h == 0.0 ? 4.9406564584124654e-324 : h;
+    else return h;
 }
 
 // Error-free transformations for double-float arithmetic (Knuth TwoSum, Dekker Fast2Sum).

@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(kBS) direct_f64_kernel(const F64Params p) {
     pdl_next();  // (the finish may start and wait)
     if (i < p.n) {
         pi = p.posm[i];
-        if constexpr (!USOFT) h = p.hsoft[i];
+        if constexpr (!USOFT) h = pair_soft(p.hsoft[i]);
     }
     double ax = 0, ay = 0, az = 0, ap = 0;
     const int64_t jb = static_cast<int64_t>(blockIdx.y) * p.jchunk;
@@ -699,7 +699,7 @@ void launch_direct(const DirectLaunch& L) {
         F64Params p;
         p.posm = static_cast<const V4<double>*>(L.posm);
         p.hsoft = static_cast<const double*>(L.hsoft);
-        p.uniform_h = L.uniform_hsoft;
+        p.uniform_h = pair_soft(L.uniform_hsoft);
         p.n = L.n;
         p.jchunk = jchunk;
         p.part = static_cast<V4<double>*>(L.scratch);

@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kThreads) direct_small_kernel(const SmallParam
     R hi = p.uniform_h;
     if (i < p.n) {
         pi = p.posm[i];
-        if constexpr (!USOFT) hi = p.hsoft[i];
+        if constexpr (!USOFT) hi = pair_soft(p.hsoft[i]);
         if constexpr (MIXED) li = p.poslo[i];
     }
     const R hh = USOFT ? hi + hi : hi;
@@ -239,7 +239,7 @@ void launch_direct_small(const DirectLaunch& L, int sms) {
         p.posm = static_cast<const V4<R>*>(L.posm);
         p.poslo = static_cast<const V4<float>*>(L.poslo);
         p.hsoft = static_cast<const R*>(L.hsoft);
-        p.uniform_h = static_cast<R>(L.uniform_hsoft);
+        p.uniform_h = pair_soft(static_cast<R>(L.uniform_hsoft));
         p.uniform_m = static_cast<R>(L.uniform_mass);
         p.n = static_cast<int>(L.n);
         p.epi = make_epi<R>(L.epi);

@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kBS, 2) direct_sym64_kernel(const SymParams<do
             hi[g] = USOFT ? p.uniform_h + p.uniform_h : 1.0;
             if (i < pl.n) {
                 pi = p.posm[i];
-                if constexpr (!USOFT) hi[g] = p.hsoft[i];
+                if constexpr (!USOFT) hi[g] = pair_soft(p.hsoft[i]);
             }
             xi[g] = pi.x;
             yi[g] = pi.y;
@@ -645,7 +645,7 @@ void launch_direct_sym(const DirectLaunch& L, int sms) {
         p.plan = pl;
         p.posm = static_cast<const V4<double>*>(L.posm);
         p.hsoft = static_cast<const double*>(L.hsoft);
-        p.uniform_h = L.uniform_hsoft;
+        p.uniform_h = pair_soft(L.uniform_hsoft);
         p.js = static_cast<V4<double>*>(L.sym_scratch);
         p.is = p.js + rows * L.n;
         p.js2 = p.is + static_cast<size_t>(pl.islots) * L.n;

@@ -58,3 +58,39 @@ def test_fp64_force_over_the_exponent_range():
         got = c.get_particles()["acc"]
     assert np.all(np.isfinite(got)) and abs(got[0, 0] - 1.0001 ** -1.5) <= 1e-14
     assert np.all(got[2] == 0.0)
+
+
+@pytest.mark.parametrize("n", [4000, 6000, 9000])  # one launch, ordered pairs, each pair once
+def test_fp64_reciprocal_root_over_all_exponents(n):
+    """Massless particles on top of one of mass 1 without softening: the potential of a particle is
+    -1 / sqrt(x) of half its softening squared, with no other rounding. Within 2 ulp; the mass-1
+    particle's own term at distance 0 is -inf."""
+    rng = np.random.default_rng(n)
+    x = np.ldexp(rng.uniform(1.0, 2.0, n), rng.integers(-1000, 1001, n))
+    x[1:4] = [2.0 ** -1000, 1e300, 2.0 ** 1001]
+    s2, m = 2.0 * x, np.zeros(n)
+    s2[0], m[0] = 0.0, 1.0
+    with rg.Context(0, "fp64") as c:
+        c.load_particles(np.zeros((n, 3)), np.zeros((n, 3)), m, s2)
+        c.nbody_grav()
+        pot = c.get_particles()["grav"]
+    assert pot[0] == -np.inf
+    want = -1.0 / np.sqrt(x[1:].astype(np.longdouble))
+    assert np.max(np.abs(pot[1:] - want) / np.spacing(np.abs(want.astype(np.float64)))) <= 2.0
+
+
+@pytest.mark.parametrize("n", [3, 6000, 9000])
+def test_fp64_potential_shows_a_particle_without_a_position(n):
+    """A particle without softening has no force from itself (0 / 0), so its next position is NaN,
+    and the potentials of all others show it."""
+    pos, _, m, s2 = _case(n, "")
+    s2 = np.array(s2)
+    s2[2] = 0.0
+    with rg.Context(0, "fp64") as c:
+        c.load_particles(pos, np.zeros((n, 3)), m, s2)
+        c.nbody_acceleration()
+        c.predict_step(1e-3)
+        c.nbody_grav()
+        got = c.get_particles()
+    assert np.flatnonzero(np.isnan(got["pos"]).any(1)).tolist() == [2]
+    assert np.all(np.isnan(got["grav"]))
