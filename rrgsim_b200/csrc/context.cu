@@ -265,15 +265,25 @@ void direct(rrg_ctx* c, bool want_pot, const DirectEpi& epi) {
 
 void drop_graphs(rrg_ctx* c);
 
+// Allocations that a caller's stream capture may surround: the calling thread's capture mode is
+// relaxed meanwhile (in the default mode cudaMalloc fails and invalidates the capture).
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // The pair slots of the symmetric direct sum (direct_sym.cu), where that is the faster path; a
 // device without room for them runs the ordered kernels. Called before the first direct sum on
-// new particles, never while a graph is recorded.
+// new particles, never while the context records a graph of its own. The slots serve equal and
+// unequal masses, so that a reload of as many particles keeps the buffer.
 void ensure_sym(rrg_ctx* c) {
     if (c->n <= 0) return;
     const void* before = c->sym_scratch.p;
+    const RelaxedCapture relaxed;
     try {
-        c->sym_scratch.alloc(
-            direct_sym_scratch_bytes(c->prec, c->n, c->uniform_mass >= 0.0, c->sms));
+        c->sym_scratch.alloc(std::max(direct_sym_scratch_bytes(c->prec, c->n, true, c->sms),
+                                      direct_sym_scratch_bytes(c->prec, c->n, false, c->sms)));
     } catch (const Error&) {
         c->sym_scratch.release();
     }

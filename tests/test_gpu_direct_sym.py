@@ -92,3 +92,30 @@ def test_reload_with_another_mass_and_size(prec):
             want = steps(c, n, scale)
         for k in ("pos", "vel", "acc"):
             np.testing.assert_array_equal(g[k], want[k])
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+def test_first_evaluation_under_capture(prec):
+    """The first evaluation of a context may be one that its caller captures (in the default mode, in
+    which an allocation breaks a capture); the replay gives the bits of an evaluation outside."""
+    torch = pytest.importorskip("torch")
+    pos, vel, m, s2 = plummer(9000, seed=3)
+    with rg.Context(0, prec) as c:
+        c.load_particles(pos, vel, m, s2)
+        c.nbody_acceleration()
+        want = c.get_particles()["acc"]
+    s = torch.cuda.Stream()
+    with rg.Context(0, prec) as c:
+        c.load_particles(pos, vel, m, s2)
+        c.synchronize()
+        c.set_stream(s.cuda_stream)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            c.nbody_acceleration()
+        with torch.cuda.stream(s):
+            graph.replay()
+        got = c.get_particles()["acc"]
+        c.nbody_acceleration()  # outside the capture again
+        again = c.get_particles()["acc"]
+    np.testing.assert_array_equal(got, want)
+    np.testing.assert_array_equal(again, want)
