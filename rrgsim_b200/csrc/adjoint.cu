@@ -1116,11 +1116,15 @@ void vjp_pair_dispatch(const VjpPairParams& p, bool mgrad, bool force, cudaStrea
 // step; then the adjoint update upd.
 void vjp_pair_launch(const void* posm, const void* hsoft, double uniform_h, double uniform_m,
                      int64_t n, const void* lam, void* out, bool accumulate, void* slots,
-                     int sms, cudaStream_t s, const AdjUpd<float>& upd, const RevStep* r,
+                     size_t slot_bytes, int sms, cudaStream_t s, const AdjUpd<float>& upd, const RevStep* r,
                      bool mgrad) {
     const bool umass = uniform_m >= 0;
+    RRG_REQUIRE(pair_plan_range(n), RRG_ERR_INVALID,
+                "vjp: too few or too many particles for pair slots");
     VjpPairParams p{};
     p.plan = vjp_pair_plan(n, sms, umass);
+    RRG_REQUIRE(slot_bytes >= 2 * sizeof(V4<float>) * static_cast<size_t>(vjp_pair_records(p.plan)),
+                RRG_ERR_INVALID, "vjp: pair slots smaller than the schedule needs");
     p.posm = static_cast<const V4<float>*>(posm);
     p.hsoft = static_cast<const float*>(hsoft);
     p.uniform_h = static_cast<float>(uniform_h);
@@ -1282,6 +1286,7 @@ void forces(rrg_adjoint* A, const void* x, void* acc, cudaStream_t s) {
     L.scratch = A->scratch.p;
     L.scratch_bytes = A->scratch.bytes;
     L.sym_scratch = A->force_sym ? A->scratch.p : nullptr;
+    L.sym_scratch_bytes = A->force_sym ? A->scratch.bytes : 0;
     L.stream = s;
     launch_direct(L);
 }
@@ -1308,6 +1313,7 @@ void direct_step(rrg_adjoint* A, const void* in, void* out, void* vel, void* acc
     L.scratch = A->scratch.p;
     L.scratch_bytes = A->scratch.bytes;
     L.sym_scratch = A->force_sym ? A->scratch.p : nullptr;
+    L.sym_scratch_bytes = A->force_sym ? A->scratch.bytes : 0;
     L.stream = s;
     launch_direct(L);
 }
@@ -1339,8 +1345,8 @@ void vjp(rrg_adjoint* A, const void* x, int m, cudaStream_t s) {
                                A->sym_slots.p, A->sms, s, step_update<double>(A, m));
     else if (A->vjp_pairs)
         vjp_pair_launch(x, A->hsoft.p, A->uniform_h, A->uniform_m, A->n, A->c.p, A->X.p, true,
-                        A->vjp_part.p, A->sms, s, step_update<float>(A, m), nullptr,
-                        A->mass_grad);
+                        A->vjp_part.p, A->vjp_part.bytes, A->sms, s, step_update<float>(A, m),
+                        nullptr, A->mass_grad);
     else
         vjp_f32x2_launch(x, A->hsoft.p, A->uniform_h, A->uniform_m, A->n, A->c.p, A->X.p, true,
                          A->vjp_part.p, A->vjp_chunks, s, step_update<float>(A, m),
@@ -1611,7 +1617,7 @@ RRG_API rrg_status rrg_adjoint_backward(rrg_adjoint* A, const void* gx_final,
                     r.dt = static_cast<float>(A->dt);
                     if (A->vjp_pairs)
                         vjp_pair_launch(r.x, A->hsoft.p, A->uniform_h, A->uniform_m, A->n, A->c.p,
-                                        A->X.p, true, A->vjp_part.p, A->sms, s,
+                                        A->X.p, true, A->vjp_part.p, A->vjp_part.bytes, A->sms, s,
                                         step_update<float>(A, m - 1), &r, A->mass_grad);
                     else
                         vjp_reverse_launch(A->hsoft.p, A->uniform_h, A->uniform_m, A->n, A->c.p,

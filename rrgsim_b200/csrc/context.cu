@@ -259,6 +259,7 @@ void direct(rrg_ctx* c, bool want_pot, const DirectEpi& epi) {
     L.scratch = c->scratch.p;
     L.scratch_bytes = c->scratch.bytes;
     L.sym_scratch = c->sym_scratch.p;
+    L.sym_scratch_bytes = c->sym_scratch.bytes;
     L.stream = c->stream;
     launch_direct(L);
 }

@@ -616,8 +616,11 @@ SymPlan plan_for(int prec, int64_t n, bool umass, int sms) {
     return best;
 }
 
-size_t slot_bytes(int prec) {
-    return prec == RRG_PREC_FP32 ? sizeof(V4<float>) : sizeof(V4<double>);
+// js, is and js2 of a plan
+size_t slot_bytes(int prec, const SymPlan& pl) {
+    return (prec == RRG_PREC_FP32 ? sizeof(V4<float>) : sizeof(V4<double>)) *
+           (static_cast<size_t>(pl.n) * static_cast<size_t>(pl.tiles - 1 + pl.islots) +
+            static_cast<size_t>(pl.blocks) * kBS);
 }
 
 }  // namespace
@@ -627,15 +630,17 @@ size_t slot_bytes(int prec) {
 // 131,072 particles the slots stay below 600 MB.
 size_t direct_sym_scratch_bytes(int prec, int64_t n, bool umass, int sms) {
     if (!pair_plan_range(n)) return 0;
-    const SymPlan pl = plan_for(prec, n, umass, sms);
-    return slot_bytes(prec) * (static_cast<size_t>(n) * static_cast<size_t>(pl.tiles - 1 + pl.islots) +
-                               static_cast<size_t>(pl.blocks) * kBS);
+    return slot_bytes(prec, plan_for(prec, n, umass, sms));
 }
 
 void launch_direct_sym(const DirectLaunch& L, int sms) {
+    RRG_REQUIRE(pair_plan_range(L.n), RRG_ERR_INVALID,
+                "direct sum: too few or too many particles for pair slots");
     const bool umass = L.uniform_mass >= 0.0;
     const SymPlan pl = plan_for(L.prec, L.n, umass, sms);
     const size_t rows = static_cast<size_t>(pl.tiles - 1);
+    RRG_REQUIRE(L.sym_scratch_bytes >= slot_bytes(L.prec, pl), RRG_ERR_INVALID,
+                "direct sum: pair slots smaller than the schedule needs");
     RRG_REQUIRE(L.sym_scratch != nullptr && (reinterpret_cast<uintptr_t>(L.sym_scratch) & 31u) == 0,
                 RRG_ERR_INVALID, "direct sum: pair slots must start on a 32-byte boundary");
     const bool usoft = L.hsoft == nullptr;

@@ -43,6 +43,7 @@ struct DirectLaunch {
     void* scratch = nullptr;      // partial sums when splits > 1
     size_t scratch_bytes = 0;
     void* sym_scratch = nullptr;  // direct_sym_scratch_bytes of slots: each pair once (direct_sym.cu)
+    size_t sym_scratch_bytes = 0;
     cudaStream_t stream = nullptr;
 };
 

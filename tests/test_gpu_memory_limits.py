@@ -1,0 +1,84 @@
+"""What runs when the device's memory is nearly full: the pair slots of the direct sums and of the
+adjoint give way to the ordered kernels."""
+from contextlib import contextmanager
+
+import numpy as np
+import pytest
+
+import rrgsim_b200 as rg
+from helpers import plummer, rel_err
+from test_gpu_direct_sym import TOL_MAX, TOL_MEDIAN, _direct, _sample
+
+pytestmark = pytest.mark.gpu
+
+
+@contextmanager
+def memory_left(mb):
+    """All but about `mb` MB of the device's memory held by someone else."""
+    from cuda.bindings import runtime as cudart
+    ok = cudart.cudaError_t.cudaSuccess
+    held = []
+    try:
+        part = 1 << 62
+        while True:
+            part = min(part, cudart.cudaMemGetInfo()[1] - (mb << 20))
+            if part < 2 << 20:
+                break
+            err, p = cudart.cudaMalloc(part)
+            if err == ok:
+                held.append(p)
+            else:
+                cudart.cudaGetLastError()
+                part //= 2
+        yield
+    finally:
+        for p in held:
+            cudart.cudaFree(p)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+def test_direct_sum_without_room_for_pair_slots(prec):
+    n = 131072
+    pos, vel, m, s2 = plummer(n, seed=4)
+
+    def forces(c):
+        c.load_particles(pos, vel, m, s2)
+        c.nbody_acceleration()
+        return c.get_particles()["acc"]
+
+    with rg.Context(0, prec) as c:
+        pairs = forces(c)
+    with rg.Context(0, prec) as c:
+        # the ordered kernels once, one particle above the pair form's range
+        p, v, mm, ss = plummer(n + 1, seed=4)
+        c.load_particles(p, v, mm, ss)
+        c.nbody_acceleration()
+        c.get_particles()
+        with memory_left(100):
+            got = forces(c)
+    at = _sample(n)
+    err = rel_err(got[at], _direct(pos, m, s2, at)[0])
+    assert np.median(err) <= TOL_MEDIAN[prec] and np.max(err) <= TOL_MAX[prec]
+    assert not np.array_equal(got, pairs)  # the other form
+
+
+def test_adjoint_without_room_for_pair_slots():
+    """The ordered product's gradient against the pair form's: FP32 sums of at most 256 terms."""
+    torch = pytest.importorskip("torch")
+    from rrgsim_b200.adjoint import LeapfrogEngine, nbody_leapfrog
+    pos, vel, m, s2 = plummer(131072, seed=4)
+
+    def gradient(n):
+        t = lambda a: torch.tensor(a[:n], dtype=torch.float32, device="cuda")  # noqa: E731
+        x, v, mm = (t(a).requires_grad_(True) for a in (pos, vel, m))
+        engine = LeapfrogEngine(n, 1e-3, 2, 1e-4, "fp32", 2)
+        xn, _ = nbody_leapfrog(x, v, mm, 1e-4, 1e-3, 2, engine=engine)
+        return torch.autograd.grad(((xn - 1.0) ** 2).sum(1).mean(), (x, v, mm))
+
+    want = [g.cpu() for g in gradient(131072)]
+    gradient(6000)  # the ordered kernels once
+    with memory_left(160):
+        got = [g.cpu() for g in gradient(131072)]
+    assert not all(torch.equal(a, b) for a, b in zip(got, want))  # the other form
+    for a, b in zip(got, want):
+        assert float(torch.linalg.norm(a - b) / torch.linalg.norm(b)) <= 256 * 2.0 ** -24
