@@ -205,6 +205,12 @@ void require_particles(rrg_ctx* c) {
 void require_grid(rrg_ctx* c) {
     RRG_REQUIRE(c->has_grid, RRG_ERR_STATE, "no grid: call rrg_init_grid first");
 }
+// (a load or a grid that failed after rrg_solver_init leaves none)
+void require_solver(rrg_ctx* c) {
+    RRG_REQUIRE(c->solver_ready, RRG_ERR_STATE, "rrg_solver_init first");
+    require_particles(c);
+    if (c->wave_mode) require_grid(c);
+}
 
 size_t v4b(const rrg_ctx* c) { return 4 * c->rsz; }
 
@@ -648,17 +654,20 @@ void sort_particles(rrg_ctx* c) {
     require_grid(c);
     const int64_t n = c->n;
     const int64_t nc = static_cast<int64_t>(c->grid.nx) * c->grid.nx * c->grid.nx;
+    // (the buffer that is asked for its size last: it has it only when the others have theirs)
     if (c->sort_keys.bytes < 4 * static_cast<size_t>(n)) {
-        c->sort_keys.alloc(4 * n);
+        c->sort_keys.release();
         c->sort_dest.alloc(4 * n);
         c->sort_stage.alloc(v4b(c) * n);
+        c->sort_keys.alloc(4 * n);
     }
     if (c->sort_counts.bytes < 4 * static_cast<size_t>(nc + 1)) {
-        c->sort_counts.alloc(4 * (nc + 1));
+        c->sort_counts.release();
         c->sort_offsets.alloc(4 * (nc + 1));
         c->sort_cursor.alloc(4 * (nc + 1));
         c->sort_temp_bytes = sort_scan_temp_bytes(nc);
         c->sort_temp.alloc(std::max<size_t>(c->sort_temp_bytes, 256));
+        c->sort_counts.alloc(4 * (nc + 1));
     }
     if (!c->sorted) {
         c->id.alloc(4 * n);
@@ -1046,32 +1055,39 @@ RRG_API rrg_status rrg_load_particles(rrg_ctx* ctx, int64_t n, const double* pos
             ctx->shift_s = 26 - e;  // m_max 2^S <= 2^26: one contribution fits 27 bits
         }
         const size_t vb = v4b(ctx) * n;
-        ctx->posm[0].alloc(vb);
-        ctx->posm[1].alloc(vb);
-        if (ctx->prec == RRG_PREC_MIXED) {
-            ctx->poslo[0].alloc(sizeof(V4<float>) * n);
-            ctx->poslo[1].alloc(sizeof(V4<float>) * n);
-        } else {
-            ctx->poslo[0].release();
-            ctx->poslo[1].release();
+        try {
+            ctx->posm[0].alloc(vb);
+            ctx->posm[1].alloc(vb);
+            if (ctx->prec == RRG_PREC_MIXED) {
+                ctx->poslo[0].alloc(sizeof(V4<float>) * n);
+                ctx->poslo[1].alloc(sizeof(V4<float>) * n);
+            } else {
+                ctx->poslo[0].release();
+                ctx->poslo[1].release();
+            }
+            ctx->vel.alloc(vb);
+            ctx->acc.alloc(vb);
+            ctx->u.alloc(vb);
+            ctx->pot.alloc(ctx->rsz * n);
+            if (!uniform) ctx->hsoft.alloc(ctx->rsz * n);
+            else ctx->hsoft.release();
+            // the id buffer stays allocated (its contents are rewritten by the first sort); freeing
+            // and allocating it again on every reload cost the host two synchronous driver calls
+            ctx->steps_since_sort = INT64_MAX / 2;
+            ctx->splits = direct_choose_splits(ctx->prec, n, ctx->sms);
+            const size_t sb = direct_scratch_bytes(ctx->prec, n, ctx->splits);
+            if (sb) ctx->scratch.alloc(sb);
+            if (ctx->sym_scratch.p || (ctx->solver_ready && !ctx->wave_mode)) ensure_sym(ctx);
+            const int rb = conservation_blocks(n);
+            ctx->red_partial.alloc(static_cast<size_t>(rb) * 12 * 2 * sizeof(double));  // (hi, lo)
+            ctx->red_out.alloc(16 * sizeof(double));
+            alloc_step_partial(ctx);
+        } catch (...) {
+            // some buffers are gone, others have another size: no particles until the next load
+            ctx->n = 0;
+            drop_graphs(ctx);
+            throw;
         }
-        ctx->vel.alloc(vb);
-        ctx->acc.alloc(vb);
-        ctx->u.alloc(vb);
-        ctx->pot.alloc(ctx->rsz * n);
-        if (!uniform) ctx->hsoft.alloc(ctx->rsz * n);
-        else ctx->hsoft.release();
-        // the id buffer stays allocated (its contents are rewritten by the first sort); freeing
-        // and allocating it again on every reload cost the host two synchronous driver calls
-        ctx->steps_since_sort = INT64_MAX / 2;
-        ctx->splits = direct_choose_splits(ctx->prec, n, ctx->sms);
-        const size_t sb = direct_scratch_bytes(ctx->prec, n, ctx->splits);
-        if (sb) ctx->scratch.alloc(sb);
-        if (ctx->sym_scratch.p || (ctx->solver_ready && !ctx->wave_mode)) ensure_sym(ctx);
-        const int rb = conservation_blocks(n);
-        ctx->red_partial.alloc(static_cast<size_t>(rb) * 12 * 2 * sizeof(double));  // (hi, lo)
-        ctx->red_out.alloc(16 * sizeof(double));
-        alloc_step_partial(ctx);
         if (layout() != before || n != n_before || ctx->shift_s != shift_before ||
             ctx->uniform_hsoft != hsoft_before || ctx->soft_uniform != uniform_before ||
             ctx->uniform_mass != uniform_mass_before)
@@ -1138,7 +1154,8 @@ RRG_API rrg_status rrg_init_grid(rrg_ctx* ctx, const rrg_grid_info* grid) {
         ctx->gdev.inv_dx = 1.0 / grid->dx;
         ctx->gdev.sim_l = grid->sim_l;
         const size_t nc = static_cast<size_t>(grid->nx) * grid->nx * grid->nx;
-        {
+        ctx->has_grid = false;
+        try {
             // the two deposit grids and the two wave levels in one allocation, so that one L2
             // access-policy window covers them
             const auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
@@ -1149,12 +1166,16 @@ RRG_API rrg_status rrg_init_grid(rrg_ctx* ctx, const rrg_grid_info* grid) {
             ctx->mg[1].view(base + bm, nc * 8);
             ctx->phi[0].view(base + 2 * bm, nc * ctx->rsz);
             ctx->phi[1].view(base + 2 * bm + bp, nc * ctx->rsz);
+            ctx->acc4.alloc(nc * v4b(ctx));
+            ctx->src.alloc(nc * ctx->rsz);
+            apply_l2_window(ctx);
+            ctx->maxbits.alloc(kRelaxBytes);
+            ctx->wsync.alloc(wave_solve_sync_bytes(grid->nx));
+        } catch (...) {
+            clear_l2_window(ctx);  // no grid until the next call
+            drop_graphs(ctx);
+            throw;
         }
-        ctx->acc4.alloc(nc * v4b(ctx));
-        ctx->src.alloc(nc * ctx->rsz);
-        apply_l2_window(ctx);
-        ctx->maxbits.alloc(kRelaxBytes);
-        ctx->wsync.alloc(wave_solve_sync_bytes(grid->nx));
         for (Buf* b : {&ctx->mg[0], &ctx->mg[1], &ctx->src, &ctx->phi[0], &ctx->phi[1],
                        &ctx->acc4, &ctx->maxbits, &ctx->wsync})
             RRG_CUDA(cudaMemsetAsync(b->p, 0, b->bytes, ctx->stream));
@@ -1518,7 +1539,7 @@ RRG_API rrg_status rrg_solver_init(rrg_ctx* ctx, const rrg_sim_params* sim) {
 RRG_API rrg_status rrg_solver_precalc(rrg_ctx* ctx) {
     RRG_ENTRY(ctx, {
         drop_pending(ctx);
-        RRG_REQUIRE(ctx->solver_ready, RRG_ERR_STATE, "rrg_solver_init first");
+        require_solver(ctx);
         if (ctx->wave_mode) {
             deposit_operator(ctx);
             set_periodic(ctx, 1.0, 0);  // total mass fixed to 1: rrgsim_integration_rect.cuh:65
@@ -1541,7 +1562,7 @@ RRG_API rrg_status rrg_solver_precalc(rrg_ctx* ctx) {
 RRG_API rrg_status rrg_solver_resume(rrg_ctx* ctx) {
     RRG_ENTRY(ctx, {
         drop_pending(ctx);
-        RRG_REQUIRE(ctx->solver_ready, RRG_ERR_STATE, "rrg_solver_init first");
+        require_solver(ctx);
         if (ctx->wave_mode) {
             deposit_operator(ctx);
             set_periodic(ctx, 1.0, 0);  // as precalc: rrgsim_integration_rect.cuh:65
@@ -1601,7 +1622,7 @@ RRG_API rrg_status rrg_set_wave_state(rrg_ctx* ctx, const double* phi_cur,
 
 RRG_API rrg_status rrg_solver_calc_steps(rrg_ctx* ctx, int nsteps) {
     RRG_ENTRY(ctx, {
-        RRG_REQUIRE(ctx->solver_ready, RRG_ERR_STATE, "rrg_solver_init first");
+        require_solver(ctx);
         RRG_REQUIRE(nsteps >= 0, RRG_ERR_INVALID, "nsteps must be >= 0");
         if (nsteps > 0) {
             if (checks_inside_steps(ctx)) {
@@ -1630,7 +1651,7 @@ RRG_API rrg_status rrg_solver_calc_steps(rrg_ctx* ctx, int nsteps) {
 
 RRG_API rrg_status rrg_solver_prepare(rrg_ctx* ctx, int nsteps) {
     RRG_ENTRY(ctx, {
-        RRG_REQUIRE(ctx->solver_ready, RRG_ERR_STATE, "rrg_solver_init first");
+        require_solver(ctx);
         RRG_REQUIRE(nsteps >= 0, RRG_ERR_INVALID, "nsteps must be >= 0");
         if (nsteps > 0 && !checks_inside_steps(ctx)) {
             // walk the chunks of that call, recording what is missing, then put the roles back
@@ -1657,7 +1678,7 @@ RRG_API rrg_status rrg_solver_prepare(rrg_ctx* ctx, int nsteps) {
 
 RRG_API rrg_status rrg_solver_sync(rrg_ctx* ctx) {
     RRG_ENTRY(ctx, {
-        RRG_REQUIRE(ctx->solver_ready, RRG_ERR_STATE, "rrg_solver_init first");
+        require_solver(ctx);
         if (ctx->wave_mode) {
             launch_ngp_phi(ctx->prec, ctx->n, ctx->P(), ctx->L(), ctx->gdev,
                            ctx->phi[ctx->phi_cur].p, ctx->pot.p, ctx->stream);
@@ -1698,7 +1719,12 @@ RRG_API rrg_status rrg_set_sort_interval(rrg_ctx* ctx, int interval) {
 RRG_API rrg_status rrg_set_step_sums(rrg_ctx* ctx, int enable) {
     RRG_ENTRY(ctx, {
         ctx->step_sums = enable != 0;
-        alloc_step_partial(ctx);
+        try {
+            alloc_step_partial(ctx);
+        } catch (...) {
+            ctx->step_sums = false;
+            throw;
+        }
     })
 }
 

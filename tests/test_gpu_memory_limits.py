@@ -1,12 +1,13 @@
 """What runs when the device's memory is nearly full: the pair slots of the direct sums and of the
-adjoint give way to the ordered kernels."""
+adjoint give way to the ordered kernels, and a load or a grid that does not fit leaves a context that
+says so instead of one that runs on what is left of it."""
 from contextlib import contextmanager
 
 import numpy as np
 import pytest
 
 import rrgsim_b200 as rg
-from helpers import plummer, rel_err
+from helpers import disk, plummer, rel_err
 from test_gpu_direct_sym import TOL_MAX, TOL_MEDIAN, _direct, _sample
 
 pytestmark = pytest.mark.gpu
@@ -82,3 +83,69 @@ def test_adjoint_without_room_for_pair_slots():
     assert not all(torch.equal(a, b) for a, b in zip(got, want))  # the other form
     for a, b in zip(got, want):
         assert float(torch.linalg.norm(a - b) / torch.linalg.norm(b)) <= 256 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("wave", [0, 1])
+def test_a_load_that_does_not_fit_leaves_no_particles(wave):
+    sim = rg.SimParams(time_max=1.0, dt_save=0.1, dt_dynamics=1e-3, saves_without_dump=0,
+                       use_wave_model=wave)
+    small, big = disk(2000, seed=1), disk(1 << 20, seed=2)
+    with rg.Context(0, "fp32") as c:
+        c.load_particles(*big)
+        c.get_particles()  # (the staging buffer has its size)
+        c.load_particles(*small)
+        g = rg.GridInfo.from_values(32, 0.5, 0.0)
+        c.init_grid(g)
+        c.set_wave_params(rg.WaveParams.make(g.dx, diss_base=0.5, wave_speed=8.0, iterations=4,
+                                             setup_iterations=4))
+        c.solver_init(sim)
+        c.precalc()
+        c.calc_steps(2)
+        want = c.get_particles()
+        with memory_left(50):
+            with pytest.raises(rg.RRGError):
+                c.load_particles(*big)
+            for call in (lambda: c.calc_steps(2), lambda: c.prepare_steps(2), c.precalc, c.resume,
+                         c.sync_particles_and_grid, c.nbody_acceleration, c.get_particles):
+                with pytest.raises(rg.RRGError):
+                    call()
+        c.load_particles(*small)
+        c.init_grid(g)
+        c.precalc()
+        c.calc_steps(2)
+        got = c.get_particles()
+    for k in ("pos", "vel"):
+        np.testing.assert_array_equal(got[k], want[k])
+
+
+def test_a_grid_that_does_not_fit_leaves_no_grid():
+    sim = rg.SimParams(time_max=1.0, dt_save=0.1, dt_dynamics=1e-3, saves_without_dump=0,
+                       use_wave_model=1)
+    small, large = (rg.GridInfo.from_values(nx, 16.0 / nx, 0.0) for nx in (32, 192))
+    with rg.Context(0, "fp32") as c:
+        c.load_particles(*disk(2000, seed=1))
+
+        def steps():
+            c.init_grid(small)
+            c.precalc()
+            c.calc_steps(2)
+            return c.get_particles()["pos"]
+
+        c.init_grid(small)
+        c.set_wave_params(rg.WaveParams.make(small.dx, diss_base=0.5, wave_speed=8.0, iterations=4,
+                                             setup_iterations=4))
+        c.solver_init(sim)
+        c.precalc()
+        c.calc_steps(2)
+        with memory_left(50):
+            with pytest.raises(rg.RRGError):
+                c.init_grid(large)
+            for call in (lambda: c.calc_steps(2), lambda: c.prepare_steps(2), c.precalc, c.resume,
+                         c.sync_particles_and_grid, c.convert_particles_to_grid,
+                         c.calc_acceleration_field):
+                with pytest.raises(rg.RRGError):
+                    call()
+        c.load_particles(*disk(2000, seed=1))
+        a = steps()
+        c.load_particles(*disk(2000, seed=1))
+        np.testing.assert_array_equal(a, steps())
