@@ -539,8 +539,15 @@ void build_worklist(rrg_ensemble* e, int variant, int jchunk) {
     drop_ens_graphs(e);
 }
 
-// The schedule of the kernels that evaluate each pair once, with g i-particles per thread.
-void build_pairs(rrg_ensemble* e, int variant) {
+// The largest pair slots that the autotuner lets an ensemble hold: n^2 / 64 bytes for a galaxy of n
+// particles with 4 i per thread and n^2 / 128 with 8, kept as long as the ensemble. The ordered
+// forms' partials are n^2 / 512 bytes at 8,192 particles a chunk. 64 galaxies of up to 65,536 particles
+// take 0.6 GB; one galaxy beyond 524,000 (4 i) or 741,000 (8 i) runs in an ordered form.
+constexpr size_t kMaxPairSlots = size_t(4) << 30;
+
+// The schedule of the kernels that evaluate each pair once, with g i-particles per thread. False,
+// changing nothing, where its slots are beyond kMaxPairSlots.
+bool build_pairs(rrg_ensemble* e, int variant) {
     const int g = variant == 4 ? 8 : 4;
     EnsPairParams p{};
     p.ngal = e->ngal;
@@ -572,8 +579,11 @@ void build_pairs(rrg_ensemble* e, int variant) {
         y.slots = records;
         records += static_cast<int64_t>(y.tiles - 1 + islots) * y.n;
     }
+    const size_t slots = sizeof(V4<float>) *
+                         static_cast<size_t>(records + static_cast<int64_t>(p.blocks) * kBS);
+    if (slots > kMaxPairSlots) return false;
     e->pair_gal.alloc(sizeof(EnsPairGalaxy) * gal.size());
-    e->part.alloc(sizeof(V4<float>) * static_cast<size_t>(records + static_cast<int64_t>(p.blocks) * kBS));
+    e->part.alloc(slots);
     RRG_CUDA(cudaMemcpy(e->pair_gal.p, gal.data(), sizeof(EnsPairGalaxy) * gal.size(),
                         cudaMemcpyHostToDevice));
     p.gal = e->pair_gal.as<EnsPairGalaxy>();
@@ -584,6 +594,7 @@ void build_pairs(rrg_ensemble* e, int variant) {
     e->jchunk = kBS;
     e->num_items = p.blocks;
     drop_ens_graphs(e);
+    return true;
 }
 
 void launch_forces(rrg_ensemble* e, const void* posm) {
@@ -688,25 +699,34 @@ void run_steps(rrg_ensemble* e, int nsteps) {
 }
 
 // Times one force evaluation per candidate (the pair forms, tile variants and j-chunks) and keeps the
-// fastest. An ordered variant is sampled at two j-chunks, and at the others only where one of the two
+// fastest; one whose slots or partials the device has no room for, or beyond kMaxPairSlots, is left
+// out. An ordered variant is sampled at two j-chunks, and at the others only where one of the two
 // comes within 15 % of the best: creating an ensemble of 8 galaxies 11.7 -> 8.3 ms, 24 galaxies of up to
 // 16,384 particles 44 -> 31.
 void autotune(rrg_ensemble* e) {
-    cudaEvent_t a, b;
-    RRG_CUDA(cudaEventCreate(&a));
-    RRG_CUDA(cudaEventCreate(&b));
-    float best = 1e30f;
-    int bv = 1, bj = 4096;
+    struct Event {
+        cudaEvent_t p = nullptr;
+        Event() { RRG_CUDA(cudaEventCreate(&p)); }
+        ~Event() { cudaEventDestroy(p); }
+    } a, b;
+    constexpr float none = 1e30f;
+    float best = none;
+    int bv = 0, bj = 0;
     auto consider = [&](int v, int j) {
-        if (v >= 3) build_pairs(e, v);
-        else build_worklist(e, v, j);
+        try {
+            if (v < 3) build_worklist(e, v, j);
+            else if (!build_pairs(e, v)) return none;
+        } catch (const Error& x) {
+            if (x.code != RRG_ERR_NOMEM) throw;
+            return none;
+        }
         launch_forces(e, e->posm[e->cur].p);  // warm
-        RRG_CUDA(cudaEventRecord(a, e->stream));
+        RRG_CUDA(cudaEventRecord(a.p, e->stream));
         for (int r = 0; r < 2; ++r) launch_forces(e, e->posm[e->cur].p);
-        RRG_CUDA(cudaEventRecord(b, e->stream));
-        RRG_CUDA(cudaEventSynchronize(b));
+        RRG_CUDA(cudaEventRecord(b.p, e->stream));
+        RRG_CUDA(cudaEventSynchronize(b.p));
         float ms = 0.f;
-        RRG_CUDA(cudaEventElapsedTime(&ms, a, b));
+        RRG_CUDA(cudaEventElapsedTime(&ms, a.p, b.p));
         if (ms < best) {
             best = ms;
             bv = v;
@@ -720,8 +740,8 @@ void autotune(rrg_ensemble* e) {
         if (two <= 1.15f * best)
             for (int j : {1024, 4096, 16384}) consider(v, j);
     }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
+    RRG_REQUIRE(bv != 0, RRG_ERR_NOMEM,
+                "rrg_ensemble_create: no room for the partial sums of any force form");
     if (bv >= 3) build_pairs(e, bv);
     else build_worklist(e, bv, bj);
     e->tuned_ms = best / 2;

@@ -39,3 +39,18 @@ def test_every_form_of_the_forces_matches_the_oracle(ngal, nmin, nmax, masses):
         else:
             assert np.median(rel_err(a, ref)) <= 1e-5
         at += n
+
+
+def test_a_galaxy_beyond_the_pair_slots_bound():
+    """One galaxy whose pair slots would take more than 4 GiB in either pair form runs in an ordered
+    form."""
+    n = 786_437
+    P, V = rg.generate_plummer(1, n, 1.0, 1.0, 20.0)
+    with rg.Ensemble([n], P, V, np.full(n, 1.0 / n), [1e-4], 1e-3) as e:
+        assert e.tuning()["variant"] in (1, 2)
+        got = e.get()
+    for i in (0, 255, n - 1):
+        d = got["pos"] - got["pos"][i]
+        r = ((d * d).sum(1) + 1e-4) ** -1.5
+        want = (r[:, None] * d).sum(0) / n
+        assert np.linalg.norm(got["acc"][i] - want) <= 1e-3 * np.linalg.norm(want)

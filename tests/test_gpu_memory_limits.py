@@ -1,6 +1,6 @@
-"""What runs when the device's memory is nearly full: the pair slots of the direct sums and of the
-adjoint give way to the ordered kernels, and a load or a grid that does not fit leaves a context that
-says so instead of one that runs on what is left of it."""
+"""What runs when the device's memory is nearly full: the pair slots of the direct sums, the adjoint
+and the ensemble give way to the ordered kernels, and a load or a grid that does not fit leaves a
+context that says so instead of one that runs on what is left of it."""
 from contextlib import contextmanager
 
 import numpy as np
@@ -83,6 +83,24 @@ def test_adjoint_without_room_for_pair_slots():
     assert not all(torch.equal(a, b) for a, b in zip(got, want))  # the other form
     for a, b in zip(got, want):
         assert float(torch.linalg.norm(a - b) / torch.linalg.norm(b)) <= 256 * 2.0 ** -24
+
+
+def test_ensemble_without_room_for_pair_slots():
+    n = 131072
+    pos, vel, m, s2 = plummer(n, seed=4)
+
+    def create():
+        return rg.Ensemble([n], pos, vel, m, s2[:1], 1e-3)
+
+    with create() as e:
+        e.get()
+    with memory_left(100):
+        with create() as e:
+            tuned, got = e.tuning(), e.get()["acc"]
+    assert tuned["variant"] in (1, 2) and tuned["jchunk"] >= 8192
+    at = _sample(n)
+    err = rel_err(got[at], _direct(pos, m, s2, at)[0])
+    assert np.median(err) <= 1e-5 and np.max(err) <= 1e-3
 
 
 @pytest.mark.parametrize("wave", [0, 1])
