@@ -16,6 +16,7 @@
 // Bound: the FP32 pipe.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <string>
 #include <vector>
 
@@ -734,8 +735,13 @@ void autotune(rrg_ensemble* e) {
         }
         return ms;
     };
-    for (int v : {3, 4}) consider(v, 1024);  // (no j-chunk)
+    const char* fixed = std::getenv("RRG_ENSEMBLE_FORM");  // 1 to 4: this form alone
+    const int form = fixed ? std::atoi(fixed) : 0;
+    const bool any = form < 1 || form > 4;
+    for (int v : {3, 4})
+        if (any || v == form) consider(v, 1024);  // (no j-chunk)
     for (int v : {1, 2}) {
+        if (!any && v != form) continue;
         const float two = std::min(consider(v, 2048), consider(v, 8192));
         if (two <= 1.15f * best)
             for (int j : {1024, 4096, 16384}) consider(v, j);

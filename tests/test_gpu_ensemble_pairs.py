@@ -41,6 +41,50 @@ def test_every_form_of_the_forces_matches_the_oracle(ngal, nmin, nmax, masses):
         at += n
 
 
+@pytest.fixture(scope="module")
+def galaxies():
+    """Twelve galaxies of 700 to 16,000 particles in no order of size: far more units than blocks
+    in every form, so that runs start inside units and cross i-tiles and galaxies. The reference
+    accelerations of both mass forms, of the FP32 positions, masses and softenings."""
+    rng = np.random.default_rng(5)
+    counts = rng.permutation(np.geomspace(700, 16000, 12).astype(np.int64))
+    P, V = (np.vstack(a) for a in zip(*(rg.generate_plummer(k + 1, int(n), 1.0, 1.0, 20.0)
+                                        for k, n in enumerate(counts))))
+    s2 = (0.01 * (1 + np.arange(12) % 3)) ** 2
+    spread = rng.uniform(0.5, 1.5, len(P))
+    spread[7::101] = 0.0
+    masses = {"equal": 1.0 / np.repeat(counts, counts)}
+    masses["spread"] = masses["equal"] * spread
+    at = np.concatenate([[0], np.cumsum(counts)])
+    p32 = P.astype(np.float32).astype(np.float64)
+    ref = {k: np.vstack([orc.direct_acc(p32[a:b], m[a:b], np.full(b - a, s2[g]))
+                         for g, (a, b) in enumerate(zip(at, at[1:]))]) for k, m in masses.items()}
+    return counts, P, V, masses, s2, ref
+
+
+@pytest.mark.parametrize("form", [1, 2, 3, 4])
+@pytest.mark.parametrize("masses", ["equal", "spread"])
+def test_each_form_with_runs_across_tiles_and_galaxies(monkeypatch, galaxies, masses, form):
+    """Every particle's acceleration in each form, bars of the direct sums (median 1e-5, maximum
+    1e-3), and the same bits from another ensemble, at creation and after steps (the ordered forms
+    where both settled on one j-chunk)."""
+    counts, P, V, m, s2, ref = galaxies
+    monkeypatch.setenv("RRG_ENSEMBLE_FORM", str(form))
+    got = []
+    for _ in range(2):
+        with rg.Ensemble(counts, P, V, m[masses], s2, 1e-3) as e:
+            tuned = e.tuning()
+            assert tuned["variant"] == form
+            first = e.get()
+            e.step(3)
+            got.append((first, e.get(), tuned["jchunk"]))
+    err = rel_err(got[0][0]["acc"], ref[masses])
+    assert np.median(err) <= 1e-5 and np.max(err) <= 1e-3, (np.median(err), np.max(err))
+    for a, b in zip(got[0][:2], got[1][:2]) if got[0][2] == got[1][2] else ():
+        for k in ("pos", "vel", "acc"):
+            np.testing.assert_array_equal(a[k], b[k])
+
+
 def test_a_galaxy_beyond_the_pair_slots_bound():
     """One galaxy whose pair slots would take more than 4 GiB in either pair form runs in an ordered
     form."""
