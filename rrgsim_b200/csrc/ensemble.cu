@@ -908,18 +908,24 @@ RRG_API rrg_status rrg_ensemble_step_sequential(rrg_ensemble* e, int nsteps, int
 RRG_API rrg_status rrg_ensemble_get(rrg_ensemble* e, double* pos, double* vel, double* acc) {
     ENS_ENTRY(e, {
         // widened on the device, straight into the caller's arrays (131,000 particles: converting
-        // in host loops from three staging vectors took 5.7 ms)
-        const size_t each = 3 * static_cast<size_t>(e->ntot);
-        if (e->widened.bytes < 3 * each * sizeof(double)) e->widened.alloc(3 * each * sizeof(double));
+        // in host loops from three staging vectors took 5.7 ms), 2^20 particles at a time: 75 MB
+        // of staging at most
+        const int64_t piece = std::min<int64_t>(e->ntot, int64_t(1) << 20);
+        const size_t each = 3 * static_cast<size_t>(piece);
+        if (!e->widened.p) e->widened.alloc(3 * each * sizeof(double));
         double* d = e->widened.as<double>();
-        launch_unpack_state(RRG_PREC_FP32, e->ntot, nullptr, e->posm[e->cur].p, nullptr, e->vel.p,
-                            e->acc.p, nullptr, pos ? d : nullptr, vel ? d + each : nullptr,
-                            acc ? d + 2 * each : nullptr, nullptr, e->stream);
         double* const out[3] = {pos, vel, acc};
-        for (int k = 0; k < 3; ++k)
-            if (out[k])
-                RRG_CUDA(cudaMemcpyAsync(out[k], d + k * each, each * sizeof(double),
-                                         cudaMemcpyDeviceToHost, e->stream));
+        for (int64_t i = 0; i < e->ntot; i += piece) {
+            const int64_t n = std::min(piece, e->ntot - i);
+            launch_unpack_state(RRG_PREC_FP32, n, nullptr, e->posm[e->cur].as<V4<float>>() + i,
+                                nullptr, e->vel.as<V4<float>>() + i, e->acc.as<V4<float>>() + i,
+                                nullptr, pos ? d : nullptr, vel ? d + each : nullptr,
+                                acc ? d + 2 * each : nullptr, nullptr, e->stream);
+            for (int k = 0; k < 3; ++k)
+                if (out[k])
+                    RRG_CUDA(cudaMemcpyAsync(out[k] + 3 * i, d + k * each, 3 * n * sizeof(double),
+                                             cudaMemcpyDeviceToHost, e->stream));
+        }
         RRG_CUDA(cudaStreamSynchronize(e->stream));
     })
 }

@@ -85,6 +85,27 @@ def test_each_form_with_runs_across_tiles_and_galaxies(monkeypatch, galaxies, ma
             np.testing.assert_array_equal(a[k], b[k])
 
 
+def test_download_of_many_galaxies_stages_a_bounded_piece():
+    """3.1 million particles in galaxies of about 1,000: the download keeps at most 80 MB on the
+    device, and every particle comes back in its place."""
+    pytest.importorskip("torch")
+    from cuda.bindings import runtime as cudart
+    counts = np.where(np.arange(3072) % 2 == 0, 1021, 1030).astype(np.int64)
+    n = int(counts.sum())
+    rng = np.random.default_rng(2)
+    P, V = rng.standard_normal((n, 3)), rng.standard_normal((n, 3))
+    with rg.Ensemble(counts, P, V, np.full(n, 1e-6), np.full(3072, 1e-4), 1e-3,
+                     autotune=False) as e:
+        free = cudart.cudaMemGetInfo()[1]
+        got = e.get()
+        assert free - cudart.cudaMemGetInfo()[1] <= 80 << 20
+    np.testing.assert_array_equal(got["pos"], P.astype(np.float32))
+    np.testing.assert_array_equal(got["vel"], V.astype(np.float32))
+    last = slice(n - 1030, n)
+    ref = orc.direct_acc(got["pos"][last], np.full(1030, 1e-6), np.full(1030, 1e-4))
+    assert np.median(rel_err(got["acc"][last], ref)) <= 1e-5
+
+
 def test_a_galaxy_beyond_the_pair_slots_bound():
     """One galaxy whose pair slots would take more than 4 GiB in either pair form runs in an ordered
     form."""
