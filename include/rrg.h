@@ -164,8 +164,8 @@ RRG_API rrg_status rrg_destroy(rrg_ctx* ctx);
  * Once an FP32 or MIXED context has a grid of 32, 64 or 128 cells, the stream it launches on
  * carries a persisting L2 access-policy window over the context's deposit grids and wave levels
  * (48 MB at 128^3), and the process's persisting L2 set-aside is sized to the largest such
- * window, and never below the host's own: every PM step reads and rewrites those grids, and keeping them in L2 shortens the step
- * by ~3%. (Other grids have none: their substeps use L2 themselves.) The window moves with the
+ * window, and never below the host's own: every PM step reads and rewrites those grids, and keeping
+ * them in L2 shortens the step by ~3%. (Other grids have none: their substeps use L2 themselves.) The window moves with the
  * context to a new stream, and rrg_destroy takes it off a caller's stream and gives its share
  * of the set-aside back: with the last window the size that the host had set before stands again
  * (0: the persisting lines are dropped too). Environment RRG_L2_PERSIST=0 leaves L2 alone. */

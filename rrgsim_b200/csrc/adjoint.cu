@@ -821,18 +821,8 @@ struct VjpChunks {
     int splits;
 };
 VjpChunks vjp_f32x2_chunks(int64_t n, int sms) {
-    static int resident = 0;
-    if (!resident) {
-        int nb = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                &nb, reinterpret_cast<const void*>(&vjp_f32x2_kernel<true, true, true, false>), kBS, 0) !=
-                cudaSuccess ||
-            nb < 1) {
-            (void)cudaGetLastError();
-            nb = 1;
-        }
-        resident = nb;
-    }
+    const int resident = resident_blocks_per_sm(
+        reinterpret_cast<const void*>(&vjp_f32x2_kernel<true, true, true, false>), kBS, 0);
     const int64_t kblocks = (n + 2 * kBS - 1) / (2 * kBS);
     const int64_t tiles = (n + kBS - 1) / kBS;
     const int64_t slots = static_cast<int64_t>(sms) * resident;
@@ -1074,10 +1064,7 @@ int vjp_pair_blocks(int sms, bool umass) {
 }
 
 SymPlan vjp_pair_plan(int64_t n, int sms, bool umass) {
-    static int cache[2] = {};
-    int& blocks = cache[umass];
-    if (!blocks) blocks = vjp_pair_blocks(sms, umass);
-    return make_pair_plan(n, 4, blocks);
+    return make_pair_plan(n, 4, vjp_pair_blocks(sms, umass));
 }
 
 // V4 records of one slot array (js, is and js2 together)

@@ -13,6 +13,9 @@
 // reduced in FP64 in a fixed order by a second kernel (deterministic).
 #include <algorithm>
 #include <cstdlib>
+#include <map>
+#include <mutex>
+#include <tuple>
 
 #include "direct_epi.cuh"
 #include "kernels.cuh"
@@ -604,11 +607,8 @@ int ipt_of(int variant) {
 
 int ipt_for(int prec, int64_t n) { return ipt_of(variant_for(prec, n)); }
 
-// Resident 256-thread blocks per SM of the kernel a variant launches (queried once).
+// Resident 256-thread blocks per SM of the kernel a variant launches.
 int resident_blocks(int prec, int variant) {
-    static int cache[3][8] = {};
-    int& r = cache[prec][variant];
-    if (r) return r;
     const void* k = nullptr;
     if (prec == RRG_PREC_FP64) k = reinterpret_cast<const void*>(&direct_f64_kernel<true, false>);
     else if (prec == RRG_PREC_MIXED)
@@ -621,13 +621,7 @@ int resident_blocks(int prec, int variant) {
     else if (variant == 5) k = reinterpret_cast<const void*>(&direct_f32x2_kernel<3, true, false, false>);
     else if (variant == 6) k = reinterpret_cast<const void*>(&direct_f32jp_kernel<1, true, false, false>);
     else k = reinterpret_cast<const void*>(&direct_f32jp_kernel<2, true, false, false>);
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, kBS, 0) != cudaSuccess || nb < 1) {
-        (void)cudaGetLastError();
-        nb = 1;
-    }
-    r = nb;
-    return r;
+    return resident_blocks_per_sm(k, kBS, 0);
 }
 
 }  // namespace
@@ -637,6 +631,25 @@ int resident_blocks(int prec, int variant) {
 // extra split only adds n x 16 B of partials and a tiny reduction). The count is a request:
 // the launch rounds it to whole j-tile chunks, and on B200 that measured faster at N = 16,384
 // than choosing among realisable counts only.
+int resident_blocks_per_sm(const void* kernel, int threads, size_t smem) {
+    static std::mutex mu;
+    static std::map<std::tuple<int, const void*, int, size_t>, int> known;
+    int dev = 0;
+    RRG_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    int& nb = known[{dev, kernel, threads, smem}];
+    if (nb > 0) return nb;
+    if (smem > 48 * 1024)
+        RRG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(smem)));
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem) != cudaSuccess ||
+        nb < 1) {
+        (void)cudaGetLastError();
+        nb = 1;
+    }
+    return nb;
+}
+
 int direct_choose_splits(int prec, int64_t n, int sms) {
     const int variant = variant_for(prec, n);
     const int ipt = ipt_of(variant);

@@ -564,26 +564,20 @@ void dispatch64(bool usoft, bool pot, const SymParams<double, double>& p, cudaSt
 #undef RRG_SYM
 }
 
-// Blocks per SM of the kernels of (prec, g), queried once (the force kernel without potential;
-// the one with it has as many or leaves the runs a little longer).
+// Blocks per SM of the kernels of (prec, g) (the force kernel without potential; the one with it
+// has as many or leaves the runs a little longer).
 int resident_blocks(int prec, int g) {
-    static int cache[3][9] = {};
-    int& r = cache[prec][g];
-    if (r) return r;
-    int v = 1;
     if (prec == RRG_PREC_FP64) {
-        if (g == 2) v = pair_blocks_per_sm(direct_sym64_kernel<2, true, false>, Sym64<2, true, false>::smem);
-        else v = pair_blocks_per_sm(direct_sym64_kernel<4, true, false>, Sym64<4, true, false>::smem);
-    } else if (prec == RRG_PREC_MIXED) {
-        if (g == 2) v = pair_blocks_per_sm(direct_sym32_kernel<1, true, false, false, true>, Sym32<1, true, false, false, true>::smem);
-        else v = pair_blocks_per_sm(direct_sym32_kernel<2, true, false, false, true>, Sym32<2, true, false, false, true>::smem);
-    } else {
-        if (g == 2) v = pair_blocks_per_sm(direct_sym32_kernel<1, true, false, true, false>, Sym32<1, true, false, true, false>::smem);
-        else if (g == 4) v = pair_blocks_per_sm(direct_sym32_kernel<2, true, false, true, false>, Sym32<2, true, false, true, false>::smem);
-        else v = pair_blocks_per_sm(direct_sym32_kernel<4, true, false, true, false>, Sym32<4, true, false, true, false>::smem);
+        if (g == 2) return pair_blocks_per_sm(direct_sym64_kernel<2, true, false>, Sym64<2, true, false>::smem);
+        return pair_blocks_per_sm(direct_sym64_kernel<4, true, false>, Sym64<4, true, false>::smem);
     }
-    r = v;
-    return r;
+    if (prec == RRG_PREC_MIXED) {
+        if (g == 2) return pair_blocks_per_sm(direct_sym32_kernel<1, true, false, false, true>, Sym32<1, true, false, false, true>::smem);
+        return pair_blocks_per_sm(direct_sym32_kernel<2, true, false, false, true>, Sym32<2, true, false, false, true>::smem);
+    }
+    if (g == 2) return pair_blocks_per_sm(direct_sym32_kernel<1, true, false, true, false>, Sym32<1, true, false, true, false>::smem);
+    if (g == 4) return pair_blocks_per_sm(direct_sym32_kernel<2, true, false, true, false>, Sym32<2, true, false, true, false>::smem);
+    return pair_blocks_per_sm(direct_sym32_kernel<4, true, false, true, false>, Sym32<4, true, false, true, false>::smem);
 }
 
 // i-particles per thread: the more, the fewer shuffles and tile reads a pair costs, but the fewer

@@ -47,6 +47,9 @@ struct DirectLaunch {
     cudaStream_t stream = nullptr;
 };
 
+// Resident blocks of `threads` per SM of a kernel on the current device, at least 1: queried once per
+// device, kernel and shape (several threads may ask).
+int resident_blocks_per_sm(const void* kernel, int threads, size_t smem);
 int direct_choose_splits(int prec, int64_t n, int sms);
 size_t direct_scratch_bytes(int prec, int64_t n, int splits);
 void launch_direct(const DirectLaunch& L);

@@ -57,12 +57,7 @@ __device__ __forceinline__ float half_sum(float2 v) { return __fadd_rn(v.x, v.y)
 // resident blocks of kDirectThreads per SM with `smem` bytes of dynamic shared memory
 template <typename Kern>
 int pair_blocks_per_sm(Kern k, size_t smem) {
-    if (smem > 48 * 1024)
-        RRG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(smem)));
-    int nb = 0;
-    RRG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, kDirectThreads, smem));
-    return std::max(nb, 1);
+    return resident_blocks_per_sm(reinterpret_cast<const void*>(k), kDirectThreads, smem);
 }
 
 // From 32 j-tiles to 131,072 particles (the sizes at which the schedule fills the SMs and its slots

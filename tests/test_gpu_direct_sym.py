@@ -119,3 +119,22 @@ def test_first_evaluation_under_capture(prec):
         again = c.get_particles()["acc"]
     np.testing.assert_array_equal(got, want)
     np.testing.assert_array_equal(again, want)
+
+
+def test_threads_with_contexts_of_their_own():
+    """Eight threads that create contexts and evaluate at once get the bits of one after the other."""
+    from concurrent.futures import ThreadPoolExecutor
+    cases = [(prec, n) for prec in ("fp32", "mixed", "fp64") for n in (8001, 9000, 12287, 16001)]
+
+    def acc(case):
+        prec, n = case
+        pos, vel, m, s2 = _case(n, "m" if n % 2 else "")
+        with rg.Context(0, prec) as c:
+            c.load_particles(pos, vel, m, s2)
+            c.nbody_acceleration()
+            return c.get_particles()["acc"]
+
+    with ThreadPoolExecutor(8) as pool:
+        got = list(pool.map(acc, cases))
+    for case, g in zip(cases, got):
+        np.testing.assert_array_equal(g, acc(case))
