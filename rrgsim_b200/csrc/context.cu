@@ -595,7 +595,7 @@ int solve_wave(rrg_ctx* c, int max_iterations, double* last_rel) {
         // MIXED grids of 32, 64 or 128 cells) and its start (the levels and the source into the
         // SMs and back, ~10 us) is paid
         if (left >= 8 && c->prec != RRG_PREC_FP64 && c->bc_type == RRG_BC_PERIODIC &&
-            !c->keep_layer) {
+            !c->keep_layer && wave_relax_applicable(c->grid.nx)) {
             auto* checks = c->maxbits.as<RelaxCheck>();
             auto* result = reinterpret_cast<RelaxResult*>(checks + kRelaxChecks);
             const RelaxControl control{check ? static_cast<int>(next) - it : left,

@@ -290,6 +290,9 @@ struct RelaxControl {
     int first, every, hold, hold_steps;
     double tolerance;
 };
+// wave_relax_applicable: false where launch_wave_relax does not apply whatever its other arguments
+// (the caller then has nothing to zero).
+bool wave_relax_applicable(int nx);
 bool launch_wave_relax(int nx, int iterations, float* phi0, float* phi1, int cur,
                        const float* src, const WaveCoef& w, const RelaxControl& control,
                        RelaxCheck* checks, RelaxResult* result, unsigned int* sync,

@@ -1066,11 +1066,15 @@ bool launch_wave_solve(int nx, int iterations, float* phi0, float* phi1, int cur
     return launch_persistent(nx, false, nx == 128 && use_tb(), a, sync_bytes, s);
 }
 
+bool wave_relax_applicable(int nx) {
+    return wave_solve_applicable(nx) && !(nx == 128 && use_tb());
+}
+
 bool launch_wave_relax(int nx, int iterations, float* phi0, float* phi1, int cur,
                        const float* src, const WaveCoef& w, const RelaxControl& control,
                        RelaxCheck* checks, RelaxResult* result, unsigned int* sync,
                        size_t sync_bytes, cudaStream_t s) {
-    if (!wave_solve_applicable(nx) || iterations < 1 || (nx == 128 && use_tb())) return false;
+    if (!wave_relax_applicable(nx) || iterations < 1) return false;
     SolveArgs a{};
     a.phi0 = phi0;
     a.phi1 = phi1;

@@ -47,3 +47,39 @@ def test_relaxation_equals_one_launch_per_substep(monkeypatch, prec, nx, every, 
         np.testing.assert_array_equal(prev1, prev0)
     if tol > 0:
         assert out[0][0][0] < runs[0]  # it stopped on the steady check
+
+
+@pytest.mark.parametrize("prec,nx,kernels", [("fp32", 40, 11), ("fp64", 64, 11), ("fp32", 64, 2)])
+def test_relaxation_without_a_check_adds_nothing_to_its_substeps(prec, nx, kernels):
+    """A relaxation of ten substeps under capture: the source and one launch per substep (or the
+    persistent one), and a cleared buffer only where the persistent kernel reads it."""
+    torch = pytest.importorskip("torch")
+    from cuda.bindings import runtime as cudart
+    ok = cudart.cudaError_t.cudaSuccess
+    pos, vel, m, s2 = disk(2000, seed=nx)
+    g = rg.GridInfo.from_values(nx, 16.0 / nx, 0.2)
+    s = torch.cuda.Stream()
+    with rg.Context(0, prec) as c:
+        c.load_particles(pos, vel, m, s2)
+        c.init_grid(g)
+        c.set_wave_params(rg.WaveParams.make(g.dx, diss_base=1.0 / (4 * g.dx), wave_speed=8.0))
+        c.convert_particles_to_grid()
+        c.set_boundary_periodic(1.0)
+        c.synchronize()
+        c.set_stream(s.cuda_stream)
+        err, = cudart.cudaStreamBeginCapture(
+            s.cuda_stream, cudart.cudaStreamCaptureMode.cudaStreamCaptureModeRelaxed)
+        assert err == ok
+        try:
+            c.solve_wave_equation(10)
+        finally:
+            err, graph = cudart.cudaStreamEndCapture(s.cuda_stream)
+        assert err == ok
+        err, _, count = cudart.cudaGraphGetNodes(graph)
+        err, nodes, count = cudart.cudaGraphGetNodes(graph, count)
+        assert err == ok
+        kinds = [cudart.cudaGraphNodeGetType(n)[1] for n in nodes[:count]]
+        cudart.cudaGraphDestroy(graph)
+    types = cudart.cudaGraphNodeType
+    assert kinds.count(types.cudaGraphNodeTypeKernel) == kernels
+    assert len(kinds) - kernels == (1 if nx == 64 and prec == "fp32" else 0)
