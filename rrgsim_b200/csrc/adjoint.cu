@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kBS, 2) vjp_f32x2_kernel(const VjpParams<float
 // masses) instead of twice 29. The j sums (T, m-bar and the force) travel along the warp. G2 packed
 // pairs of i-particles per thread. NV sums per particle: T (3), m-bar, FORCE: the force (3).
 // Slots as in direct_sym.cu, one array of (T, m-bar) and, FORCE, one of the force behind it.
-// Bound: the FP32 pipe (64% of its peak). N = 16,384, equal masses, with the finish, us, ordered
+// Bound: the FP32 pipe (77% of the active cycles; the runs end unevenly). N = 16,384, equal masses, with the finish, us, ordered
 // pairs (vjp_f32x2_kernel) -> here: with the force and the mass gradient 284 -> 246, without the
 // force 252 -> 205.
 // ----------------------------------------------------------------------------------------------
@@ -537,8 +537,9 @@ __global__ void __launch_bounds__(kBS, 2) vjp_pair_kernel(const VjpPairParams p)
 // (x-bar_j -= T, m-bar_j += f (lam_k . d)) travel along the warp with the j they belong to (one
 // shuffle per sum and step, see the kernel) and each warp adds its sums for a chunk of 32 j into
 // a shared accumulator; block (a, b) then writes its tile-a sums to slot [a][b] and its
-// tile-b sums to slot [b][a]. A finish pass adds the T slots of each particle in order
-// (deterministic). Diagonal tiles evaluate only the k-side, as a non-symmetric pass would.
+// tile-b sums to slot [b][a]. A finish pass adds the T slots of each particle in order. (The four
+// warps add to the shared accumulator in no fixed order: the last bits of an FP64 gradient may differ
+// from run to run.) Diagonal tiles evaluate only the k-side, as a non-symmetric pass would.
 template <typename R>
 struct VjpSymParams {
     const V4<R>* posm;

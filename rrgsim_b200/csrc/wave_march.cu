@@ -17,8 +17,9 @@
 // so that every ring index is a constant and no value moves. New levels go to other buffers than
 // the ones read: the neighbours' halos need the old ones.
 //
-// Bound: shared-memory and shuffle throughput (256^3: DRAM 3.4 TB/s, issue 38 %, LSU 37 %, the
-// longest waits on shared-memory results and their queue; the halos cost 1.9 times the arithmetic).
+// Bound: shared-memory and shuffle throughput (256^3, a steady launch: shared-memory wavefronts 69 %,
+// DRAM 3.5 TB/s, issue 42 % of the active cycles, the longest waits on shared-memory results and their
+// queue; the halos cost 1.9 times the arithmetic).
 // Tried and slower at 256^3, us per substep: loads three planes ahead into registers instead of
 // the copies 32.0, the sums over the steps before formed for all levels first 30.6, 40 rows per
 // block 29.9, four cells per lane with 48 rows and one even share of all planes per block 33.8
